@@ -39,6 +39,7 @@
 #include "divide.cuh"
 #include "internal.h"
 #include "fdmt_plan.h"
+#include "fdmt_run.h"
 
 namespace bfs {
 namespace {
@@ -1174,14 +1175,47 @@ static std::vector<std::vector<int>> row_exponents(const FdmtPlanHost& h) {
 }
 
 constexpr int kSegDefaultLevels = 3;
+constexpr int kRunDefaultLevels = 4;          // two stages of two levels
+constexpr size_t kRunSmem = 113 * 1024;       // two CTAs per SM
+constexpr int kRunCtas = 2 * 148;
 
+// The run segment of a fused pass.  Output rows per tile: the count whose
+// tiles finish first by this estimate: a tile of G rows reads
+// G + 2^m - 1 input rows and forms G + 2^s2 - 1 mid rows, eight warps share a
+// stage's rows, a step of stage 1 costs 1.25 of stage 2's and copying a row a
+// quarter of it (shared-memory wavefronts), and the tiles run in waves of two
+// CTAs per SM.  Large planes take the most rows that fit (4096 x 45001: 40
+// rows 1.05 ms, 32 1.09, 24 1.19, 16 1.43), short ones fewer (256 x 22005: 32
+// rows 36.9 us, 40 41.1; 64 x 1000: 16 rows 12.5 us, 32 16.5).
+static void plan_run(const FdmtPlanHost& h, int l0, int l1, bool from_input, RunPlan* out) {
+    const int m = l1 - l0, s2 = m == 4 ? 2 : 1;
+    const long long tt = (h.ncols + kSegTile - 1) / kSegTile;
+    std::vector<std::pair<double, int>> order;
+    for (int G = 8; G <= 48; G += 4) {
+        long long tiles = 0, left = 0;   // the cut of build_run_plan
+        for (int r : h.lv[l1].rows) {
+            if (r > G) { tiles += (r + G - 1) / G; left = 0; }
+            else if (left >= r) { left -= r; }
+            else { ++tiles; left = G - r; }
+        }
+        const long long waves = (tiles * tt + kRunCtas - 1) / kRunCtas;
+        const double tile = 0.25 * (G + (1 << m) - 1) / 8.0 + 1.25 * ((G + (1 << s2) - 1 + 7) / 8) + (G + 7) / 8;
+        order.push_back({waves * tile, G});
+    }
+    std::sort(order.begin(), order.end());
+    for (const auto& o : order)
+        if (build_run_plan(h, l0, l1, o.second, kRunSmem, out, from_input)) return;
+}
+
+// `tables`: k_fdmt_seg's tables are wanted for passes that run segments serve
+// too (introspection, and refusals of explicit schedules it cannot run).
 // The passes after the head (or level 0): levels k+1..niter cut into fused
 // segments of about desc->seg_levels levels (FP32 plans), or one plain merge
 // pass per level; then the ping-pong plane of every level that reaches HBM.
-static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p) {
+static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int default_levels, bool tables) {
     const FdmtPlanHost& h = p->host;
-    const int k = p->head.depth;
-    const int want = desc->seg_levels == 0 ? kSegDefaultLevels : desc->seg_levels;
+    const int k = p->fuse_depth;
+    const int want = desc->seg_levels == 0 ? default_levels : desc->seg_levels;
     BFS_ARG(want >= 1 && want <= kSegMaxLevels, "seg_levels %d out of range (0..%d)", desc->seg_levels,
             kSegMaxLevels);
     BFS_ARG(desc->seg_rows >= 0, "seg_rows %d is negative", desc->seg_rows);
@@ -1194,11 +1228,27 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p) {
     BFS_ARG(!explicit_seg || p->precision == BFS_PREC_F32,
             "fused merge segments are implemented for FP32 plans");
     p->passes.clear();
+    p->runs.clear();
     auto plain = [&](int l) {
         SegPlan sp;
         sp.l0 = l - 1;
         sp.l1 = l;
         p->passes.push_back(sp);
+    };
+    // a fused pass runs as a run segment where one fits two CTAs on an SM,
+    // unless the description names a CTA size or buffering of k_fdmt_seg
+    const bool run_ok = desc->seg_threads == 0 && desc->seg_flags == 0;
+    auto run_alone = [&](int l0, int l1, bool from_input) {
+        if (tables || !run_ok) return false;
+        RunPlan rp;
+        plan_run(h, l0, l1, from_input, &rp);
+        if (rp.s1 == 0) return false;
+        SegPlan sp;
+        sp.l0 = l0; sp.l1 = l1; sp.r0c = rp.r0c;
+        p->passes.push_back(sp);
+        p->runs.resize(p->passes.size());
+        p->runs.back() = std::move(rp);
+        return true;
     };
     const int left = h.niter - k;
     if (want < 2 || p->precision != BFS_PREC_F32 || left < 2) {
@@ -1211,7 +1261,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p) {
             // no head: the first segment reads the channels and forms level 0
             // itself (no level-0 plane), where the plan's level 0 allows it
             if (i == 0 && k == 0 && h.kind == BFS_PLAN_KEITH && l1 >= 2) {
-                bool ok = false;
+                bool ok = run_alone(0, l1, true);
                 for (int G : {desc->seg_rows > 0 ? desc->seg_rows : 32, 16}) {
                     for (size_t limit : {kHeadSmemTwoPerSm, kHeadSmemMax}) {
                         SegPlan sp;
@@ -1228,7 +1278,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p) {
             }
             if (l1 == l0 + 1) {
                 plain(l1);
-            } else {
+            } else if (!run_alone(l0, l1, false)) {
                 // rows per tile: the most that keep two CTAs per SM, else one
                 std::vector<std::pair<int, size_t>> rows_try = {
                     {64, kHeadSmemTwoPerSm}, {32, kHeadSmemTwoPerSm}, {16, kHeadSmemTwoPerSm},
@@ -1252,6 +1302,11 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p) {
         }
     }
     for (SegPlan& sp : p->passes) sp.threads = desc->seg_threads;
+    p->runs.resize(p->passes.size());
+    for (size_t i = 0; i < p->passes.size(); ++i) {
+        const SegPlan& sp = p->passes[i];
+        if (run_ok && p->runs[i].s1 == 0 && !sp.tiles.empty()) plan_run(h, sp.l0, sp.l1, sp.r0c > 0, &p->runs[i]);
+    }
     // planes in HBM: level k (unless an input segment forms it on chip), then
     // every pass's output, alternating between the two buffers (the last
     // level goes to the caller's output)
@@ -1269,7 +1324,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p) {
     return BFS_OK;
 }
 
-static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_fdmt_plan>& p) {
+static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_fdmt_plan>& p, bool tables) {
     BFS_ARG(desc != nullptr, "null argument");
     BFS_ARG(desc->plan_kind == BFS_PLAN_KEITH || desc->plan_kind == BFS_PLAN_PRAVIR,
             "unsupported plan_kind %d", desc->plan_kind);
@@ -1286,7 +1341,7 @@ static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_
                                           desc->dt_step > 0 ? desc->dt_step : 1, desc->dt_min, &p->host);
         if (st != BFS_OK) return st;
         p->fuse_depth = 0;
-        return build_passes(desc, p.get());
+        return build_passes(desc, p.get(), kSegDefaultLevels, tables);
     }
     bfs_status st = build_fdmt_plan(desc->fmin, desc->fmax, desc->nchan, desc->ncols,
                                     desc->max_dt, &p->host);
@@ -1311,8 +1366,17 @@ static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_
         BFS_ARG(desc->fuse_depth <= 0 || p->head.depth == desc->fuse_depth,
                 "fuse_depth %d is not usable for this plan", desc->fuse_depth);
     }
+    // default schedule: level 0 formed by an input run segment where the plan
+    // has one (4096 x 45001: 1.05 ms against 2.32 with the head, 512 x 32768:
+    // 0.113 against 0.208); the head stays for bfs_fdmt_execute_noalloc
+    if (desc->fuse_depth < 0 && p->precision == BFS_PREC_F32 && desc->head_tile == 0 && desc->seg_levels == 0 &&
+        desc->seg_rows == 0 && desc->seg_threads == 0 && desc->seg_flags == 0) {
+        p->fuse_depth = 0;
+        if (build_passes(desc, p.get(), kRunDefaultLevels, tables) == BFS_OK && !p->runs.empty() && p->runs[0].s1 > 0)
+            return BFS_OK;
+    }
     p->fuse_depth = p->head.depth;
-    return build_passes(desc, p.get());
+    return build_passes(desc, p.get(), kSegDefaultLevels, tables);
 }
 
 static inline int bfs_fdmt_plan_depth_of(int d) { return d; }
@@ -1357,6 +1421,16 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
     }
     struct Cand { int depth, tile, seg, rows, flags; };
     std::vector<Cand> cands;
+    // plans with an input run segment: levels per segment (the rows per tile
+    // of run segments follow their own rule)
+    std::unique_ptr<bfs_fdmt_plan> probe;
+    bfs_fdmt_desc d0 = base;
+    d0.fuse_depth = -1;
+    d0.head_tile = d0.seg_levels = d0.seg_rows = d0.seg_threads = d0.seg_flags = 0;
+    const bool runs = plan_host_part(&d0, probe, false) == BFS_OK && !probe->runs.empty() && probe->runs[0].s1 > 0;
+    if (runs) {
+        for (int seg : {4, 3, 2}) cands.push_back({0, 0, seg, 32, 0});
+    } else {
     // one merge pass per level: head depth x head tile
     cands.push_back({0, 0, 1, 0, 0});
     for (int k : {2, 3, 4, 5})
@@ -1374,6 +1448,7 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
                 if (rows == 16 || rows == 32)
                     for (int k : {2, 3, 4}) cands.push_back({k, 256, seg, rows, 0});
             }
+    }
     const size_t in_n = static_cast<size_t>(base.nchan) * base.ncols;
     const size_t out_n = static_cast<size_t>(base.max_dt) * base.ncols;
     float *d_in = nullptr, *d_out = nullptr;
@@ -1471,7 +1546,7 @@ extern "C" bfs_status bfs_fdmt_plan_create_host(const bfs_fdmt_desc* desc, bfs_f
     BFS_ARG(plan != nullptr, "null argument");
     *plan = nullptr;
     std::unique_ptr<bfs_fdmt_plan> p;
-    bfs_status st = plan_host_part(desc, p);
+    bfs_status st = plan_host_part(desc, p, true);
     if (st != BFS_OK) return st;
     *plan = p.release();
     return BFS_OK;
@@ -1494,12 +1569,12 @@ extern "C" bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc_in, bfs_fdm
     }
     const bfs_fdmt_desc* desc = &tuned;
     std::unique_ptr<bfs_fdmt_plan> p;
-    bfs_status st = plan_host_part(desc, p);
+    bfs_status st = plan_host_part(desc, p, desc_in->seg_rows > 0);
     if (st != BFS_OK) return st;
     p->host_only = false;
     BFS_CUDA(cudaGetDevice(&p->device));
     const FdmtPlanHost& h = p->host;
-    if (p->head.depth > 0) {
+    if (p->fuse_depth > 0) {
         const HeadPlan& hp = p->head;
         BFS_CUDA(cudaMalloc(&p->d_head_groups, hp.groups.size() * sizeof(HeadGroup)));
         BFS_CUDA(cudaMemcpy(p->d_head_groups, hp.groups.data(),
@@ -1556,6 +1631,26 @@ extern "C" bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc_in, bfs_fdm
                                 cudaMemcpyHostToDevice));
             BFS_CUDA(cudaMalloc(&p->d_seg_ent, ent.size() * sizeof(int)));
             BFS_CUDA(cudaMemcpy(p->d_seg_ent, ent.data(), ent.size() * sizeof(int), cudaMemcpyHostToDevice));
+        }
+    }
+    {
+        std::vector<RunTile> tiles;
+        std::vector<int> rows, ent;
+        for (const RunPlan& rp : p->runs) {
+            p->run_tile0.push_back(tiles.size());
+            p->run_row0.push_back(rows.size());
+            p->run_ent0.push_back(ent.size());
+            tiles.insert(tiles.end(), rp.tiles.begin(), rp.tiles.end());
+            rows.insert(rows.end(), rp.rows.begin(), rp.rows.end());
+            ent.insert(ent.end(), rp.ent.begin(), rp.ent.end());
+        }
+        if (!tiles.empty()) {
+            BFS_CUDA(cudaMalloc(&p->d_run_tiles, tiles.size() * sizeof(RunTile)));
+            BFS_CUDA(cudaMalloc(&p->d_run_rows, rows.size() * sizeof(int)));
+            BFS_CUDA(cudaMalloc(&p->d_run_ent, ent.size() * sizeof(int)));
+            BFS_CUDA(cudaMemcpy(p->d_run_tiles, tiles.data(), tiles.size() * sizeof(RunTile), cudaMemcpyHostToDevice));
+            BFS_CUDA(cudaMemcpy(p->d_run_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice));
+            BFS_CUDA(cudaMemcpy(p->d_run_ent, ent.data(), ent.size() * sizeof(int), cudaMemcpyHostToDevice));
         }
     }
     // ping-pong planes (sized by build_passes); levels inside the fused head
@@ -1615,6 +1710,31 @@ extern "C" bfs_status bfs_fdmt_plan_passes(const bfs_fdmt_plan* plan, int* npass
                                static_cast<int>(sp.ent.size() / 4), sp.r0c};
             std::memcpy(params + 13 * i, v, sizeof(v));
         }
+    }
+    return BFS_OK;
+}
+
+extern "C" bfs_status bfs_fdmt_plan_run(const bfs_fdmt_plan* plan, int pass, int* params, int* tiles, int tiles_cap,
+                                        int* rows, int rows_cap, int* ent, int ent_cap) {
+    BFS_ARG(plan != nullptr && params != nullptr, "null argument");
+    BFS_ARG(pass >= 0 && pass < static_cast<int>(plan->runs.size()), "pass %d out of range", pass);
+    const RunPlan& rp = plan->runs[pass];
+    constexpr int ti = static_cast<int>(sizeof(RunTile) / sizeof(int));
+    const int v[14] = {rp.s1, rp.s2, rp.r0c, rp.pitch_x, rp.zero_x, rp.y0, rp.zero_y, rp.ent0, rp.max_ent, rp.edge,
+                       static_cast<int>(rp.smem_bytes), static_cast<int>(rp.tiles.size()),
+                       static_cast<int>(rp.rows.size() / 2), static_cast<int>(rp.ent.size() / 4)};
+    std::memcpy(params, v, sizeof(v));
+    if (tiles) {
+        BFS_ARG(tiles_cap >= ti * v[11], "tiles needs %d ints", ti * v[11]);
+        std::memcpy(tiles, rp.tiles.data(), rp.tiles.size() * sizeof(RunTile));
+    }
+    if (rows) {
+        BFS_ARG(rows_cap >= 2 * v[12], "rows needs %d ints", 2 * v[12]);
+        std::memcpy(rows, rp.rows.data(), rp.rows.size() * sizeof(int));
+    }
+    if (ent) {
+        BFS_ARG(ent_cap >= 4 * v[13], "ent needs %d ints", 4 * v[13]);
+        std::memcpy(ent, rp.ent.data(), rp.ent.size() * sizeof(int));
     }
     return BFS_OK;
 }
@@ -1814,7 +1934,7 @@ static bfs_status fdmt_run(bfs_fdmt_plan* plan, const float* d_in, float* d_out,
     float* bufs[2] = {buf0, buf1};
     auto plane = [&](int l) { return l == h.niter ? d_out : bufs[plan->plane_buf[l]]; };
     auto pitch = [&](int l) { return l == h.niter ? T : P; };
-    const int k = plan->head.depth;
+    const int k = plan->fuse_depth;
     const bool in_seg = !plan->passes.empty() && plan->passes[0].r0c > 0;
     if (k > 0) {
         const HeadPlan& hp = plan->head;
@@ -1833,7 +1953,12 @@ static bfs_status fdmt_run(bfs_fdmt_plan* plan, const float* d_in, float* d_out,
         const SegPlan& sp = plan->passes[i];
         const float* src = sp.r0c > 0 ? d_in : plane(sp.l0);
         cudaError_t e;
-        if (sp.tiles.empty()) {
+        if (plan->runs[i].s1 > 0) {  // (an input segment reads the caller's filterbank: pitch ncols)
+            e = launch_run(plan->runs[i], src, plane(sp.l1), plan->d_run_tiles + plan->run_tile0[i],
+                           reinterpret_cast<const int2*>(plan->d_run_rows + plan->run_row0[i]),
+                           reinterpret_cast<const int4*>(plan->d_run_ent + plan->run_ent0[i]), T,
+                           sp.r0c > 0 ? T : P, pitch(sp.l1), sp.r0c > 0 && b_ones ? 1 : 0, s);
+        } else if (sp.tiles.empty()) {
             e = launch_level(src, plane(sp.l1), plan->d_tab + plan->tab_off[sp.l1],
                              h.lv[sp.l1].total_rows(), T, P, pitch(sp.l1), s);
         } else if (sp.r0c > 0) {  // input segment: the caller's filterbank (pitch ncols)

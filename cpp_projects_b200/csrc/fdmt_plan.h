@@ -25,10 +25,15 @@ struct bfs_fdmt_plan {
     // passes after the head (or level 0): a fused segment of levels l0+1..l1
     // (tiles non-empty) or one plain merge level (l1 = l0 + 1, no tiles)
     std::vector<bfs::SegPlan> passes;
+    std::vector<bfs::RunPlan> runs;    // per pass: its run segment (s1 = 0: k_fdmt_seg or a plain level)
     std::vector<int> plane_buf;        // per level: ping-pong plane holding it in HBM (-1: never)
     bfs::SegTile* d_seg_tiles = nullptr;  // every fused segment's tiles, concatenated
     int* d_seg_ent = nullptr;          // every fused segment's entries, concatenated
     std::vector<size_t> seg_tile0, seg_ent0;  // per pass: offsets into the two arrays
+    bfs::RunTile* d_run_tiles = nullptr;  // every run segment's tiles, input rows and entries
+    int* d_run_rows = nullptr;
+    int* d_run_ent = nullptr;
+    std::vector<size_t> run_tile0, run_row0, run_ent0;
     int* d_lvl0 = nullptr;             // Pravir plans: level-0 row cumsum (nchan+1) then delays
     int* d_ones_tau = nullptr;         // FDMT of 0/1 rows: tau [out_row][channel] (first use)
     int ones_max_tau = -1;
@@ -45,6 +50,9 @@ struct bfs_fdmt_plan {
         if (d_lvl0) cudaFree(d_lvl0);
         if (d_seg_tiles) cudaFree(d_seg_tiles);
         if (d_seg_ent) cudaFree(d_seg_ent);
+        if (d_run_tiles) cudaFree(d_run_tiles);
+        if (d_run_rows) cudaFree(d_run_rows);
+        if (d_run_ent) cudaFree(d_run_ent);
         if (d_ones_tau) cudaFree(d_ones_tau);
         for (void* b : d_buf)
             if (b) cudaFree(b);

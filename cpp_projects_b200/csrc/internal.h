@@ -206,4 +206,64 @@ struct SegPlan {
 bool build_seg_plan(const FdmtPlanHost& p, int l0, int l1, int rows, int tile, size_t smem_limit,
                     SegPlan* out, bool from_input = false, bool single = false);
 
+// ---------------------------------------------------------------------------
+// Run segment: levels l0+1..l1 (two, three or four) in one pass over HBM, as
+// two stages of one or two merge levels each.  A stage forms a row from the
+// two or four rows below it at once, in registers: with two levels,
+//   out[t] = (A[t] + B[t - p]) + (C[t - q] + D[t - q - r])
+// (the adds of the two levels, each rounded as there).  Consecutive rows of
+// a sub-band step along a staircase through the tables: from one row to the
+// next either the tail changes or the head does, so most of the four inputs
+// stay where they were and are kept in registers; an entry says which of
+// them moved.  Stage 1 goes from the input rows (buffer X) to the mid level
+// (buffer Y), stage 2 from there to HBM.
+//
+// A tile is `n2` consecutive rows of the level-l1 plane from row out0 on (cut
+// at sub-band borders, so its mid rows belong to few sub-bands) x kSegTile
+// samples.  The mid rows of one sub-band share one window (samples
+// t0 - hi .. ), which keeps an unchanged input at one offset from row to row.
+// X holds the input rows, `pitch_x` floats each, then a row of -0.0 (the head
+// of rows without one); samples before 0 hold -0.0 as well, so no merge
+// tests t >= shift: x + -0 is x bit for bit.  Y holds the mid rows, kRunMid
+// floats each, then its -0.0 row.  Each buffer's -0.0 row is long enough for
+// a read of its last row that runs past the row's end (columns no written
+// sample depends on).
+// Input segments (r0c > 0): the input rows are channels and an input of
+// stage 1 is a level-0 row of one: entry bits 20.. give its row number r, the
+// running mean over r + 1 samples is formed where it is read.
+// ---------------------------------------------------------------------------
+constexpr int kRunMidChunks = 9;                  // 32-column chunks of a mid row
+constexpr int kRunMid = 32 * kRunMidChunks;
+constexpr int kRunOutChunks = kSegTile / 32;
+constexpr int kRunMaxPitch = 384;
+
+struct RunTile {                 // device-side
+    int row;                     // first of the tile's input rows
+    int ent;                     // first of its entries: n1 of stage 1, then n2 of stage 2
+    int n_in, n1, n2;
+    int out0;                    // first row in the level-l1 plane
+    int pad[2];
+};
+
+struct RunPlan {
+    int l0 = 0, l1 = 0;
+    int s1 = 0, s2 = 0;          // levels merged by each stage (0: no plan)
+    int r0c = 0;                 // input segment: level-0 rows per channel
+    int pitch_x = 0;             // floats per row of X
+    int zero_x = 0, zero_y = 0;  // offsets of the -0.0 rows
+    int y0 = 0, ent0 = 0;        // offsets of Y and of the two staged entry buffers
+    int max_ent = 0;             // most entries of one tile
+    int edge = 0;                // tiles with t0 >= edge read no sample before the last level-0 row number
+    size_t smem_bytes = 0;
+    std::vector<RunTile> tiles;
+    std::vector<int> rows;       // 2 ints per input row: {plane row, lead}: its window starts at t0 - lead
+    std::vector<int> ent;        // 4 ints per entry: byte offsets of the inputs | 1 where it moved | r << 20
+};
+
+// False when a window, a row or smem_limit does not allow it.  ncols fixes
+// the leads of an input segment: a channel's window starts on a 16-byte
+// boundary of the filterbank, whose rows are ncols floats.
+bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int rows, size_t smem_limit, RunPlan* out,
+                    bool from_input);
+
 }  // namespace bfs

@@ -374,6 +374,167 @@ bool build_seg_plan(const FdmtPlanHost& p, int l0, int l1, int G, int TT, size_t
     return true;
 }
 
+bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_limit, RunPlan* out,
+                    bool from_input) {
+    const int m = l1 - l0;
+    if (m < 2 || m > 4 || l0 < 0 || l1 > p.niter || G < 1) return false;
+    const int r0c = p.rows_per_chan0;
+    if (from_input && (p.kind != BFS_PLAN_KEITH || l0 != 0 || r0c < 1 || r0c > 5)) return false;
+    RunPlan s;
+    s.l0 = l0; s.l1 = l1; s.s1 = m >= 3 ? 2 : 1; s.s2 = m - s.s1; s.r0c = from_input ? r0c : 0;
+    const int lm = l1 - s.s2;
+    struct Leaf { int row, shift; };             // row -1: the -0.0 row
+    struct Row { int row, lo, hi; };             // needs samples t0 - hi .. t0 + kSegTile - lo
+    auto leaves = [&](int level, int g, int levels, Leaf (&v)[4]) {
+        const FdmtLevel& L = p.lv[level];
+        const Leaf a{L.a_row[g], 0};
+        const Leaf b = L.b_row[g] >= 0 ? Leaf{L.b_row[g], L.shift[g]} : Leaf{-1, 0};
+        if (levels == 1) { v[0] = a; v[1] = b; v[2] = v[3] = Leaf{-1, 0}; return; }
+        const FdmtLevel& P = p.lv[level - 1];
+        auto split = [&](const Leaf& x, Leaf& lo, Leaf& hi) {
+            lo = hi = Leaf{-1, 0};
+            if (x.row < 0) return;
+            lo = Leaf{P.a_row[x.row], x.shift};
+            if (P.b_row[x.row] >= 0) hi = Leaf{P.b_row[x.row], x.shift + P.shift[x.row]};
+        };
+        split(a, v[0], v[1]);
+        split(b, v[2], v[3]);
+    };
+    auto add = [](std::vector<Row>& v, int row, int lo, int hi) { v.push_back({row, lo, hi}); };
+    auto unite = [](std::vector<Row>& v) {       // sorted by row, one entry per row
+        std::sort(v.begin(), v.end(), [](const Row& a, const Row& b) { return a.row < b.row; });
+        size_t k = 0;
+        for (size_t i = 0; i < v.size(); ++i) {
+            if (k && v[k - 1].row == v[i].row) {
+                v[k - 1].lo = std::min(v[k - 1].lo, v[i].lo);
+                v[k - 1].hi = std::max(v[k - 1].hi, v[i].hi);
+            } else {
+                v[k++] = v[i];
+            }
+        }
+        v.resize(k);
+    };
+    // tiles: sub-bands of more than G rows are cut into equal parts, shorter
+    // ones taken together while they fit
+    std::vector<std::pair<int, int>> cuts;
+    const FdmtLevel& top = p.lv[l1];
+    for (int b = 0; b < top.nsub;) {
+        if (top.rows[b] > G) {
+            const int parts = (top.rows[b] + G - 1) / G;
+            for (int i = 0; i < parts; ++i)
+                cuts.push_back({top.cum[b] + top.rows[b] * i / parts, top.cum[b] + top.rows[b] * (i + 1) / parts});
+            ++b;
+            continue;
+        }
+        int e = b + 1;
+        while (e < top.nsub && top.cum[e + 1] - top.cum[b] <= G) ++e;
+        cuts.push_back({top.cum[b], top.cum[e]});
+        b = e;
+    }
+    struct Tile { int g0, g1; std::vector<Row> mid, in; };
+    std::vector<Tile> tiles;
+    const std::vector<int>& mcum = p.lv[lm].cum;
+    int spread = 0, max_in = 0, max_mid = 0, max_lead = 0;
+    for (const auto& c : cuts) {
+        Tile t;
+        t.g0 = c.first; t.g1 = c.second;
+        if (t.g0 == t.g1) continue;
+        Leaf v[4];
+        for (int g = t.g0; g < t.g1; ++g) {
+            leaves(l1, g, s.s2, v);
+            for (const Leaf& x : v)
+                if (x.row >= 0) add(t.mid, x.row, x.shift, x.shift);
+        }
+        unite(t.mid);
+        // one window per sub-band of the mid level
+        for (size_t i = 0; i < t.mid.size();) {
+            const int band = static_cast<int>(std::upper_bound(mcum.begin(), mcum.end(), t.mid[i].row) - mcum.begin()) - 1;
+            size_t e = i;
+            int lo = t.mid[i].lo, hi = t.mid[i].hi;
+            for (; e < t.mid.size() && t.mid[e].row < mcum[band + 1]; ++e) {
+                lo = std::min(lo, t.mid[e].lo);
+                hi = std::max(hi, t.mid[e].hi);
+            }
+            if (kSegTile + hi - lo > kRunMid) return false;
+            for (; i < e; ++i) { t.mid[i].lo = lo; t.mid[i].hi = hi; }
+        }
+        for (const Row& r : t.mid) {
+            leaves(lm, r.row, s.s1, v);
+            for (const Leaf& x : v) {
+                if (x.row < 0) continue;
+                if (from_input) add(t.in, x.row / r0c, r.lo + x.shift, r.hi + x.shift + x.row % r0c);
+                else add(t.in, x.row, r.lo + x.shift, r.hi + x.shift);
+            }
+        }
+        unite(t.in);
+        for (Row& r : t.in) {
+            // first sample t0 - hi on a 16-byte boundary (t0 a multiple of 4)
+            const int phase = from_input ? static_cast<int>((static_cast<long long>(r.row) * p.ncols) & 3) : 0;
+            while ((r.hi & 3) != phase) ++r.hi;
+            spread = std::max(spread, r.hi - r.lo);
+            max_lead = std::max(max_lead, r.hi);
+        }
+        max_in = std::max(max_in, static_cast<int>(t.in.size()));
+        max_mid = std::max(max_mid, static_cast<int>(t.mid.size()));
+        s.max_ent = std::max(s.max_ent, static_cast<int>(t.mid.size()) + t.g1 - t.g0);
+        if (4ull * (static_cast<size_t>(max_in) * (kSegTile + spread) + static_cast<size_t>(max_mid) * kRunMid) > smem_limit)
+            return false;
+        tiles.push_back(std::move(t));
+    }
+    s.pitch_x = (kSegTile + spread + 3) & ~3;
+    if (s.pitch_x > kRunMaxPitch) return false;
+    s.zero_x = max_in * s.pitch_x;
+    s.y0 = s.zero_x + kRunMid;
+    s.zero_y = s.y0 + max_mid * kRunMid;
+    s.ent0 = s.zero_y + kSegTile;
+    s.edge = max_lead + r0c;
+    ++s.max_ent;   // (the kernel reads one entry ahead)
+    s.smem_bytes = static_cast<size_t>(s.ent0) * sizeof(float) + 2 * static_cast<size_t>(s.max_ent) * 16;
+    if (s.smem_bytes > smem_limit) return false;
+    auto slot_of = [](const std::vector<Row>& v, int row) {
+        return static_cast<int>(std::lower_bound(v.begin(), v.end(), row, [](const Row& w, int r) { return w.row < r; }) -
+                                v.begin());
+    };
+    // one stage's entries; prev = the inputs of the row before
+    auto entries = [&](int level, int levels, const std::vector<Row>& from, int base, int pitch, int zero, bool chan,
+                       int row, int hi, int (&prev)[4]) {
+        Leaf v[4];
+        leaves(level, row, levels, v);
+        for (int i = 0; i < 4; ++i) {
+            int e = zero * 4;
+            if (v[i].row >= 0) {
+                const int src = chan ? v[i].row / r0c : v[i].row, r = chan ? v[i].row % r0c : 0;
+                const int j = slot_of(from, src);
+                const int off = from[j].hi - hi - v[i].shift;
+                if (off < r || off + kSegTile > pitch) return false;
+                e = (base + j * pitch + off) * 4 | (r << 20);
+            }
+            s.ent.push_back(e | (e != prev[i] ? 1 : 0));
+            prev[i] = e;
+        }
+        return true;
+    };
+    for (const Tile& t : tiles) {
+        RunTile r{};
+        r.row = static_cast<int>(s.rows.size() / 2);
+        r.ent = static_cast<int>(s.ent.size() / 4);
+        r.n_in = static_cast<int>(t.in.size());
+        r.n1 = static_cast<int>(t.mid.size());
+        r.n2 = t.g1 - t.g0;
+        r.out0 = t.g0;
+        for (const Row& w : t.in) s.rows.insert(s.rows.end(), {w.row, w.hi});
+        int prev[4] = {-1, -1, -1, -1};
+        for (const Row& w : t.mid)
+            if (!entries(lm, s.s1, t.in, 0, s.pitch_x, s.zero_x, from_input, w.row, w.hi, prev)) return false;
+        for (int& x : prev) x = -1;
+        for (int g = t.g0; g < t.g1; ++g)
+            if (!entries(l1, s.s2, t.mid, s.y0, kRunMid, s.zero_y, false, g, 0, prev)) return false;
+        s.tiles.push_back(r);
+    }
+    *out = std::move(s);
+    return true;
+}
+
 void build_adjoint_tables(const FdmtPlanHost& p, AdjointTables* out) {
     out->off_pos.assign(p.niter + 1, 0);
     out->ent_pos.assign(p.niter + 1, 0);

@@ -79,8 +79,10 @@ typedef struct bfs_fdmt_desc {
     int max_dt;        /* output rows (>= 1)                            */
     int plan_kind;     /* BFS_PLAN_KEITH                                */
     int precision;     /* BFS_PREC_F32 (default), BFS_PREC_F16, BFS_PREC_BF16 */
-    int fuse_depth;    /* BFS_FUSE_AUTOTUNE (-2): measured per shape (cached); -1: deepest
-                          head keeping 2 CTAs/SM; 0: level-by-level; k: fuse levels 0..k */
+    int fuse_depth;    /* BFS_FUSE_AUTOTUNE (-2): measured per shape (cached); -1: with no
+                          other schedule field set, run segments of 4 levels from the
+                          channels on (FP32), else, or where the plan has none, the
+                          deepest head keeping 2 CTAs/SM; 0: no head; k: fuse levels 0..k */
     int flags;         /* BFS_FDMT_EXTERNAL_WS: the plan allocates no planes; use _execute_ws */
     int head_tile;     /* samples per CTA of the fused head (0 = 256)                  */
     int dt_min;        /* BFS_PLAN_PRAVIR: smallest delay of the grid (0)              */
@@ -89,12 +91,12 @@ typedef struct bfs_fdmt_desc {
     int seg_levels;    /* merge levels fused per HBM pass after the head (FP32 plans):
                           0: 3; 1: one pass per level; 2..6                              */
     int seg_rows;      /* output rows per tile of a fused pass (0: the most that keep
-                          two CTAs per SM, of 64 / 32 / 16; the autotuner also tries
-                          24 and 28, which fit a single-buffered input segment into
-                          half an SM's shared memory)                                    */
-    int seg_threads;   /* threads per CTA of the fused passes: 256, 512, 1024 (0: 256
-                          when two CTAs fit an SM, else 512)                             */
-    int seg_flags;     /* BFS_SEG_SINGLE_BUFFER: one input buffer per CTA (the next
+                          two CTAs per SM, of 64 / 32 / 16; run segments choose theirs) */
+    int seg_threads;   /* 0 with seg_flags 0: passes of 2..4 levels are run segments
+                          (bfs_fdmt_plan_run); 256, 512, 1024: the one-level-at-a-time
+                          segment kernel with that many threads per CTA                  */
+    int seg_flags;     /* BFS_SEG_SINGLE_BUFFER: the one-level-at-a-time segment kernel
+                          with one input buffer per CTA (the next
                           tile loads after the current one is merged; half the shared
                           memory, so two CTAs fit an SM)                                 */
 } bfs_fdmt_desc;
@@ -118,9 +120,10 @@ typedef struct bfs_fdmt_info {
 } bfs_fdmt_info;
 
 bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc, bfs_fdmt_plan** plan);
-/* The autotuner alone (no reference counterpart): times fusion depths
- * {0,2,3,4,5} x head tiles {256,512} x merge segments of 1..4 levels on this shape with zero input (the
- * kernels' cost does not depend on the values) and returns the fastest;
+/* The autotuner alone (no reference counterpart): times run segments of 2,
+ * 3 and 4 levels (plans without them: fusion depths {0,2,3,4,5} x
+ * head tiles {256,512} x merge segments of 1..4 levels) on this shape with
+ * zero input (the kernels' cost does not depend on the values) and returns the fastest;
  * results are cached per (nchan, max_dt, band, ncols rounded up to 2^k). */
 bfs_status bfs_fdmt_autotune(const bfs_fdmt_desc* desc, int* depth, int* head_tile, float* ms);
 /* The same measurement over fusion depth, head tile and fused merge-segment
@@ -167,6 +170,15 @@ bfs_status bfs_fdmt_plan_passes(const bfs_fdmt_plan* plan, int* npasses, int* pa
  * shared buffer holds its rows, a row of -0.0 and a guard row. */
 bfs_status bfs_fdmt_plan_segment(const bfs_fdmt_plan* plan, int pass, int* tiles, int tiles_cap,
                                  int* ent, int ent_cap);
+/* Run segment of a pass (levels l0+1..l1 as two stages of one or two merge
+ * levels; the layout is described in the sources).  params[14] = {levels of
+ * stage 1 (0: the pass is no run segment), levels of stage 2, level-0 rows
+ * per channel, pitch of an input row, offset of its -0.0 row, offset of the
+ * mid rows, of their -0.0 row, of the staged entries, most entries of a tile,
+ * first sample of an edge-free tile, shared bytes, tiles, input rows,
+ * entries}; tiles: 8 ints each, rows: 2, ent: 4 (each may be NULL). */
+bfs_status bfs_fdmt_plan_run(const bfs_fdmt_plan* plan, int pass, int* params, int* tiles, int tiles_cap,
+                             int* rows, int rows_cap, int* ent, int ent_cap);
 /* d_in: nchan*ncols floats (ignored when b_ones != 0: an all-ones image is used,
  * the reference's normalisation mode), d_out: max_dt*ncols floats. */
 bfs_status bfs_fdmt_execute(bfs_fdmt_plan* plan, const float* d_in, float* d_out, int b_ones,
