@@ -1239,7 +1239,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
     // unless the description names a CTA size or buffering of k_fdmt_seg
     const bool run_ok = desc->seg_threads == 0 && desc->seg_flags == 0;
     auto run_alone = [&](int l0, int l1, bool from_input) {
-        if (tables || !run_ok) return false;
+        if ((tables && !(from_input && h.kind == BFS_PLAN_PRAVIR)) || !run_ok) return false;
         RunPlan rp;
         plan_run(h, l0, l1, from_input, &rp);
         if (rp.s1 == 0) return false;
@@ -1260,7 +1260,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
             const int l1 = l0 + left / nseg + (i < left % nseg ? 1 : 0);
             // no head: the first segment reads the channels and forms level 0
             // itself (no level-0 plane), where the plan's level 0 allows it
-            if (i == 0 && k == 0 && h.kind == BFS_PLAN_KEITH && l1 >= 2) {
+            if (i == 0 && k == 0 && l1 >= 2) {
                 bool ok = run_alone(0, l1, true);
                 for (int G : {desc->seg_rows > 0 ? desc->seg_rows : 32, 16}) {
                     for (size_t limit : {kHeadSmemTwoPerSm, kHeadSmemMax}) {
@@ -1341,7 +1341,7 @@ static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_
                                           desc->dt_step > 0 ? desc->dt_step : 1, desc->dt_min, &p->host);
         if (st != BFS_OK) return st;
         p->fuse_depth = 0;
-        return build_passes(desc, p.get(), kSegDefaultLevels, tables);
+        return build_passes(desc, p.get(), kRunDefaultLevels, tables);
     }
     bfs_status st = build_fdmt_plan(desc->fmin, desc->fmax, desc->nchan, desc->ncols,
                                     desc->max_dt, &p->host);

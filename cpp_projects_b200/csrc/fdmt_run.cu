@@ -47,13 +47,20 @@ __device__ __forceinline__ void load_row(float (&v)[K], const char* p) {
 
 // Level-0 row R of a channel (the reference's running mean, one rounding per
 // operation) from its samples: p addresses x[t] of this lane's first column.
-template <int R, int K>
+// POS: -0.0 samples count as +0 (RunPlan::positive).
+template <int R, int K, bool POS>
 __device__ __forceinline__ void mean_row(float (&v)[K], const char* p) {
-    load_row<K>(v, p);
+    auto samples = [](float (&x)[K], const char* at) {
+        load_row<K>(x, at);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (POS) x[k] = __fadd_rn(x[k], 0.0f);
+    };
+    samples(v, p);
 #pragma unroll
     for (int r = 1; r <= R; ++r) {
         float x[K];
-        load_row<K>(x, p - 4 * r);
+        samples(x, p - 4 * r);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const float m = r == 1 ? v[k] : __fmul_rn(v[k], static_cast<float>(r));
@@ -76,19 +83,22 @@ struct RunArgs {
 
 // An input of stage 1 of an input segment: the level-0 row its entry names; `edge` tiles hold samples before the row number, where the
 // level-0 row is 0 (and -0.0 before sample 0, as everywhere).
-template <int R0C, int K>
+template <int R0C, int K, bool POS>
 __device__ __forceinline__ void load_input(float (&v)[K], const char* lane_base, int q, bool edge, const RunArgs& a,
                                            const RunTile& t, int t0) {
     const int off = q & 0xffffc, r = q >> 20;
     const char* p = lane_base + off;
     switch (r) {
-        case 0: load_row<K>(v, p); return;
-        case 1: mean_row<1, K>(v, p); break;
-        case 2: if constexpr (R0C > 2) mean_row<2, K>(v, p); break;
-        case 3: if constexpr (R0C > 3) mean_row<3, K>(v, p); break;
-        default: if constexpr (R0C > 4) mean_row<4, K>(v, p); break;
+        case 0:   // (the -0.0 row stays as it is)
+            if (POS && off != 4 * a.zero_x) mean_row<0, K, true>(v, p);
+            else load_row<K>(v, p);
+            break;
+        case 1: mean_row<1, K, POS>(v, p); break;
+        case 2: if constexpr (R0C > 2) mean_row<2, K, POS>(v, p); break;
+        case 3: if constexpr (R0C > 3) mean_row<3, K, POS>(v, p); break;
+        default: if constexpr (R0C > 4) mean_row<4, K, POS>(v, p); break;
     }
-    if (edge) {
+    if (edge && (POS || r > 0) && off != 4 * a.zero_x) {
         const int j = (off >> 2) / a.pitch_x;
         const int first = t0 - __ldg(&a.rows[t.row + j].y) + (off >> 2) - j * a.pitch_x + (threadIdx.x & 31);
 #pragma unroll
@@ -115,7 +125,7 @@ __device__ __forceinline__ void load_input(float (&v)[K], const char* lane_base,
 // L2), two CTAs per SM.  A warp forms consecutive rows, lanes on consecutive
 // columns: every shared access is one wavefront whatever the offsets.  The
 // next tile's input is copied into X while stage 2 reads Y.
-template <int S1, int S2, int R0C>
+template <int S1, int S2, int R0C, bool POS>
 __global__ void __launch_bounds__(kRunThreads, 2) k_fdmt_run(const RunArgs a) {
     constexpr int K1 = kRunMidChunks, K2 = kRunOutChunks;
     extern __shared__ __align__(16) float sm[];
@@ -202,7 +212,7 @@ __global__ void __launch_bounds__(kRunThreads, 2) k_fdmt_run(const RunArgs a) {
                 for (int i = 0; i < 2 * S1; ++i) {
                     if (q[i] & 1) {
                         if constexpr (R0C <= 1) load_row<K1>(v[i], lane_base + (q[i] - 1));
-                        else load_input<R0C, K1>(v[i], lane_base, q[i], edge, a, t, t0);
+                        else load_input<R0C, K1, POS>(v[i], lane_base, q[i], edge, a, t, t0);
                     }
                 }
                 float o[K1];
@@ -257,9 +267,9 @@ __global__ void __launch_bounds__(kRunThreads, 2) k_fdmt_run(const RunArgs a) {
     }
 }
 
-template <int S1, int S2, int R0C>
+template <int S1, int S2, int R0C, bool POS>
 cudaError_t launch(const RunPlan& rp, const RunArgs& args, cudaStream_t s) {
-    auto kern = k_fdmt_run<S1, S2, R0C>;
+    auto kern = k_fdmt_run<S1, S2, R0C, POS>;
     // The shared-memory opt-in (one value per kernel and device, it only ever
     // grows) and the resident CTAs of a size are set on the size's first
     // launch, which therefore comes before any stream capture.
@@ -293,11 +303,11 @@ cudaError_t launch(const RunPlan& rp, const RunArgs& args, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int R0C>
+template <int R0C, bool POS = false>
 cudaError_t launch_stages(const RunPlan& rp, const RunArgs& a, cudaStream_t s) {
-    if (rp.s1 == 2 && rp.s2 == 2) return launch<2, 2, R0C>(rp, a, s);
-    if (rp.s1 == 2 && rp.s2 == 1) return launch<2, 1, R0C>(rp, a, s);
-    if (rp.s1 == 1 && rp.s2 == 1) return launch<1, 1, R0C>(rp, a, s);
+    if (rp.s1 == 2 && rp.s2 == 2) return launch<2, 2, R0C, POS>(rp, a, s);
+    if (rp.s1 == 2 && rp.s2 == 1) return launch<2, 1, R0C, POS>(rp, a, s);
+    if (rp.s1 == 1 && rp.s2 == 1) return launch<1, 1, R0C, POS>(rp, a, s);
     return cudaErrorInvalidValue;
 }
 
@@ -318,6 +328,7 @@ cudaError_t launch_run(const RunPlan& rp, const float* src, float* dst, const Ru
     // on a 16-byte boundary when the filterbank does
     a.vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (rp.r0c > 0 || in_pitch % 4 == 0) ? 1 : 0;
     a.ones = ones;
+    if (rp.positive) return launch_stages<5, true>(rp, a, s);
     switch (rp.r0c) {
         case 0: case 1: return launch_stages<0>(rp, a, s);
         case 2: return launch_stages<2>(rp, a, s);

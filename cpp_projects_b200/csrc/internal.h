@@ -228,8 +228,9 @@ bool build_seg_plan(const FdmtPlanHost& p, int l0, int l1, int rows, int tile, s
 // floats each, then its -0.0 row.  Each buffer's -0.0 row is long enough for
 // a read of its last row that runs past the row's end (columns no written
 // sample depends on).
-// Input segments (r0c > 0): the input rows are channels and an input of
-// stage 1 is a level-0 row of one: entry bits 20.. give its row number r, the
+// Input segments (r0c > 0; Keith plans, and Pravir plans with delays 0, 1,
+// 2, .. per channel): the input rows are channels and an input of stage 1 is
+// a level-0 row of one: entry bits 20.. give its row number r, the
 // running mean over r + 1 samples is formed where it is read.
 // ---------------------------------------------------------------------------
 constexpr int kRunMidChunks = 9;                  // 32-column chunks of a mid row
@@ -248,7 +249,9 @@ struct RunTile {                 // device-side
 struct RunPlan {
     int l0 = 0, l1 = 0;
     int s1 = 0, s2 = 0;          // levels merged by each stage (0: no plan)
-    int r0c = 0;                 // input segment: level-0 rows per channel
+    int r0c = 0;                 // input segment: most level-0 rows of a channel
+    bool positive = false;       // input segment of a Pravir plan: its window sums start at +0,
+                                 // so a channel's -0.0 counts as +0
     int pitch_x = 0;             // floats per row of X
     int zero_x = 0, zero_y = 0;  // offsets of the -0.0 rows
     int y0 = 0, ent0 = 0;        // offsets of Y and of the two staged entry buffers

@@ -378,10 +378,25 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
                     bool from_input) {
     const int m = l1 - l0;
     if (m < 2 || m > 4 || l0 < 0 || l1 > p.niter || G < 1) return false;
-    const int r0c = p.rows_per_chan0;
-    if (from_input && (p.kind != BFS_PLAN_KEITH || l0 != 0 || r0c < 1 || r0c > 5)) return false;
+    const std::vector<int>& ccum = p.lv[0].cum;   // level-0 rows by channel
+    int r0c = 0;
+    if (from_input) {
+        if (l0 != 0) return false;
+        for (int c = 0; c < p.nchan; ++c) {
+            r0c = std::max(r0c, ccum[c + 1] - ccum[c]);
+            // row r of a channel is its mean over r + 1 samples
+            for (int i = ccum[c]; p.kind == BFS_PLAN_PRAVIR && i < ccum[c + 1]; ++i)
+                if (p.dt0[i] != i - ccum[c]) return false;
+        }
+        if (r0c < 1 || r0c > 5) return false;
+    }
+    auto chan_of = [&](int row) {
+        if (p.kind == BFS_PLAN_KEITH) return row / r0c;
+        return static_cast<int>(std::upper_bound(ccum.begin(), ccum.end(), row) - ccum.begin()) - 1;
+    };
     RunPlan s;
-    s.l0 = l0; s.l1 = l1; s.s1 = m >= 3 ? 2 : 1; s.s2 = m - s.s1; s.r0c = from_input ? r0c : 0;
+    s.l0 = l0; s.l1 = l1; s.s1 = m >= 3 ? 2 : 1; s.s2 = m - s.s1; s.r0c = r0c;
+    s.positive = from_input && p.kind == BFS_PLAN_PRAVIR;
     const int lm = l1 - s.s2;
     struct Leaf { int row, shift; };             // row -1: the -0.0 row
     struct Row { int row, lo, hi; };             // needs samples t0 - hi .. t0 + kSegTile - lo
@@ -462,8 +477,12 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
             leaves(lm, r.row, s.s1, v);
             for (const Leaf& x : v) {
                 if (x.row < 0) continue;
-                if (from_input) add(t.in, x.row / r0c, r.lo + x.shift, r.hi + x.shift + x.row % r0c);
-                else add(t.in, x.row, r.lo + x.shift, r.hi + x.shift);
+                if (from_input) {
+                    const int c = chan_of(x.row);
+                    add(t.in, c, r.lo + x.shift, r.hi + x.shift + x.row - ccum[c]);
+                } else {
+                    add(t.in, x.row, r.lo + x.shift, r.hi + x.shift);
+                }
             }
         }
         unite(t.in);
@@ -503,7 +522,7 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         for (int i = 0; i < 4; ++i) {
             int e = zero * 4;
             if (v[i].row >= 0) {
-                const int src = chan ? v[i].row / r0c : v[i].row, r = chan ? v[i].row % r0c : 0;
+                const int src = chan ? chan_of(v[i].row) : v[i].row, r = chan ? v[i].row - ccum[src] : 0;
                 const int j = slot_of(from, src);
                 const int off = from[j].hi - hi - v[i].shift;
                 if (off < r || off + kSegTile > pitch) return false;

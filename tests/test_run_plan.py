@@ -145,6 +145,22 @@ def test_search_shapes_run_in_two_ctas_per_sm(nchan, levels):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("case", [(64, 1000, 64, 1, 0), (96, 701, 96, 1, 0), (33, 515, 100, 1, 0), (128, 2050, 50, 1, 0),
+                                  (1024, 3001, 1024, 1, 0), (64, 900, 64, 2, 0), (64, 900, 64, 1, 3)])
+def test_pravir_plans_bit_exact_vs_oracle(cuda, case):
+    """Delays 0, 1, 2, .. per channel form level 0 on chip, other grids in a plane."""
+    import torch
+    from cpp_projects_b200.fdmt import FDMTGPU
+    nchan, ncols, max_dt, step, lo = case
+    x = np.random.default_rng(nchan + ncols).standard_normal((nchan, ncols)).astype(np.float32)
+    x[:, ::7] = np.float32(-0.0)
+    x[::3, 5::11] = np.float32(-1e-40)
+    got = FDMTGPU(1200.0, 1600.0, nchan, ncols, 1e-3, max_dt, step, lo)(torch.from_numpy(x).to(cuda)).cpu().numpy()
+    want = pyoracle.pravir_fdmt(1200.0, 1600.0, x, nchan, ncols, max_dt, step, lo)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("case", CASES + [(1024, 4099, 1024, 4), (512, 20000, 512, 3), (256, 60001, 256, 4)])
 @pytest.mark.parametrize("shift", [0, 1])   # input base on and off a 16-byte boundary
 def test_run_segments_bit_exact_vs_oracle(cuda, case, shift):
