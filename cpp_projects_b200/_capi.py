@@ -100,6 +100,7 @@ _SIGNATURES = {
     "bfs_fdmt_autotune_desc": (_I, [ctypes.POINTER(FdmtDesc), ctypes.POINTER(FdmtDesc), ctypes.POINTER(_F)]),
     "bfs_fdmt_plan_passes": (_I, [_P, ctypes.POINTER(_I), _P, _I]),
     "bfs_fdmt_plan_segment": (_I, [_P, _I, _P, _I, _P, _I]),
+    "bfs_fdmt_plan_adjoint_run": (_I, [_P, _I, _P, _P, _I, _P, _I, _P, _I]),
     "bfs_fdmt_plan_run": (_I, [_P, _I, _P, _P, _I, _P, _I, _P, _I]),
     "bfs_fdmt_plan_destroy": (_I, [_P]),
     "bfs_fdmt_plan_info": (_I, [_P, ctypes.POINTER(FdmtInfo)]),

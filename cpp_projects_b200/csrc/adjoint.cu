@@ -29,9 +29,13 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <map>
+#include <mutex>
 
 #include "fdmt_plan.h"
 #include "internal.h"
+#include "row_ops.cuh"
 
 namespace bfs {
 namespace {
@@ -264,6 +268,259 @@ k_fdmt_adj_level0(const float* __restrict__ gout, float* __restrict__ gx, const 
     }
 }
 
+// ---- adjoint run segments (layout and blob: AdjRun, internal.h) ---------------
+constexpr int kAdjRunThreads = 256;
+constexpr int kAdjRunWarps = kAdjRunThreads / 32;
+
+struct AdjRunArgs {
+    const float* in;      // gradient of level l1
+    float* out;           // of level l0, or of the channels (FINAL)
+    const AdjTile* tiles;
+    const int2* rows;
+    const int* blob;
+    int ncols, in_pitch, out_pitch, nrt, total;
+    int pitch_x, y0, blob0, max_blob;
+    int vec;              // the input rows' windows start on 16-byte boundaries
+};
+
+// A row's sum over K chunks; `at` = the index of its terms in B (a multiple of
+// 4) | its kind.  Most rows are two inner sums of two terms, or of one, whose
+// loads are all issued before the first add; the others take their terms one
+// by one.  (x + 0 turns -0 into the +0 that the sums start from.)
+template <int K>
+__device__ __forceinline__ void sum_terms(float (&acc)[K], const int* B, int at, const char* lane_base) {
+    const int4* q4 = reinterpret_cast<const int4*>(B + (at & ~3));
+    const int4 f = *q4;
+    const int kind = at & 3;
+    if (kind == kAdjPairs || kind == kAdjOnes) {
+        float v[4][K];
+        load_row<K>(v[0], lane_base + (f.x & 0xffffc));
+        load_row<K>(v[1], lane_base + (f.y & 0xffffc));
+        if (kind == kAdjPairs) {
+            load_row<K>(v[2], lane_base + (f.z & 0xffffc));
+            load_row<K>(v[3], lane_base + (f.w & 0xffffc));
+            add_rows<K>(v[0], v[0], v[1]);
+            add_rows<K>(v[1], v[2], v[3]);
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[0][k] = __fadd_rn(v[0][k], 0.0f);
+        add_rows<K>(acc, v[0], v[1]);
+        return;
+    }
+    float part[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] = part[k] = 0.0f;
+    if (kind == kAdjZero) return;
+    const int* t = B + (at & ~3);
+    int q = f.x;
+#pragma unroll 1
+    for (bool more = true; more;) {
+        const int cur = q;
+        q = *++t;
+        more = (cur & kAdjEnd) == 0;
+        float v[K];
+        load_row<K>(v, lane_base + (cur & 0xffffc));
+        add_rows<K>(part, part, v);
+        if (cur & 1) {
+            add_rows<K>(acc, acc, part);
+#pragma unroll
+            for (int k = 0; k < K; ++k) part[k] = 0.0f;
+        }
+    }
+}
+
+// A channel's gradient: per level-0 row r' the sum w of its value g at
+// offsets 0..r' (only samples u + r >= r' where the window reaches them),
+// times RN(1 / (r' + 1)), rows in ascending order.  u0 = this lane's first
+// sample.
+template <int K>
+__device__ __forceinline__ void sum_channel(float (&gx)[K], const int* B, int at, const char* lane_base, int u0,
+                                            bool edge) {
+    float part[K], g[K], w[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) gx[k] = part[k] = g[k] = w[k] = 0.0f;
+    if ((at & 3) == kAdjZero) return;
+    const int* t = B + (at & ~3);
+    int q = *t;
+#pragma unroll 1
+    for (bool more = true; more;) {
+        const int cur = q;
+        q = *++t;
+        more = (cur & kAdjEnd) == 0;
+        float v[K];
+        load_row<K>(v, lane_base + (cur & 0xffffc));
+        add_rows<K>(part, part, v);
+        if (cur & 1) {
+            add_rows<K>(g, g, part);
+#pragma unroll
+            for (int k = 0; k < K; ++k) part[k] = 0.0f;
+        }
+        if (cur & 2) {
+            const int rr = (cur >> 20) & 7, r = (cur >> 23) & 7;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                if (!edge || u0 + 32 * k + r >= rr) w[k] = __fadd_rn(w[k], g[k]);
+                g[k] = 0.0f;
+            }
+            if (cur & (1 << 26)) {
+                const float rcp = __frcp_rn(static_cast<float>(rr + 1));
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    gx[k] = __fadd_rn(gx[k], __fmul_rn(w[k], rcp));
+                    w[k] = 0.0f;
+                }
+            }
+        }
+    }
+}
+
+// Persistent, two CTAs per SM, tiles and copies as in k_fdmt_run (the next
+// tile's input is copied into X while stage 2 reads Y); a warp forms whole
+// rows, its share of a stage's rows one after another.
+// What bounds it: shared-memory wavefronts, about four loads per row and pair
+// of levels and one store, and the loop over the rows that are not two pairs.
+// It replaces one gather pass over HBM per level: 1024 x 65536 0.568 ms
+// against 1.29 ms, 256 x 24485 60 us against 123 (its odd rows were read one
+// sample at a time).  Terms taken one by one for every row: 0.591; two terms
+// per turn of the loop: 0.642.
+template <bool FINAL>
+__global__ void __launch_bounds__(kAdjRunThreads, 2) k_adj_run(const AdjRunArgs a) {
+    constexpr int K1 = kRunMidChunks, K2 = kRunOutChunks;
+    extern __shared__ __align__(16) float sm[];
+    const unsigned sbase = static_cast<unsigned>(__cvta_generic_to_shared(sm));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const char* lane_base = reinterpret_cast<const char*>(sm) + 4 * lane;
+    auto tile_of = [&](int rt) {
+        const int4* p = reinterpret_cast<const int4*>(a.tiles + rt);
+        const int4 lo = __ldg(p), hi = __ldg(p + 1);
+        AdjTile t{};
+        t.row = lo.x; t.blob = lo.y; t.len = lo.z; t.n_in = lo.w; t.n1 = hi.x; t.n2 = hi.y; t.max_e = hi.z;
+        return t;
+    };
+    auto row_entries = [&](const AdjTile& t) {
+        const int j = warp + kAdjRunWarps * lane;
+        return j < t.n_in ? __ldg(a.rows + t.row + j) : make_int2(0, 0);
+    };
+    auto issue = [&](const AdjTile& t, int2 mine, int tt, int eb) {
+        const unsigned sb = sbase + 4u * (a.blob0 + eb * a.max_blob);
+        for (int i = threadIdx.x; i < (t.len >> 2); i += kAdjRunThreads) copy16(sb + 16u * i, a.blob + t.blob + 4 * i);
+        const int t0 = tt * kSegTile;
+        if (t0 >= a.ncols + t.max_e) return;   // every output of the tile is past the row's end
+        const int pieces = a.pitch_x >> 2;
+        for (int i = 0, j = warp; j < t.n_in; ++i, j += kAdjRunWarps) {
+            const int row = __shfl_sync(0xffffffffu, mine.x, i), lead = __shfl_sync(0xffffffffu, mine.y, i);
+            const int ts = t0 - lead;
+            const float* src = a.in + static_cast<size_t>(row) * a.in_pitch + ts;
+            float* d = sm + j * a.pitch_x;
+            const unsigned dst = sbase + 4u * (j * a.pitch_x);
+            if (ts >= a.ncols) {   // wholly past the end
+                for (int c = lane; c < pieces; c += 32) reinterpret_cast<float4*>(d)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else if (a.vec && ts >= 0 && ts + a.pitch_x <= a.ncols) {
+                const float* s0 = src + 4 * lane;
+                const unsigned d0 = dst + 16u * lane;
+                copy16(d0, s0);
+                copy16(d0 + 512u, s0 + 128);
+                if (lane + 64 < pieces) copy16(d0 + 1024u, s0 + 256);
+            } else {
+                for (int c = lane; c < a.pitch_x; c += 32) {
+                    if (ts + c >= 0 && ts + c < a.ncols) copy4(dst + 4u * c, src + c);
+                    else d[c] = 0.0f;
+                }
+            }
+        }
+    };
+    const int G = static_cast<int>(gridDim.x);
+    const int gq = G / a.nrt, gr = G % a.nrt;
+    int w = blockIdx.x;
+    int rt = w % a.nrt, tt = w / a.nrt;
+    AdjTile t = tile_of(rt);
+    issue(t, row_entries(t), tt, 0);
+    for (int eb = 0; w < a.total; eb ^= 1, w += G) {
+        const bool more = w + G < a.total;
+        int rn = rt + gr, tn = tt + gq;
+        if (rn >= a.nrt) { rn -= a.nrt; ++tn; }
+        if (!more) rn = rt;
+        const AdjTile next = tile_of(rn);
+        const int2 next_rows = row_entries(next);
+        copy_wait();
+        __syncthreads();   // X and the blob are in, every warp is done with Y
+        const int t0 = tt * kSegTile;
+        const bool live = t0 < a.ncols + t.max_e;
+        const int* B = reinterpret_cast<const int*>(sm) + a.blob0 + eb * a.max_blob;
+        if (live) {
+            const int r0 = t.n1 * warp / kAdjRunWarps, r1 = t.n1 * (warp + 1) / kAdjRunWarps;
+            char* dst = reinterpret_cast<char*>(sm + a.y0 + r0 * kRunMid) + 4 * lane;
+#pragma unroll 1
+            for (int r = r0; r < r1; ++r, dst += 4 * kRunMid) {
+                float o[K1];
+                sum_terms<K1>(o, B, B[r], lane_base);
+#pragma unroll
+                for (int k = 0; k < K1; ++k) *reinterpret_cast<float*>(dst + 128 * k) = o[k];
+            }
+        }
+        __syncthreads();   // Y is in, every warp is done with X
+        if (more) issue(next, next_rows, tn, eb ^ 1);
+        if (live) {
+            const int* H = B + t.n1;
+            const int r0 = t.n2 * warp / kAdjRunWarps, r1 = t.n2 * (warp + 1) / kAdjRunWarps;
+#pragma unroll 1
+            for (int r = r0; r < r1; ++r) {
+                const int row = H[3 * r], first = t0 - H[3 * r + 1];   // the window's first sample
+                if (first >= a.ncols || first + kSegTile <= 0) continue;
+                const int u0 = first + lane;
+                float o[K2];
+                if constexpr (FINAL) sum_channel<K2>(o, B, H[3 * r + 2], lane_base, u0, first < 8);
+                else sum_terms<K2>(o, B, H[3 * r + 2], lane_base);
+                float* dst = a.out + static_cast<size_t>(row) * a.out_pitch + u0;
+                if (first >= 0 && first + kSegTile <= a.ncols) {
+#pragma unroll
+                    for (int k = 0; k < K2; ++k) dst[32 * k] = o[k];
+                } else {
+#pragma unroll
+                    for (int k = 0; k < K2; ++k)
+                        if (u0 + 32 * k >= 0 && u0 + 32 * k < a.ncols) dst[32 * k] = o[k];
+                }
+            }
+        }
+        t = next;
+        rt = rn;
+        tt = tn;
+    }
+}
+
+template <bool FINAL>
+bfs_status launch_adj_run(const AdjRun& ar, const AdjRunArgs& args, cudaStream_t s) {
+    auto kern = k_adj_run<FINAL>;
+    // opt-in and resident CTAs as for the forward's run segments
+    static std::mutex mu;
+    static std::map<int, size_t> optin;
+    static std::map<std::pair<int, size_t>, int> resident;
+    int dev = 0;
+    BFS_CUDA(cudaGetDevice(&dev));
+    int ctas = 0;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        size_t& have = optin[dev];
+        if (have < ar.smem_bytes) {
+            BFS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(ar.smem_bytes)));
+            have = ar.smem_bytes;
+        }
+        auto it = resident.find({dev, ar.smem_bytes});
+        if (it == resident.end()) {
+            int per_sm = 0, sms = 0;
+            BFS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kAdjRunThreads, ar.smem_bytes));
+            BFS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            if (per_sm < 1) return fail(BFS_ERR_CUDA, "k_adj_run does not fit an SM");
+            it = resident.emplace(std::make_pair(dev, ar.smem_bytes), per_sm * sms).first;
+        }
+        ctas = it->second;
+    }
+    kern<<<std::min(args.total, ctas), kAdjRunThreads, ar.smem_bytes, s>>>(args);
+    BFS_LAUNCH_CHECK("k_adj_run");
+    return BFS_OK;
+}
+
 // Adjoint of a Pravir plan's level 0 (rows with delays dt_k per channel,
 // lvl0 = row cumsum then delays): the same window-mean transpose,
 //   gx[c][u] = sum_k RN(1/(dt_k+1)) * sum_{j=0..dt_k} [u+j >= dt_k][u+j < ncols] g0[k][u+j].
@@ -307,13 +564,20 @@ __global__ void k_snr_cells(const float* __restrict__ plane, int rows, int cols,
     snr[k] = __fdiv_rn(sum, __fsqrt_rn(static_cast<float>(w)));
 }
 
-// Gradient of sum_k gsnr[k] * S_k with respect to the plane: one CTA per
-// row; warp 0 collects the row's cells in cell order (ballot compaction,
-// up to kMaxCellsPerRow) and the row constants; then every sample of the
-// row is written (rows without cells get zeros).
+// Gradient of sum_k gsnr[k] * S_k with respect to the plane: each CTA writes
+// one of gridDim.y parts of a row; its warp 0 collects the row's cells in
+// cell order (ballot compaction, up to kMaxCellsPerRow) and the row constants;
+// then every sample of the part is written (rows without cells get zeros).
+// HBM-bound by the stores; a row with cells is a chain of loads and stores,
+// so it is cut into parts and each thread keeps four 16-byte groups (VEC:
+// rows 16-byte aligned) or four samples in flight.  1024 x 65536, 8 cells:
+// 184 us with one CTA per row and one sample at a time.
 constexpr int kMaxCellsPerRow = 512;
+constexpr int kSnrThreads = 256;
+constexpr int kSnrPart = 8192;   // samples per CTA
 
-__global__ void __launch_bounds__(256)
+template <bool VEC>
+__global__ void __launch_bounds__(kSnrThreads)
 k_snr_cells_adjoint(const float* __restrict__ plane, int rows, int cols, const float* __restrict__ stats,
                     const int* __restrict__ cells, int n, const float* __restrict__ snr,
                     const float* __restrict__ gsnr, float* __restrict__ gplane, int* __restrict__ err) {
@@ -365,14 +629,44 @@ k_snr_cells_adjoint(const float* __restrict__ plane, int rows, int cols, const f
     const float a = s_a, b = s_b;
     const float* y = plane + static_cast<size_t>(d) * cols;
     float* g = gplane + static_cast<size_t>(d) * cols;
-    for (int u = threadIdx.x; u < cols; u += blockDim.x) {
-        float v = 0.0f;
-        if (cnt > 0) {
-            v = a + b * (__ldg(y + u) - m);
-            for (int j = 0; j < cnt; ++j)
-                if (u >= s_t[j] && u < s_t[j] + s_w[j]) v += s_c[j];
+    const int beg = blockIdx.y * kSnrPart, end = min(cols, beg + kSnrPart);
+    auto value = [&](int u, float yu) {
+        float v = a + b * (yu - m);
+        for (int j = 0; j < cnt; ++j)
+            if (u >= s_t[j] && u < s_t[j] + s_w[j]) v += s_c[j];
+        return v;
+    };
+    constexpr int kStep = VEC ? 4 : 1, kFly = 4;
+    for (int u0 = beg + kStep * threadIdx.x; u0 < end; u0 += kStep * kFly * kSnrThreads) {
+        if constexpr (VEC) {   // (cols a multiple of 4: a group lies wholly inside or outside the row)
+            float4 q[kFly];
+#pragma unroll
+            for (int k = 0; k < kFly; ++k) {
+                const int u = u0 + 4 * k * kSnrThreads;
+                q[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (cnt > 0 && u < end) q[k] = __ldg(reinterpret_cast<const float4*>(y + u));
+            }
+#pragma unroll
+            for (int k = 0; k < kFly; ++k) {
+                const int u = u0 + 4 * k * kSnrThreads;
+                if (u >= end) break;
+                if (cnt > 0)
+                    q[k] = make_float4(value(u, q[k].x), value(u + 1, q[k].y), value(u + 2, q[k].z), value(u + 3, q[k].w));
+                *reinterpret_cast<float4*>(g + u) = q[k];
+            }
+        } else {
+            float q[kFly];
+#pragma unroll
+            for (int k = 0; k < kFly; ++k) {
+                const int u = u0 + k * kSnrThreads;
+                q[k] = cnt > 0 && u < end ? __ldg(y + u) : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < kFly; ++k) {
+                const int u = u0 + k * kSnrThreads;
+                if (u < end) g[u] = cnt > 0 ? value(u, q[k]) : 0.0f;
+            }
         }
-        g[u] = v;
     }
 }
 
@@ -395,17 +689,68 @@ size_t adjoint_ws_bytes(const FdmtPlanHost& h) {
     return align256(rows[0] * P * sizeof(float)) + align256(rows[1] * P * sizeof(float));
 }
 
+constexpr size_t kAdjRunSmem = 113 * 1024;   // two CTAs per SM
+
+// The plan's levels as adjoint run segments of two to four levels, from the
+// top down; empty where one does not fit (one gather pass per level then).
+// Outputs per tile: as many as fit; fewer where all tiles would run at once.
+void plan_adjoint_runs(const FdmtPlanHost& h, const AdjointTables& tab, std::vector<AdjRun>* out) {
+    out->clear();
+    if (h.niter < 2) return;
+    const int nseg = (h.niter + 3) / 4;
+    size_t rows[2];
+    adjoint_plane_rows(h, rows);
+    int l1 = h.niter;
+    for (int i = 0; i < nseg; ++i) {
+        const int l0 = l1 - (h.niter / nseg + (i < h.niter % nseg ? 1 : 0));
+        const bool final = l0 == 0 && h.kind == BFS_PLAN_KEITH && h.rows_per_chan0 <= 5;
+        if (!final && static_cast<size_t>(h.lv[l0].total_rows()) > rows[(nseg - 1 - i) & 1]) {
+            out->clear();
+            return;
+        }
+        const int in_pitch = l1 == h.niter ? h.ncols : plane_pitch4(h.ncols);
+        const long long tt = (h.ncols + kSegTile - 1) / kSegTile;
+        const int outputs = final ? h.nchan : h.lv[l0].total_rows();
+        std::vector<int> per_tile;
+        for (int G = 48; G >= 8; G -= 4)
+            if (G <= 12 || outputs / G * tt >= 2 * 148) per_tile.push_back(G);
+        AdjRun ar;
+        if (!build_adj_run(h, tab, l0, l1, final, per_tile, in_pitch, kAdjRunSmem, &ar)) {
+            out->clear();
+            return;
+        }
+        out->push_back(std::move(ar));
+        l1 = l0;
+    }
+}
+
 bfs_status ensure_adjoint_tables(bfs_fdmt_plan* p) {
-    if (p->d_adj_off) return BFS_OK;
-    if (!p->adj.built) build_adjoint_tables(p->host, &p->adj);
+    if (p->d_adj_tables) return BFS_OK;
+    if (!p->adj.built) {
+        build_adjoint_tables(p->host, &p->adj);
+        plan_adjoint_runs(p->host, p->adj, &p->adj_runs);
+    }
     const AdjointTables& A = p->adj;
-    BFS_CUDA(cudaMalloc(&p->d_adj_off, std::max<size_t>(1, A.off.size()) * sizeof(int)));
-    BFS_CUDA(cudaMalloc(&p->d_adj_ent, std::max<size_t>(1, A.ent.size() / 2) * sizeof(int2)));
-    if (!A.off.empty())
-        BFS_CUDA(cudaMemcpy(p->d_adj_off, A.off.data(), A.off.size() * sizeof(int), cudaMemcpyHostToDevice));
-    if (!A.ent.empty())
-        BFS_CUDA(cudaMemcpy(p->d_adj_ent, A.ent.data(), A.ent.size() * sizeof(int), cudaMemcpyHostToDevice));
-    return BFS_OK;
+    TableUpload up;
+    std::vector<int2> pairs;
+    std::vector<AdjTile> tiles;
+    std::vector<int> rows, blob;
+    p->adj_run0.clear();
+    for (const AdjRun& r : p->adj_runs) {
+        p->adj_run0.push_back({tiles.size(), rows.size(), blob.size()});
+        tiles.insert(tiles.end(), r.tiles.begin(), r.tiles.end());
+        rows.insert(rows.end(), r.rows.begin(), r.rows.end());
+        blob.insert(blob.end(), r.blob.begin(), r.blob.end());
+    }
+    up.add(&p->d_adj_tiles, tiles);
+    up.add(&p->d_adj_rows, rows);
+    up.add(&p->d_adj_blob, blob);
+    if (p->adj_runs.empty()) {   // one gather pass per level
+        for (size_t i = 0; i + 1 < A.ent.size(); i += 2) pairs.push_back(make_int2(A.ent[i], A.ent[i + 1]));
+        up.add(&p->d_adj_off, A.off);
+        up.add(&p->d_adj_ent, pairs);
+    }
+    return up.commit(&p->d_adj_tables);
 }
 
 bfs_status adjoint_run(bfs_fdmt_plan* p, const float* d_gy, float* d_gx, float* buf0, float* buf1,
@@ -414,6 +759,28 @@ bfs_status adjoint_run(bfs_fdmt_plan* p, const float* d_gy, float* d_gx, float* 
     const int T = h.ncols;
     const int P = plane_pitch4(T);
     float* bufs[2] = {buf0, buf1};
+    const size_t nrun = p->adj_runs.size();
+    for (size_t i = 0; i < nrun; ++i) {
+        const AdjRun& ar = p->adj_runs[i];
+        AdjRunArgs a;
+        a.in = i == 0 ? d_gy : bufs[(nrun - i) & 1];
+        a.out = ar.final ? d_gx : bufs[(nrun - 1 - i) & 1];
+        a.tiles = p->d_adj_tiles + p->adj_run0[i][0];
+        a.rows = reinterpret_cast<const int2*>(p->d_adj_rows + p->adj_run0[i][1]);
+        a.blob = p->d_adj_blob + p->adj_run0[i][2];
+        a.ncols = T;
+        a.in_pitch = i == 0 ? T : P;
+        a.out_pitch = ar.final ? T : P;
+        a.nrt = static_cast<int>(ar.tiles.size());
+        const long long total = static_cast<long long>(a.nrt) * ((T + ar.max_e + kSegTile - 1) / kSegTile);
+        BFS_ARG(total <= (1LL << 30), "too many adjoint tiles");
+        a.total = static_cast<int>(total);
+        a.pitch_x = ar.pitch_x; a.y0 = ar.y0; a.blob0 = ar.blob0; a.max_blob = ar.max_blob;
+        a.vec = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0 ? 1 : 0;
+        bfs_status st = ar.final ? launch_adj_run<true>(ar, a, s) : launch_adj_run<false>(ar, a, s);
+        if (st != BFS_OK) return st;
+    }
+    if (nrun > 0 && p->adj_runs.back().final) return BFS_OK;
     const int span = kAdjThreads * kAdjVecs;
     const int gy_blocks = ((T + 3) / 4 + span - 1) / span;
     BFS_ARG(gy_blocks <= 65535, "ncols too large for this build");
@@ -422,10 +789,10 @@ bfs_status adjoint_run(bfs_fdmt_plan* p, const float* d_gy, float* d_gx, float* 
     const int r0c = h.rows_per_chan0;
     const float* src1 = (h.niter == 1) ? d_gy : bufs[1];
     const int pitch1 = (h.niter == 1) ? T : P;
-    const bool fuse0 = h.kind == BFS_PLAN_KEITH && r0c >= 1 && r0c <= 5 && pitch1 % 4 == 0 &&
+    const bool fuse0 = nrun == 0 && h.kind == BFS_PLAN_KEITH && r0c >= 1 && r0c <= 5 && pitch1 % 4 == 0 &&
                        (reinterpret_cast<uintptr_t>(src1) & 15) == 0 &&
                        h.lv[0].total_rows() == h.nchan * r0c;
-    for (int l = h.niter; l >= (fuse0 ? 2 : 1); --l) {
+    for (int l = nrun > 0 ? 0 : h.niter; l >= (fuse0 ? 2 : 1); --l) {
         const float* src = (l == h.niter) ? d_gy : bufs[l & 1];
         float* dst = bufs[(l - 1) & 1];
         const int in_pitch = (l == h.niter) ? T : P;
@@ -483,6 +850,36 @@ bfs_status adjoint_run(bfs_fdmt_plan* p, const float* d_gy, float* d_gx, float* 
 
 using namespace bfs;
 
+extern "C" bfs_status bfs_fdmt_plan_adjoint_run(const bfs_fdmt_plan* plan, int pass, int* params, int* tiles,
+                                                int tiles_cap, int* rows, int rows_cap, int* blob, int blob_cap) {
+    BFS_ARG(plan != nullptr && params != nullptr, "null argument");
+    AdjointTables tab;
+    std::vector<AdjRun> runs;
+    build_adjoint_tables(plan->host, &tab);
+    plan_adjoint_runs(plan->host, tab, &runs);
+    params[0] = static_cast<int>(runs.size());
+    if (pass < 0 || pass >= params[0]) return BFS_OK;
+    const AdjRun& ar = runs[pass];
+    constexpr int ti = static_cast<int>(sizeof(AdjTile) / sizeof(int));
+    const int v[12] = {params[0], ar.l0, ar.l1, ar.final ? 1 : 0, ar.pitch_x, ar.y0, ar.blob0, ar.max_blob, ar.max_e,
+                       static_cast<int>(ar.tiles.size()), static_cast<int>(ar.rows.size() / 2),
+                       static_cast<int>(ar.blob.size())};
+    std::copy(v, v + 12, params);
+    if (tiles) {
+        BFS_ARG(tiles_cap >= ti * v[9], "tiles needs %d ints", ti * v[9]);
+        std::memcpy(tiles, ar.tiles.data(), ar.tiles.size() * sizeof(AdjTile));
+    }
+    if (rows) {
+        BFS_ARG(rows_cap >= 2 * v[10], "rows needs %d ints", 2 * v[10]);
+        std::copy(ar.rows.begin(), ar.rows.end(), rows);
+    }
+    if (blob) {
+        BFS_ARG(blob_cap >= v[11], "blob needs %d ints", v[11]);
+        std::copy(ar.blob.begin(), ar.blob.end(), blob);
+    }
+    return BFS_OK;
+}
+
 extern "C" bfs_status bfs_fdmt_adjoint_workspace_size(const bfs_fdmt_plan* plan, size_t* bytes) {
     BFS_ARG(plan != nullptr && bytes != nullptr, "null argument");
     *bytes = adjoint_ws_bytes(plan->host);
@@ -515,6 +912,14 @@ extern "C" bfs_status bfs_fdmt_adjoint(bfs_fdmt_plan* plan, const float* d_grad_
     if (st != BFS_OK) return st;
     size_t rows[2];
     adjoint_plane_rows(plan->host, rows);
+    if (!plan->adj_runs.empty()) {   // only the planes between the segments reach HBM
+        rows[0] = rows[1] = 0;
+        const size_t n = plan->adj_runs.size();
+        for (size_t i = 0; i < n; ++i)
+            if (!plan->adj_runs[i].final)
+                rows[(n - 1 - i) & 1] = std::max<size_t>(rows[(n - 1 - i) & 1],
+                                                         plan->host.lv[plan->adj_runs[i].l0].total_rows());
+    }
     const size_t P = plane_pitch4(plan->host.ncols);
     for (int b = 0; b < 2; ++b) {
         if (plan->d_adj_buf[b] || rows[b] == 0) continue;
@@ -546,13 +951,27 @@ extern "C" bfs_status bfs_boxcar_snr_cells_adjoint(const float* d_plane, int row
     BFS_ARG(d_plane && d_stats && d_gplane && (n == 0 || (d_cells && d_snr && d_gsnr)), "null argument");
     BFS_ARG(rows >= 1 && cols >= 1 && n >= 0, "bad shape");
     cudaStream_t s = as_stream(stream);
+    BFS_ARG((cols + kSnrPart - 1) / kSnrPart <= 65535, "ncols too large for this build");
+    const bool vec = cols % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_plane) | reinterpret_cast<uintptr_t>(d_gplane)) & 15) == 0;
+    const dim3 grid(rows, (cols + kSnrPart - 1) / kSnrPart);
+    auto launch = [&](int* err) {
+        if (vec)
+            k_snr_cells_adjoint<true><<<grid, kSnrThreads, 0, s>>>(d_plane, rows, cols, d_stats, d_cells, n, d_snr, d_gsnr,
+                                                                   d_gplane, err);
+        else
+            k_snr_cells_adjoint<false><<<grid, kSnrThreads, 0, s>>>(d_plane, rows, cols, d_stats, d_cells, n, d_snr, d_gsnr,
+                                                                    d_gplane, err);
+        return cudaGetLastError();
+    };
+    if (n <= kMaxCellsPerRow) {   // no row can hold too many: nothing to read back
+        BFS_CUDA(launch(nullptr));
+        return BFS_OK;
+    }
     int* err = nullptr;
     bfs_status st = stream_alloc(reinterpret_cast<void**>(&err), sizeof(int), s);
     if (st != BFS_OK) return st;
     BFS_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-    k_snr_cells_adjoint<<<rows, 256, 0, s>>>(d_plane, rows, cols, d_stats, d_cells, n, d_snr, d_gsnr,
-                                             d_gplane, err);
-    BFS_LAUNCH_CHECK("k_snr_cells_adjoint");
+    BFS_CUDA(launch(err));
     int h_err = 0;
     BFS_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
     BFS_CUDA(cudaFreeAsync(err, s));

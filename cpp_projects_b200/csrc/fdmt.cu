@@ -1574,27 +1574,25 @@ extern "C" bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc_in, bfs_fdm
     p->host_only = false;
     BFS_CUDA(cudaGetDevice(&p->device));
     const FdmtPlanHost& h = p->host;
+    TableUpload up;
     if (p->fuse_depth > 0) {
-        const HeadPlan& hp = p->head;
-        BFS_CUDA(cudaMalloc(&p->d_head_groups, hp.groups.size() * sizeof(HeadGroup)));
-        BFS_CUDA(cudaMemcpy(p->d_head_groups, hp.groups.data(),
-                            hp.groups.size() * sizeof(HeadGroup), cudaMemcpyHostToDevice));
-        BFS_CUDA(cudaMalloc(&p->d_head_tab, hp.tab.size() * sizeof(int)));
-        BFS_CUDA(cudaMemcpy(p->d_head_tab, hp.tab.data(), hp.tab.size() * sizeof(int),
-                            cudaMemcpyHostToDevice));
+        up.add(&p->d_head_groups, p->head.groups);
+        up.add(&p->d_head_tab, p->head.tab);
     }
-
     if (h.kind == BFS_PLAN_PRAVIR) {
         std::vector<int> l0(h.lv[0].cum.begin(), h.lv[0].cum.end());
         l0.insert(l0.end(), h.dt0.begin(), h.dt0.end());
-        BFS_CUDA(cudaMalloc(&p->d_lvl0, l0.size() * sizeof(int)));
-        BFS_CUDA(cudaMemcpy(p->d_lvl0, l0.data(), l0.size() * sizeof(int), cudaMemcpyHostToDevice));
+        up.add(&p->d_lvl0, l0);
     }
-    // device row tables; with 16-bit planes w packs the per-row scale exponents
-    const std::vector<std::vector<int>> ex = row_exponents(h);
+    // row tables of the plain levels; with 16-bit planes w packs the per-row
+    // scale exponents
+    std::vector<std::vector<int>> ex;
+    if (p->precision != BFS_PREC_F32) ex = row_exponents(h);
     std::vector<int4> tab;
     p->tab_off.assign(h.niter + 1, 0);
-    for (int l = 1; l <= h.niter; ++l) {
+    for (size_t i = 0; i < p->passes.size(); ++i) {
+        if (p->runs[i].s1 > 0 || !p->passes[i].tiles.empty()) continue;
+        const int l = p->passes[i].l1;
         p->tab_off[l] = tab.size();
         const FdmtLevel& L = h.lv[l];
         for (int g = 0; g < L.total_rows(); ++g) {
@@ -1608,51 +1606,33 @@ extern "C" bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc_in, bfs_fdm
             tab.push_back(make_int4(L.a_row[g], L.b_row[g], L.shift[g], w));
         }
     }
-    if (!tab.empty()) {
-        BFS_CUDA(cudaMalloc(&p->d_tab, tab.size() * sizeof(int4)));
-        BFS_CUDA(cudaMemcpy(p->d_tab, tab.data(), tab.size() * sizeof(int4),
-                            cudaMemcpyHostToDevice));
+    up.add(&p->d_tab, tab);
+    // every pass's tables, concatenated
+    std::vector<SegTile> tiles;
+    std::vector<RunTile> run_tiles;
+    std::vector<int> ent, run_rows, run_ent;
+    for (size_t i = 0; i < p->passes.size(); ++i) {
+        const RunPlan& rp = p->runs[i];
+        p->run_tile0.push_back(run_tiles.size());
+        p->run_row0.push_back(run_rows.size());
+        p->run_ent0.push_back(run_ent.size());
+        run_tiles.insert(run_tiles.end(), rp.tiles.begin(), rp.tiles.end());
+        run_rows.insert(run_rows.end(), rp.rows.begin(), rp.rows.end());
+        run_ent.insert(run_ent.end(), rp.ent.begin(), rp.ent.end());
+        const SegPlan& sp = p->passes[i];
+        p->seg_tile0.push_back(tiles.size());
+        p->seg_ent0.push_back(ent.size());
+        if (rp.s1 > 0) continue;
+        tiles.insert(tiles.end(), sp.tiles.begin(), sp.tiles.end());
+        ent.insert(ent.end(), sp.ent.begin(), sp.ent.end());
     }
-    // fused segments: every pass's tiles and entries, concatenated
-    {
-        std::vector<SegTile> tiles;
-        std::vector<int> ent;
-        p->seg_tile0.assign(p->passes.size(), 0);
-        p->seg_ent0.assign(p->passes.size(), 0);
-        for (size_t i = 0; i < p->passes.size(); ++i) {
-            p->seg_tile0[i] = tiles.size();
-            p->seg_ent0[i] = ent.size();
-            tiles.insert(tiles.end(), p->passes[i].tiles.begin(), p->passes[i].tiles.end());
-            ent.insert(ent.end(), p->passes[i].ent.begin(), p->passes[i].ent.end());
-        }
-        if (!tiles.empty()) {
-            BFS_CUDA(cudaMalloc(&p->d_seg_tiles, tiles.size() * sizeof(SegTile)));
-            BFS_CUDA(cudaMemcpy(p->d_seg_tiles, tiles.data(), tiles.size() * sizeof(SegTile),
-                                cudaMemcpyHostToDevice));
-            BFS_CUDA(cudaMalloc(&p->d_seg_ent, ent.size() * sizeof(int)));
-            BFS_CUDA(cudaMemcpy(p->d_seg_ent, ent.data(), ent.size() * sizeof(int), cudaMemcpyHostToDevice));
-        }
-    }
-    {
-        std::vector<RunTile> tiles;
-        std::vector<int> rows, ent;
-        for (const RunPlan& rp : p->runs) {
-            p->run_tile0.push_back(tiles.size());
-            p->run_row0.push_back(rows.size());
-            p->run_ent0.push_back(ent.size());
-            tiles.insert(tiles.end(), rp.tiles.begin(), rp.tiles.end());
-            rows.insert(rows.end(), rp.rows.begin(), rp.rows.end());
-            ent.insert(ent.end(), rp.ent.begin(), rp.ent.end());
-        }
-        if (!tiles.empty()) {
-            BFS_CUDA(cudaMalloc(&p->d_run_tiles, tiles.size() * sizeof(RunTile)));
-            BFS_CUDA(cudaMalloc(&p->d_run_rows, rows.size() * sizeof(int)));
-            BFS_CUDA(cudaMalloc(&p->d_run_ent, ent.size() * sizeof(int)));
-            BFS_CUDA(cudaMemcpy(p->d_run_tiles, tiles.data(), tiles.size() * sizeof(RunTile), cudaMemcpyHostToDevice));
-            BFS_CUDA(cudaMemcpy(p->d_run_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice));
-            BFS_CUDA(cudaMemcpy(p->d_run_ent, ent.data(), ent.size() * sizeof(int), cudaMemcpyHostToDevice));
-        }
-    }
+    up.add(&p->d_seg_tiles, tiles);
+    up.add(&p->d_seg_ent, ent);
+    up.add(&p->d_run_tiles, run_tiles);
+    up.add(&p->d_run_rows, run_rows);
+    up.add(&p->d_run_ent, run_ent);
+    st = up.commit(&p->d_tables);
+    if (st != BFS_OK) return st;
     // ping-pong planes (sized by build_passes); levels inside the fused head
     // or a fused segment never reach HBM
     p->external_ws = (desc->flags & BFS_FDMT_EXTERNAL_WS) != 0;

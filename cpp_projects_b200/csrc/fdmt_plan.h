@@ -3,9 +3,37 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
+#include <cstring>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
+
+namespace bfs {
+// Host tables gathered for one device allocation and one copy.
+class TableUpload {
+public:
+    template <typename T> void add(T** dst, const std::vector<T>& v) {
+        if (v.empty()) return;
+        const size_t at = (bytes_.size() + 255) & ~static_cast<size_t>(255);
+        bytes_.resize(at + v.size() * sizeof(T));
+        std::memcpy(bytes_.data() + at, v.data(), v.size() * sizeof(T));
+        refs_.push_back({reinterpret_cast<void**>(dst), at});
+    }
+    // *arena owns the memory (cudaFree); the added pointers address it
+    bfs_status commit(void** arena) {
+        if (bytes_.empty()) return BFS_OK;
+        BFS_CUDA(cudaMalloc(arena, bytes_.size()));
+        BFS_CUDA(cudaMemcpy(*arena, bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice));
+        for (auto& r : refs_) *r.first = static_cast<char*>(*arena) + r.second;
+        return BFS_OK;
+    }
+private:
+    std::vector<unsigned char> bytes_;
+    std::vector<std::pair<void**, size_t>> refs_;
+};
+}  // namespace bfs
 
 struct bfs_fdmt_plan {
     bfs::FdmtPlanHost host;
@@ -14,6 +42,7 @@ struct bfs_fdmt_plan {
     bool external_ws = false;
     int fuse_depth = 0;
     int precision = BFS_PREC_F32;      // storage of the planes between levels
+    void* d_tables = nullptr;          // owns the forward's tables (the pointers below into it)
     int4* d_tab = nullptr;             // per level, per output row: {a, b, shift, exps}
     std::vector<size_t> tab_off;       // offset of each level's table in d_tab
     void* d_buf[2] = {nullptr, nullptr};
@@ -40,24 +69,21 @@ struct bfs_fdmt_plan {
     // adjoint (built on the first adjoint call): per level l >= 1, for every
     // row of level l-1 the level-l rows that read it, as CSR {row, shift}
     bfs::AdjointTables adj;
+    void* d_adj_tables = nullptr;      // owns the adjoint's tables
     int* d_adj_off = nullptr;
     int2* d_adj_ent = nullptr;
+    std::vector<bfs::AdjRun> adj_runs;   // run segments from the top level down (empty: a pass per level)
+    bfs::AdjTile* d_adj_tiles = nullptr;
+    int* d_adj_rows = nullptr;
+    int* d_adj_blob = nullptr;
+    std::vector<std::array<size_t, 3>> adj_run0;  // per segment: offsets into the three arrays
     void* d_adj_buf[2] = {nullptr, nullptr};  // plan-owned adjoint planes (bfs_fdmt_adjoint)
     ~bfs_fdmt_plan() {
-        if (d_tab) cudaFree(d_tab);
-        if (d_head_groups) cudaFree(d_head_groups);
-        if (d_head_tab) cudaFree(d_head_tab);
-        if (d_lvl0) cudaFree(d_lvl0);
-        if (d_seg_tiles) cudaFree(d_seg_tiles);
-        if (d_seg_ent) cudaFree(d_seg_ent);
-        if (d_run_tiles) cudaFree(d_run_tiles);
-        if (d_run_rows) cudaFree(d_run_rows);
-        if (d_run_ent) cudaFree(d_run_ent);
+        if (d_tables) cudaFree(d_tables);
+        if (d_adj_tables) cudaFree(d_adj_tables);
         if (d_ones_tau) cudaFree(d_ones_tau);
         for (void* b : d_buf)
             if (b) cudaFree(b);
-        if (d_adj_off) cudaFree(d_adj_off);
-        if (d_adj_ent) cudaFree(d_adj_ent);
         for (void* b : d_adj_buf)
             if (b) cudaFree(b);
     }

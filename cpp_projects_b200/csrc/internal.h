@@ -92,6 +92,59 @@ struct AdjointTables {
 };
 void build_adjoint_tables(const FdmtPlanHost& p, AdjointTables* out);
 
+// ---------------------------------------------------------------------------
+// Adjoint run segment: the gradient of level l1 taken down to level l0 in one
+// pass over HBM, as two stages of one or two levels (S1 = l1 -> mid, S2 = mid
+// -> l0).  A row of a stage is a sum of shifted rows above it, nested as the
+// levels are: for two levels sum over the rows g that read it of (sum over
+// the rows h that read g of h[u + s_h]), each sum from +0 in ascending row
+// order; terms past ncols are zeros (x + 0 is x for every partial sum, none
+// of which is -0).  With `final` the outputs are channels: the level-0 rows'
+// running-mean adjoint is folded in, row r' of a channel being summed again
+// at each of its r' + 1 offsets.
+//
+// A level-l1 row is read at shift 0 by a tail row and at up to the whole
+// sub-band's delay by a head row, so a tile's output row i has a window of
+// its own, samples t0 - E_i .. t0 - E_i + kSegTile - 1 with E_i the least
+// total shift of its terms (a multiple of 8 below it): all windows of the
+// tile then read the level-l1 rows at [t0, t0 + kSegTile + a few).  Time tiles
+// run until t0 - E_i passes the row's end.  A tile holds the outputs whose
+// first reader lies in a cut of consecutive level-l1 rows (channels stay
+// whole).  X holds the level-l1 rows, pitch_x floats each, the row's window
+// starting `lead` samples before t0; Y the mid rows, kRunMid floats each.
+//
+// blob (ints, per tile, staged in shared memory): per mid row the index of its
+// terms | its kind, then {row, E, index | kind} per output, then the terms,
+// every row's from a multiple of 4: byte offset | 1 (last of an inner sum) |
+// 2 (final: last term of a level-0 row's value) | r' << 20 | r << 23 | 1 << 26
+// (last of row r') | kAdjEnd (last of the row).
+// ---------------------------------------------------------------------------
+enum { kAdjTerms = 0, kAdjPairs = 1, kAdjOnes = 2, kAdjZero = 3 };  // two sums of two / of one term; no term
+constexpr int kAdjEnd = 1 << 28;
+
+struct AdjTile {                 // device-side
+    int row;                     // first of its input rows
+    int blob;                    // first int of its blob (a multiple of 4)
+    int len;                     // ints of it, a multiple of 4
+    int n_in, n1, n2;
+    int max_e;                   // largest E
+    int pad;
+};
+
+struct AdjRun {
+    int l0 = 0, l1 = 0;
+    bool final = false;
+    int pitch_x = 0, y0 = 0, blob0 = 0, max_blob = 0, max_e = 0;
+    size_t smem_bytes = 0;
+    std::vector<AdjTile> tiles;
+    std::vector<int> rows;       // 2 ints per input row: {plane row, lead}
+    std::vector<int> blob;
+};
+// rows: outputs per tile, tried in order until one fits; in_pitch: floats per
+// level-l1 row (the caller's plane: ncols), which fixes the leads.
+bool build_adj_run(const FdmtPlanHost& p, const AdjointTables& t, int l0, int l1, bool final,
+                   const std::vector<int>& rows, int in_pitch, size_t smem_limit, AdjRun* out);
+
 // FDMT of 0/1 rows: every level-0 value of a 0/1 row is exactly 0 or 1 and
 // every merge adds integers, so output row d at sample t is exactly the
 // number of channels c with weight 1 whose total delay along the merge tree,

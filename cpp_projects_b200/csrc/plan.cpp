@@ -374,6 +374,26 @@ bool build_seg_plan(const FdmtPlanHost& p, int l0, int l1, int G, int TT, size_t
     return true;
 }
 
+// Tiles of at most G rows: sub-bands of more than G rows are cut into equal
+// parts, shorter ones taken together while they fit.
+static std::vector<std::pair<int, int>> row_cuts(const FdmtLevel& top, int G) {
+    std::vector<std::pair<int, int>> cuts;
+    for (int b = 0; b < top.nsub;) {
+        if (top.rows[b] > G) {
+            const int parts = (top.rows[b] + G - 1) / G;
+            for (int i = 0; i < parts; ++i)
+                cuts.push_back({top.cum[b] + top.rows[b] * i / parts, top.cum[b] + top.rows[b] * (i + 1) / parts});
+            ++b;
+            continue;
+        }
+        int e = b + 1;
+        while (e < top.nsub && top.cum[e + 1] - top.cum[b] <= G) ++e;
+        if (top.cum[e] > top.cum[b]) cuts.push_back({top.cum[b], top.cum[e]});
+        b = e;
+    }
+    return cuts;
+}
+
 bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_limit, RunPlan* out,
                     bool from_input) {
     const int m = l1 - l0;
@@ -429,23 +449,7 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         }
         v.resize(k);
     };
-    // tiles: sub-bands of more than G rows are cut into equal parts, shorter
-    // ones taken together while they fit
-    std::vector<std::pair<int, int>> cuts;
-    const FdmtLevel& top = p.lv[l1];
-    for (int b = 0; b < top.nsub;) {
-        if (top.rows[b] > G) {
-            const int parts = (top.rows[b] + G - 1) / G;
-            for (int i = 0; i < parts; ++i)
-                cuts.push_back({top.cum[b] + top.rows[b] * i / parts, top.cum[b] + top.rows[b] * (i + 1) / parts});
-            ++b;
-            continue;
-        }
-        int e = b + 1;
-        while (e < top.nsub && top.cum[e + 1] - top.cum[b] <= G) ++e;
-        cuts.push_back({top.cum[b], top.cum[e]});
-        b = e;
-    }
+    const std::vector<std::pair<int, int>> cuts = row_cuts(p.lv[l1], G);
     struct Tile { int g0, g1; std::vector<Row> mid, in; };
     std::vector<Tile> tiles;
     const std::vector<int>& mcum = p.lv[lm].cum;
@@ -453,7 +457,6 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
     for (const auto& c : cuts) {
         Tile t;
         t.g0 = c.first; t.g1 = c.second;
-        if (t.g0 == t.g1) continue;
         Leaf v[4];
         for (int g = t.g0; g < t.g1; ++g) {
             leaves(l1, g, s.s2, v);
@@ -587,6 +590,234 @@ void build_adjoint_tables(const FdmtPlanHost& p, AdjointTables* out) {
         out->ent.insert(out->ent.end(), ent.begin(), ent.end());
     }
     out->built = true;
+}
+
+bool build_adj_run(const FdmtPlanHost& p, const AdjointTables& tab, int l0, int l1, bool final,
+                   const std::vector<int>& rows, int in_pitch, size_t smem_limit, AdjRun* out) {
+    const int m = l1 - l0;
+    if (m < 2 || m > 4 || l0 < 0 || l1 > p.niter || (final && l0 != 0)) return false;
+    const int r0c = final ? p.rows_per_chan0 : 1;
+    if (final && (p.kind != BFS_PLAN_KEITH || r0c < 1 || r0c > 5)) return false;
+    const int lm = m >= 3 ? l1 - 2 : l1 - 1;
+    // a stage's terms: row i of level `lo` over the rows of level `hi` (one or
+    // two above), nested as the levels are
+    struct Term { int row, shift; bool last; };
+    struct Terms { std::vector<int> off; std::vector<Term> v; };
+    auto terms = [&](int lo, int hi) {
+        Terms t;
+        const int* off = tab.off.data() + tab.off_pos[lo + 1];
+        const int* ent = tab.ent.data() + 2 * tab.ent_pos[lo + 1];
+        const int n = p.lv[lo].total_rows();
+        t.off.reserve(n + 1);
+        for (int i = 0; i < n; ++i) {
+            t.off.push_back(static_cast<int>(t.v.size()));
+            for (int k = off[i]; k < off[i + 1]; ++k) {
+                const int g = ent[2 * k], s = ent[2 * k + 1];
+                if (hi == lo + 1) { t.v.push_back({g, s, true}); continue; }
+                const int* off2 = tab.off.data() + tab.off_pos[lo + 2];
+                const int* ent2 = tab.ent.data() + 2 * tab.ent_pos[lo + 2];
+                for (int q = off2[g]; q < off2[g + 1]; ++q)
+                    t.v.push_back({ent2[2 * q], s + ent2[2 * q + 1], q + 1 == off2[g + 1]});
+            }
+        }
+        t.off.push_back(static_cast<int>(t.v.size()));
+        return t;
+    };
+    const Terms up = terms(lm, l1), down = terms(l0, lm);
+    constexpr int kNone = 1 << 30;
+    // per mid row: least shift of its terms (kNone: no row reads it, its
+    // gradient is zero) and first row that reads it
+    const int nmid = p.lv[lm].total_rows();
+    std::vector<int> least(nmid, kNone), reader(nmid, kNone);
+    for (int g = 0; g < nmid; ++g)
+        for (int k = up.off[g]; k < up.off[g + 1]; ++k) {
+            least[g] = std::min(least[g], up.v[k].shift);
+            reader[g] = std::min(reader[g], up.v[k].row);
+        }
+    auto with_rows = [&](const int G) {
+        // outputs (level-l0 rows, or channels) by their first reader, those of a
+        // sub-band of level l1 in parts of at most G, small sub-bands together
+        const int units = final ? p.nchan : p.lv[l0].total_rows();
+        std::vector<std::pair<int, int>> order;   // {first reader, output}
+        std::vector<std::vector<int>> outs;
+        auto cut = [&](size_t i0, size_t i1, int parts) {
+            for (int k = 0; k < parts; ++k) {
+                std::vector<int> o;
+                for (size_t i = i0 + (i1 - i0) * k / parts; i < i0 + (i1 - i0) * (k + 1) / parts; ++i)
+                    o.push_back(order[i].second);
+                std::sort(o.begin(), o.end());
+                if (!o.empty()) outs.push_back(std::move(o));
+            }
+        };
+        size_t open = 0;     // start of the outputs not yet cut
+        int weight = 0;      // of their sub-bands: the larger of their output and level-l1 rows
+        for (int band = 0, i = 0; band < p.lv[l1].nsub; ++band) {
+            const size_t b0 = order.size();
+            const int end = p.lv[l0].cum[std::min(p.lv[l0].nsub, (band + 1) << m)];
+            for (; i < units && i * r0c < end; ++i) {
+                int key = kNone;
+                for (int r = i * r0c; r < (i + 1) * r0c; ++r)
+                    for (int k = down.off[r]; k < down.off[r + 1]; ++k) key = std::min(key, reader[down.v[k].row]);
+                order.push_back({key, i});
+            }
+            std::sort(order.begin() + b0, order.end());
+            const int w = std::max(static_cast<int>(order.size() - b0), p.lv[l1].rows[band]);
+            if (weight + w > G) {
+                if (b0 > open) cut(open, b0, 1);
+                open = b0;
+                weight = 0;
+            }
+            if (w > G) {
+                cut(open, order.size(), (w + G - 1) / G);
+                open = order.size();
+            } else {
+                weight += w;
+            }
+        }
+        if (order.size() > open) cut(open, order.size(), 1);
+        AdjRun s;
+        s.l0 = l0; s.l1 = l1; s.final = final;
+        struct Tile { std::vector<int> outs, e, mid, em, in; };
+        std::vector<Tile> tiles;
+        std::vector<int> mid_slot(nmid, -1), in_slot(p.lv[l1].total_rows(), -1), width;
+        int need_x = 0, max_in = 0, max_mid = 0;
+        for (auto& o : outs) {
+            Tile t;
+            t.outs = std::move(o);
+            // an output's window starts E before t0: the least shift of its terms
+            for (int i : t.outs) {
+                int e = kNone;
+                for (int r = i * r0c; r < (i + 1) * r0c; ++r)
+                    for (int k = down.off[r]; k < down.off[r + 1]; ++k)
+                        if (least[down.v[k].row] != kNone) e = std::min(e, down.v[k].shift + least[down.v[k].row]);
+                e = e == kNone ? 0 : e & ~7;
+                t.e.push_back(e);
+                s.max_e = std::max(s.max_e, e);
+                for (int r = i * r0c; r < (i + 1) * r0c; ++r)
+                    for (int k = down.off[r]; k < down.off[r + 1]; ++k) {
+                        const int g = down.v[k].row;
+                        if (least[g] == kNone) continue;
+                        if (mid_slot[g] < 0) {
+                            mid_slot[g] = static_cast<int>(t.mid.size());
+                            t.mid.push_back(g);
+                            t.em.push_back(-kNone);
+                        }
+                        int& em = t.em[mid_slot[g]];
+                        em = std::max(em, e - down.v[k].shift);
+                    }
+            }
+            width.assign(t.mid.size(), 0);
+            for (size_t j = 0; j < t.outs.size(); ++j)
+                for (int r = t.outs[j] * r0c; r < (t.outs[j] + 1) * r0c; ++r)
+                    for (int k = down.off[r]; k < down.off[r + 1]; ++k) {
+                        const int q = mid_slot[down.v[k].row];
+                        if (q >= 0) width[q] = std::max(width[q], kSegTile + down.v[k].shift + r % r0c - t.e[j] + t.em[q]);
+                    }
+            bool fits = true;
+            for (size_t q = 0; q < t.mid.size(); ++q) {
+                fits = fits && width[q] <= kRunMid;
+                for (int k = up.off[t.mid[q]]; k < up.off[t.mid[q] + 1]; ++k) {
+                    need_x = std::max(need_x, up.v[k].shift - t.em[q] + width[q]);
+                    int& slot = in_slot[up.v[k].row];
+                    if (slot < 0) {
+                        slot = 0;
+                        t.in.push_back(up.v[k].row);
+                    }
+                }
+            }
+            std::sort(t.in.begin(), t.in.end());
+            for (int g : t.mid) mid_slot[g] = -1;
+            for (int d : t.in) in_slot[d] = -1;
+            max_in = std::max(max_in, static_cast<int>(t.in.size()));
+            max_mid = std::max(max_mid, static_cast<int>(t.mid.size()));
+            if (!fits || 4ull * (static_cast<size_t>(max_in) * need_x + static_cast<size_t>(max_mid) * kRunMid) > smem_limit)
+                return false;
+            tiles.push_back(std::move(t));
+        }
+        s.pitch_x = (need_x + 3 + 3) & ~3;   // + the largest lead
+        if (s.pitch_x > kRunMaxPitch || max_in > 256) return false;
+        s.y0 = max_in * s.pitch_x + kRunMid;          // a mid row's read may run past the last input row
+        s.blob0 = s.y0 + max_mid * kRunMid + kSegTile;
+        std::vector<int> head, term;
+        for (const Tile& t : tiles) {
+            AdjTile r{};
+            r.row = static_cast<int>(s.rows.size() / 2);
+            r.blob = static_cast<int>(s.blob.size());
+            r.n_in = static_cast<int>(t.in.size());
+            r.n1 = static_cast<int>(t.mid.size());
+            r.n2 = static_cast<int>(t.outs.size());
+            for (int e : t.e) r.max_e = std::max(r.max_e, e);
+            for (size_t j = 0; j < t.in.size(); ++j) {
+                const int lead = static_cast<int>((static_cast<long long>(t.in[j]) * in_pitch) & 3);
+                in_slot[t.in[j]] = static_cast<int>(j) * s.pitch_x + lead;
+                s.rows.insert(s.rows.end(), {t.in[j], lead});
+            }
+            head.clear();
+            term.clear();
+            const int base = (r.n1 + 3 * r.n2 + 3) & ~3;
+            // closes a row's terms from `from` on: kind, end mark, padding
+            auto close = [&](size_t from, bool channel) {
+                const int at = base + static_cast<int>(from);
+                if (term.size() == from) return at | kAdjZero;
+                const size_t n = term.size() - from;
+                int kind = kAdjTerms;
+                if (!channel && n == 2 && (term[from] & 1)) kind = kAdjOnes;
+                if (!channel && n == 4 && !(term[from] & 1) && (term[from + 1] & 1) && !(term[from + 2] & 1)) kind = kAdjPairs;
+                term.back() |= kAdjEnd;
+                while (term.size() % 4) term.push_back(0);
+                return at | kind;
+            };
+            for (size_t q = 0; q < t.mid.size(); ++q) {
+                mid_slot[t.mid[q]] = static_cast<int>(q);
+                const size_t from = term.size();
+                for (int k = up.off[t.mid[q]]; k < up.off[t.mid[q] + 1]; ++k) {
+                    const Term& x = up.v[k];
+                    if (x.shift - t.em[q] < 0) return false;
+                    term.push_back(4 * (in_slot[x.row] + x.shift - t.em[q]) | (x.last ? 1 : 0));
+                }
+                head.push_back(close(from, false));
+            }
+            for (size_t j = 0; j < t.outs.size(); ++j) {
+                const int i = t.outs[j];
+                const size_t from = term.size();
+                for (int rr = 0; rr < r0c; ++rr)
+                    for (int rd = 0; rd <= (final ? rr : 0); ++rd) {
+                        int last = -1;   // last term of this value
+                        for (int k = down.off[i * r0c + rr]; k < down.off[i * r0c + rr + 1]; ++k) {
+                            const Term& x = down.v[k];
+                            const int q = mid_slot[x.row];
+                            if (q < 0) {   // a zero mid row: an inner sum's end mark moves to the term before
+                                if (x.last && last >= 0) term[last] |= 1;
+                                continue;
+                            }
+                            last = static_cast<int>(term.size());
+                            term.push_back(4 * (s.y0 + q * kRunMid + t.em[q] + x.shift - t.e[j] + rd) | (x.last ? 1 : 0));
+                        }
+                        if (last < 0) continue;   // the row's gradient is zero
+                        if (final) term[last] |= 3 | rr << 20 | rd << 23 | (rd == rr ? 1 << 26 : 0);
+                        else term[last] |= 1;
+                    }
+                head.insert(head.end(), {i, t.e[j], close(from, final)});
+            }
+            head.resize(base, 0);
+            head.insert(head.end(), term.begin(), term.end());
+            head.insert(head.end(), {0, 0, 0, 0});   // (the kernel reads ahead)
+            while (head.size() % 4) head.push_back(0);
+            r.len = static_cast<int>(head.size());
+            s.max_blob = std::max(s.max_blob, r.len);
+            s.blob.insert(s.blob.end(), head.begin(), head.end());
+            s.tiles.push_back(r);
+            for (int g : t.mid) mid_slot[g] = -1;
+            for (int d : t.in) in_slot[d] = -1;
+        }
+        s.smem_bytes = 4 * (static_cast<size_t>(s.blob0) + 2 * static_cast<size_t>(s.max_blob));
+        if (s.smem_bytes > smem_limit) return false;
+        *out = std::move(s);
+        return true;
+    };
+    for (int G : rows)
+        if (with_rows(G)) return true;
+    return false;
 }
 
 // ---------------------------------------------------------------------------

@@ -232,6 +232,13 @@ bfs_status bfs_fdmt_noalloc_scratch_bytes(const bfs_fdmt_plan* plan, size_t* nee
 bfs_status bfs_fdmt_adjoint(bfs_fdmt_plan* plan, const float* d_grad_out, float* d_grad_in,
                             void* stream);
 bfs_status bfs_fdmt_adjoint_workspace_size(const bfs_fdmt_plan* plan, size_t* bytes);
+/* Adjoint run segment `pass` (0 = from the top level), built from the plan's
+ * tables: params[12] = {segments (0: one gather pass per level), l0, l1,
+ * final, input-row pitch, offset of the mid rows, of the staged blobs, most
+ * ints of a blob, largest lead of an output, tiles, input rows, blob ints};
+ * tiles: 8 ints each, rows: 2 (each may be NULL). */
+bfs_status bfs_fdmt_plan_adjoint_run(const bfs_fdmt_plan* plan, int pass, int* params, int* tiles, int tiles_cap,
+                                     int* rows, int rows_cap, int* blob, int blob_cap);
 bfs_status bfs_fdmt_adjoint_ws(bfs_fdmt_plan* plan, const float* d_grad_out, float* d_grad_in,
                                void* d_workspace, size_t workspace_bytes, void* stream);
 
