@@ -44,7 +44,7 @@ long long boxcar_ordered_records(int rows, int cols);
 bfs_status launch_boxcar_ordered(const float* d_plane, int rows, int cols, const float* d_stats, float thr,
                                  const float* d_thr, int mode, int param, int snr_fast, bfs_cand* d_out,
                                  unsigned capacity, unsigned* d_count, unsigned* rec_first, unsigned* rec_count,
-                                 cudaStream_t s);
+                                 unsigned* work, unsigned* work_n, cudaStream_t s);
 bfs_status compact_ordered(const bfs_cand* src, const unsigned* rec_first, const unsigned* rec_count,
                            long long nrec, const long long* beam_rec, int nb, bfs_cand* dst, int* tags,
                            cudaStream_t s);
@@ -69,7 +69,7 @@ struct bfs_batch {
     bool ordered = false;
     long long nrec = 0;
     std::vector<long long> rec0;   // first record of each beam (+ the total)
-    unsigned* rec = nullptr;       // first[nrec], count[nrec]
+    unsigned* rec = nullptr;       // first[nrec], count[nrec], work list[nrec], its length per beam
     long long* d_beam_rec = nullptr;
     bfs_cand* sorted = nullptr;    // canonical order
     int* sorted_tags = nullptr;
@@ -251,7 +251,7 @@ extern "C" bfs_status bfs_batch_create(const bfs_batch_desc* desc, bfs_batch** o
         }
         b->rec0.push_back(b->nrec);
         BFS_ARG(b->nrec < (1ll << 31), "too many boxcar tiles in the batch (%lld)", b->nrec);
-        BFS_CUDA(cudaMalloc(&b->rec, sizeof(unsigned) * 2 * b->nrec));
+        BFS_CUDA(cudaMalloc(&b->rec, sizeof(unsigned) * (3 * b->nrec + b->beams.size())));
         BFS_CUDA(cudaMalloc(&b->d_beam_rec, sizeof(long long) * b->rec0.size()));
         BFS_CUDA(cudaMemcpy(b->d_beam_rec, b->rec0.data(), sizeof(long long) * b->rec0.size(),
                             cudaMemcpyHostToDevice));
@@ -309,7 +309,8 @@ static bfs_status beam_boxcar(bfs_batch* b, int i, const float* plane, const flo
     if (b->ordered)
         return launch_boxcar_ordered(plane, d.max_dt, d.ncols, stats, b->thr, nullptr, b->widths_mode,
                                      b->param, 0, b->cands, b->capacity, b->d_count, b->rec + b->rec0[i],
-                                     b->rec + b->nrec + b->rec0[i], s);
+                                     b->rec + b->nrec + b->rec0[i], b->rec + 2 * b->nrec + b->rec0[i],
+                                     b->rec + 3 * b->nrec + i, s);
     return launch_boxcar(plane, d.max_dt, d.ncols, stats, b->thr, nullptr, b->widths_mode, b->param, 0,
                          b->cands, b->capacity, b->d_count, s, i, b->tags);
 }
@@ -326,12 +327,21 @@ static bfs_status beam_stage1(bfs_batch* b, int i, const float* d_in, float* pla
     return beam_boxcar(b, i, plane, stats, s);
 }
 
+#define BFS_TRY_BATCH(x) do { bfs_status st_ = (x); if (st_ != BFS_OK) return st_; } while (0)
+
+// The candidate count and, on the ordered path, the beams' work-list lengths.
+static bfs_status clear_counts(bfs_batch* b, cudaStream_t s) {
+    BFS_CUDA(cudaMemsetAsync(b->d_count, 0, sizeof(unsigned), s));
+    if (b->ordered) BFS_CUDA(cudaMemsetAsync(b->rec + 3 * b->nrec, 0, sizeof(unsigned) * b->beams.size(), s));
+    return BFS_OK;
+}
+
 // Stage 1 for every beam, enqueued on s (captured or eager).
 // With several lanes the beams fork from s into the lanes' streams (branches of
 // the captured graph) and join back; the candidates of both lanes go to the
 // one candidate array (their order is set by the records or the sort).
 static bfs_status enqueue_stage1(bfs_batch* b, const float* const* d_inputs, cudaStream_t s) {
-    BFS_CUDA(cudaMemsetAsync(b->d_count, 0, sizeof(unsigned), s));
+    BFS_TRY_BATCH(clear_counts(b, s));
     if (!b->lane_s[0]) {
         for (size_t i = 0; i < b->beams.size(); ++i) {
             bfs_status st = beam_stage1(b, static_cast<int>(i), d_inputs[i], b->plane, b->stats, b->ws, s);
@@ -419,7 +429,7 @@ static bfs_status ensure_async(bfs_batch* b) {
     const size_t cap = b->capacity;
     BFS_CUDA(cudaMalloc(&b->cands_alt, cap * sizeof(bfs_cand)));
     if (!b->ordered) BFS_CUDA(cudaMalloc(&b->tags_alt, cap * sizeof(int)));
-    if (b->ordered) BFS_CUDA(cudaMalloc(&b->rec_alt, sizeof(unsigned) * 2 * b->nrec));
+    if (b->ordered) BFS_CUDA(cudaMalloc(&b->rec_alt, sizeof(unsigned) * (3 * b->nrec + b->beams.size())));
     BFS_CUDA(cudaMalloc(&b->d_count_alt, sizeof(unsigned)));
     BFS_CUDA(cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming));
     for (auto& e : b->ev_done) BFS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -466,7 +476,7 @@ extern "C" bfs_status bfs_batch_collect(bfs_batch* b, void* stream) {
 static bfs_status enqueue_host_stage1(bfs_batch* b, const float* const* h_inputs,
                                       float* const* d_inputs, cudaStream_t cs, cudaStream_t cp) {
     const int nb = static_cast<int>(b->beams.size());
-    BFS_CUDA(cudaMemsetAsync(b->d_count, 0, sizeof(unsigned), cs));
+    BFS_TRY_BATCH(clear_counts(b, cs));
     BFS_CUDA(cudaEventRecord(b->events[nb], cs));
     BFS_CUDA(cudaStreamWaitEvent(cp, b->events[nb], 0));
     for (int i = 0; i < nb; ++i) {

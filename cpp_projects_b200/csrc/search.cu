@@ -21,6 +21,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
 #include <cmath>
 
 #include "internal.h"
@@ -143,35 +144,54 @@ constexpr int kRegMaxW = 128;
 
 struct WidthConsts {
     float sq[kRegMaxW + 1];  // sqrtf(w), w = 1..kRegMaxW (index w)
+    // per filter class (window_class): 0.9999 sqrt(w) of its smallest width
+    // in the set, +inf when it holds none
+    float cls[8];
 };
 
+// ---- filter ---------------------------------------------------------------
+// Most tiles hold no window near the threshold, so a light kernel first finds
+// those that may.  With thr > 0 a window's S/N cannot pass while the sum of
+// its samples' positive parts is at most thr sqrt(w): the sequential sum is at
+// most the sequential sum of the positive parts (rounding is monotone), which
+// rounds up by at most 128 2^-24; the normalisation, the quotient and the sums
+// below add a few 2^-24, and 0.9999 covers all of it.  The positive parts are
+// those of v - mean, compared with std times the bound, so the filter needs no
+// division.  A window lies inside
+//   class 0 (w = 1) one sample, 1 (w = 2) two samples: the tile's largest;
+//   classes 2..7 (w <= 5, 9, 17, 33, 65, 129) 2, 3, 5, 9, 17, 33 neighbouring
+//   blocks of 4 samples, the 16-byte pieces the row is loaded in.
+// First the tile's largest block of 4 (twice, three times) and of 16 samples
+// (twice, three times) are compared with the bounds, which noise rarely
+// exceeds at 7 sqrt(w); only then the sums of neighbouring blocks.  NaNs count
+// as 0 (a window that holds one never passes), infinities exceed every bound.
+inline int window_class(int w) {
+    return w == 1 ? 0 : w == 2 ? 1 : w <= 5 ? 2 : w <= 9 ? 3 : w <= 17 ? 4 : w <= 33 ? 5 : w <= 65 ? 6 : 7;
+}
+
 // ---- ordered boxcar over row pairs -------------------------------------------
-// The register-blocked boxcar for two rows at once, writing the candidates
-// of every warp's tile as one block in canonical order.  Each warp owns
-// kPairWarpTile consecutive starts of rows 2y and 2y + 1 and stages them
-// (with the WMAX - 1 samples after them) interleaved in its own shared
-// region: position p holds {row 2y, row 2y + 1} at sample tw + p, so one
+// The exact search of the tiles the filter lists, writing the candidates of
+// every tile as one block in canonical order.  A CTA takes tiles of
+// kPairTile consecutive starts of rows 2y and 2y + 1 from the list and stages
+// them (with the WMAX - 1 samples after them) interleaved in shared memory:
+// position p holds {row 2y, row 2y + 1} at sample tw + p, normalised, so one
 // packed add.rn.f32x2 advances the running sums of both rows at one start —
 // each half is rounded as one __fadd_rn, so the sums are the reference's
-// sequential sums bit for bit.  Per width the warp first asks whether any
-// of its sums exceeds the width's lower bound of passing sums (a
-// three-input max tree and one vote); only then are exact quotients
-// evaluated.  The width loop keeps the passing windows as bits (start j,
-// width code c) -> bit 8 j + c, which orders them by (start, width), and
-// each one's S/N in a per-lane array indexed like its bit; a warp scan of
-// the lanes' counts and one atomicAdd give the warp its block (row 2y's
-// candidates, then row 2y + 1's), and each lane writes its windows at their
-// positions in the block from the bits.  The warps never wait for one
-// another.
-// Record (row, warp tile i) = {first index, count} of row `row`'s block in
-// warp tile i (index row * ceil(cols / kPairWarpTile) + i), so a scan of
-// the counts in record order gives every candidate its canonical position
-// (compact_ordered).
-constexpr int kPairStarts = 8;                            // starts per lane
-constexpr int kPairWarpTile = 32 * kPairStarts;           // starts per warp
+// sequential sums bit for bit.  Per width a warp first asks whether any of
+// its sums exceeds the width's lower bound of passing sums; only then are
+// exact quotients evaluated.  A lane's passing windows (start j, width code
+// c) are bits 8 j + c, which orders them by (start, width); a scan of the
+// counts over the CTA and one atomicAdd give the tile its block (row 2y's
+// candidates, then row 2y + 1's).  Listed tiles are the crowded ones: two
+// starts per lane keep a tile's chain of quotients and stores short (eight
+// per lane and a warp per tile: 45 us at 0.3 M candidates, 13 us now).
+// Record (row, tile i) = {first index, count} of row `row`'s block in tile i
+// (index row * ceil(cols / kPairTile) + i), so a scan of the counts in record
+// order gives every candidate its canonical position (compact_ordered).
+constexpr int kPairStarts = 2;                            // starts per lane
 constexpr int kPairWarps = 4;
 constexpr int kPairThreads = 32 * kPairWarps;
-constexpr int kPairTile = kPairWarps * kPairWarpTile;     // starts per CTA
+constexpr int kPairTile = kPairThreads * kPairStarts;     // starts per tile (256)
 
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
     unsigned long long d;
@@ -193,219 +213,351 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
     return d;
 }
 
-// Shared layout of a warp's staged tile: logical float4 f (positions 2f,
-// 2f + 1 of both rows) sits at f + f / 4, one float4 of padding after every
-// four, so the eight lanes of a quarter warp — whose windows start 4 float4s
-// apart — read eight different bank groups.
-__device__ __forceinline__ int pad4(int f) { return f + (f >> 2); }
-
 // The width loop of one lane: kPairStarts starts from tb in both rows (win4
-// = the warp's staged tile, f0 = the lane's first logical float4).  pass[r] gets bit 8 j + c
-// for every passing window (start j, width code c) of row r, and snr[64 r +
-// 8 j + c] its S/N.  edge: some window may leave the row (tested per window).
+// = the staged tile: float4 f holds positions 2f and 2f + 1 of both rows, f0
+// = the lane's first).  pass[r] gets bit 8 j + c for every passing window
+// (start j, width code c) of row r, and snr[r][8 j + c] its S/N.  edge: some
+// window may leave the row (tested per window).
 template <int MODE, int WMAX>
 __device__ __forceinline__ void pair_widths(const float4* __restrict__ win4, int f0, int tb, int cols, bool edge,
                                             float thr, float thr_lo, int snr_fast, const WidthConsts& wc,
-                                            unsigned long long (&pass)[2], float (&snr)[128]) {
+                                            unsigned (&pass)[2], float (&snr)[2][8 * kPairStarts]) {
     constexpr int S = kPairStarts;
     constexpr int kPos = S + WMAX - 1;   // positions this lane reads
     constexpr int kVec = (kPos + 1) / 2; // float4s (two positions each)
-    constexpr int kAhead = 4;            // window pairs are read this many steps before use
+    constexpr int kAhead = 6;            // window pairs are read this many steps before use
     unsigned long long win[2 * kVec];
     unsigned long long sum[S];
     constexpr int kPre = (S + kAhead + 1) / 2 < kVec ? (S + kAhead + 1) / 2 : kVec;
 #pragma unroll
     for (int v = 0; v < kPre; ++v) {
-        const float4 q = win4[pad4(f0 + v)];
+        const float4 q = win4[f0 + v];
         win[2 * v] = pack2(q.x, q.y);
         win[2 * v + 1] = pack2(q.z, q.w);
     }
 #pragma unroll
     for (int j = 0; j < S; ++j) sum[j] = 0ull;   // +0.0 in both halves
+    int code = -1;
 #pragma unroll
     for (int w = 1; w <= WMAX; ++w) {
         // step w reads positions w - 1 .. w + S - 2; the pair starting at
         // position w + S - 2 + kAhead is fetched now, kAhead steps early
         const int pn = w + S - 2 + kAhead;
         if ((pn & 1) == 0 && pn / 2 >= kPre && pn / 2 < kVec) {
-            const float4 q = win4[pad4(f0 + pn / 2)];
+            const float4 q = win4[f0 + pn / 2];
             win[pn] = pack2(q.x, q.y);
             win[pn + 1] = pack2(q.z, q.w);
         }
 #pragma unroll
         for (int j = 0; j < S; ++j) sum[j] = add2_rn(sum[j], win[j + w - 1]);
         if (MODE == 0 && (w & (w - 1)) != 0) continue;
+        ++code;   // log2 w, or w - 1
         const float sq = wc.sq[w];
         // RN(sum / sq) > thr needs sum > RN(RN(thr sq) (1 - 1e-5)) for thr > 0
         const float lim = thr_lo > -INFINITY ? __fmul_rn(__fmul_rn(thr, sq), 0.99999f) : -INFINITY;
-        float h[2 * S], hm[S];
+        float h[S][2], mx = -INFINITY;
 #pragma unroll
         for (int j = 0; j < S; ++j) {
-            unpack2(sum[j], h[2 * j], h[2 * j + 1]);
-            hm[j] = fmaxf(h[2 * j], h[2 * j + 1]);   // both rows at start j
+            unpack2(sum[j], h[j][0], h[j][1]);
+            mx = max3f(mx, h[j][0], h[j][1]);
         }
-        float mx = max3f(hm[0], hm[1], hm[2]);
-#pragma unroll
-        for (int k = 3; k + 1 < S; k += 2) mx = max3f(mx, hm[k], hm[k + 1]);
-        if (S % 2 == 0) mx = fmaxf(mx, hm[S - 1]);
         if (!__any_sync(0xffffffffu, mx > lim)) continue;
-        const int code = (MODE == 1) ? w - 1 : 31 - __clz(w);
         // windows inside the row: starts j < inside
         const int inside = edge ? cols - (tb + w - 1) : S;
-        // windows over the bound: a bit each (one code path for all of them)
-        unsigned over = 0;
 #pragma unroll
-        for (int k = 0; k < 2 * S; ++k)
-            if (h[k] > lim && (k >> 1) < inside) over |= 1u << k;
-#pragma unroll 1
-        while (over) {
-            const int k = __ffs(over) - 1;
-            over &= over - 1;
-            float sj = h[0];
+        for (int j = 0; j < S; ++j)
 #pragma unroll
-            for (int i = 1; i < 2 * S; ++i)
-                if (i == k) sj = h[i];
-            const float q = snr_fast ? __fdividef(sj, sq) : __fdiv_rn(sj, sq);
-            if (q > thr) {
-                const int r = k & 1, bit = 8 * (k >> 1) + code;
-                pass[r] |= 1ull << bit;
-                snr[64 * r + bit] = q;
+            for (int r = 0; r < 2; ++r) {
+                if (!(h[j][r] > lim) || j >= inside) continue;
+                const float q = snr_fast ? __fdividef(h[j][r], sq) : __fdiv_rn(h[j][r], sq);
+                if (q > thr) {
+                    pass[r] |= 1u << (8 * j + code);
+                    snr[r][8 * j + code] = q;
+                }
             }
-        }
     }
 }
 
 template <int MODE, int WMAX>
-__global__ void __launch_bounds__(kPairThreads, WMAX <= 8 ? 8 : WMAX <= 32 ? 6 : WMAX <= 64 ? 4 : 2)
+__global__ void __launch_bounds__(kPairThreads)
 k_boxcar_pair(const float* __restrict__ plane, int rows, int cols, const float* __restrict__ stats,
-              const float* __restrict__ d_thr, float thr_host, float thr_lo_host, int snr_fast, int vec,
+              const float* __restrict__ d_thr, float thr_host, float thr_lo_host, int snr_fast,
               bfs_cand* __restrict__ out, unsigned capacity, unsigned* __restrict__ d_count,
-              unsigned* __restrict__ rec_first, unsigned* __restrict__ rec_count, const WidthConsts wc) {
-    // staged positions of a warp: every start's windows, a multiple of 4
-    constexpr int kSpan = (kPairWarpTile + WMAX - 1 + 3) / 4 * 4;
-    constexpr int kF4 = kSpan / 2;                      // logical float4s (kSpan positions x 2 rows)
-    __shared__ float4 tile4[kPairWarps][kF4 + kF4 / 4]; // padded (pad4)
+              unsigned* __restrict__ rec_first, unsigned* __restrict__ rec_count,
+              const unsigned* __restrict__ work, const unsigned* __restrict__ work_n, const WidthConsts wc) {
+    // staged positions: every start's windows, a multiple of 4
+    constexpr int kSpan = (kPairTile + WMAX - 1 + 3) / 4 * 4;
+    __shared__ float4 t4[kSpan / 2 + 1];   // (a lane's last float4 may reach one past the span)
+    __shared__ unsigned s_warp[2][kPairWarps], s_first;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wt = blockIdx.x * kPairWarps + warp;     // warp tile
-    const int tw = wt * kPairWarpTile;
-    if (tw >= cols) return;                            // warp-uniform; no other warp is waited for
-    const int row0 = 2 * static_cast<int>(blockIdx.y);
-    const bool has1 = row0 + 1 < rows;
-    const float* x0 = plane + static_cast<size_t>(row0) * cols;
-    const float* x1 = has1 ? x0 + cols : x0;
-    float m0 = 0.0f, s0 = 1.0f, m1 = 0.0f, s1 = 1.0f;
-    if (stats) {
-        m0 = stats[row0]; s0 = stats[rows + row0];
-        if (has1) { m1 = stats[row0 + 1]; s1 = stats[rows + row0 + 1]; }
-    }
-    auto nz = [&](float v, float m, float s) { return stats ? norm_sample(v, m, s) : v; };
-    float4* t4 = tile4[warp];
-    float* tile = reinterpret_cast<float*>(t4);        // position p, row r at 4 pad4(p / 2) + 2 (p % 2) + r
-    const bool interior = tw + kSpan <= cols;
-    if (interior && vec) {
-        // 16-byte loads of both rows, every load in flight before the first use
-        constexpr int kQ = kSpan / 4;                   // float4s per row
-        constexpr int kPer = (kQ + 31) / 32;
-        float4 a[kPer], b[kPer];
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int q = lane + 32 * k;
-            if (k < kPer - 1 || q < kQ) {
-                a[k] = __ldg(reinterpret_cast<const float4*>(x0 + tw) + q);
-                b[k] = has1 ? __ldg(reinterpret_cast<const float4*>(x1 + tw) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int q = lane + 32 * k;
-            if (k < kPer - 1 || q < kQ) {
-                const float b0 = has1 ? nz(b[k].x, m1, s1) : 0.0f, b1 = has1 ? nz(b[k].y, m1, s1) : 0.0f;
-                const float b2 = has1 ? nz(b[k].z, m1, s1) : 0.0f, b3 = has1 ? nz(b[k].w, m1, s1) : 0.0f;
-                t4[pad4(2 * q)] = make_float4(nz(a[k].x, m0, s0), b0, nz(a[k].y, m0, s0), b1);
-                t4[pad4(2 * q + 1)] = make_float4(nz(a[k].z, m0, s0), b2, nz(a[k].w, m0, s0), b3);
-            }
-        }
-    } else if (interior) {
-        // 4-byte loads (rows not 16-byte aligned), all in flight first
-        constexpr int kPer = (kSpan + 31) / 32;
-        float a[kPer], b[kPer];
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int p = lane + 32 * k;
-            if (k < kPer - 1 || p < kSpan) {
-                a[k] = __ldg(x0 + tw + p);
-                b[k] = has1 ? __ldg(x1 + tw + p) : 0.0f;
-            }
-        }
-        float2* t2 = reinterpret_cast<float2*>(t4);
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int p = lane + 32 * k;
-            if (k < kPer - 1 || p < kSpan)
-                t2[2 * pad4(p >> 1) + (p & 1)] = make_float2(nz(a[k], m0, s0), has1 ? nz(b[k], m1, s1) : 0.0f);
-        }
-    } else {
-        for (int p = lane; p < kSpan; p += 32) {
-            const int t = tw + p;
-            const bool in = t < cols;
-            const int e = 4 * pad4(p >> 1) + 2 * (p & 1);
-            tile[e] = in ? nz(__ldg(x0 + t), m0, s0) : 0.0f;
-            tile[e + 1] = (in && has1) ? nz(__ldg(x1 + t), m1, s1) : 0.0f;
-        }
-    }
-    __syncwarp();
+    const unsigned nwork = __ldg(work_n);
+    const unsigned nwt = (cols + kPairTile - 1) / kPairTile;
     float thr = thr_host, thr_lo = thr_lo_host;
     if (d_thr) {
         thr = __ldg(d_thr);
         thr_lo = thr > 0.0f ? thr * 0.99999f : -INFINITY;
     }
-    const int p0 = lane * kPairStarts;
-    const int tb = tw + p0;
-    const int f0 = p0 / 2;
-    unsigned long long pass[2] = {0ull, 0ull};
-    float snr[128];   // S/N of the passing windows (indexed like their bits)
-    pair_widths<MODE, WMAX>(t4, f0, tb, cols, !interior, thr, thr_lo, snr_fast, wc, pass, snr);
-    if (!has1) pass[1] = 0ull;
+#pragma unroll 1
+    for (unsigned item = blockIdx.x; item < nwork; item += gridDim.x) {
+        const unsigned pt = __ldg(work + item);            // row pair * nwt + tile
+        const int wt = static_cast<int>(pt % nwt);
+        const int tw = wt * kPairTile;
+        const int row0 = 2 * static_cast<int>(pt / nwt);
+        const bool has1 = row0 + 1 < rows;
+        const float* x0 = plane + static_cast<size_t>(row0) * cols;
+        const float* x1 = has1 ? x0 + cols : x0;
+        float m0 = 0.0f, s0 = 1.0f, m1 = 0.0f, s1 = 1.0f;
+        if (stats) {
+            m0 = stats[row0]; s0 = stats[rows + row0];
+            if (has1) { m1 = stats[row0 + 1]; s1 = stats[rows + row0 + 1]; }
+        }
+        __syncthreads();   // every warp is done with the tile before
+        float2* t2 = reinterpret_cast<float2*>(t4);
+        constexpr int kPer = (kSpan + kPairThreads - 1) / kPairThreads;
+        float a[kPer], b[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int p = static_cast<int>(threadIdx.x) + kPairThreads * k;
+            const bool in = p < kSpan && tw + p < cols;
+            a[k] = in ? __ldg(x0 + tw + p) : 0.0f;
+            b[k] = in && has1 ? __ldg(x1 + tw + p) : 0.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int p = static_cast<int>(threadIdx.x) + kPairThreads * k;
+            if (p >= kSpan) continue;
+            const bool in = tw + p < cols;
+            t2[p] = make_float2(in && stats ? norm_sample(a[k], m0, s0) : a[k],
+                                in && has1 && stats ? norm_sample(b[k], m1, s1) : b[k]);
+        }
+        __syncthreads();
+        const int p0 = static_cast<int>(threadIdx.x) * kPairStarts;
+        const int tb = tw + p0;
+        unsigned pass[2] = {0u, 0u};
+        float snr[2][8 * kPairStarts];   // S/N of the passing windows (indexed like their bits)
+        pair_widths<MODE, WMAX>(t4, p0 / 2, tb, cols, tw + kSpan > cols, thr, thr_lo, snr_fast, wc, pass, snr);
+        if (!has1) pass[1] = 0u;
 
-    // the warp's block: row 0's candidates, then row 1's, lanes in order
-    const unsigned c0 = __popcll(pass[0]), c1 = __popcll(pass[1]);
-    unsigned i0 = c0, i1 = c1;   // inclusive scans over the lanes
+        // the tile's block: row 0's candidates, then row 1's, threads in order
+        const unsigned c0 = __popc(pass[0]), c1 = __popc(pass[1]);
+        unsigned i01 = c0 | c1 << 16;   // inclusive scans over the lanes (at most 32 * 16 each)
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned u0 = __shfl_up_sync(0xffffffffu, i0, d), u1 = __shfl_up_sync(0xffffffffu, i1, d);
-        if (lane >= d) { i0 += u0; i1 += u1; }
-    }
-    const unsigned tot0 = __shfl_sync(0xffffffffu, i0, 31), tot1 = __shfl_sync(0xffffffffu, i1, 31);
-    unsigned first = 0;
-    if (lane == 0) {
-        first = (tot0 + tot1) ? atomicAdd(d_count, tot0 + tot1) : 0u;
-        const int nwt = (cols + kPairWarpTile - 1) / kPairWarpTile;
-        const size_t rec = static_cast<size_t>(row0) * nwt + wt;
-        rec_first[rec] = first;
-        rec_count[rec] = tot0;
-        if (has1) {
-            rec_first[rec + nwt] = first + tot0;
-            rec_count[rec + nwt] = tot1;
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, i01, d);
+            if (lane >= d) i01 += u;
         }
-    }
-    if (tot0 + tot1 == 0) return;   // warp-uniform
-    first = __shfl_sync(0xffffffffu, first, 0);
+        if (lane == 31) { s_warp[0][warp] = i01 & 0xffffu; s_warp[1][warp] = i01 >> 16; }
+        __syncthreads();
+        unsigned before[2] = {0u, 0u}, tot[2] = {0u, 0u};
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        unsigned idx = first + (r ? tot0 + i1 - c1 : i0 - c0);
-        unsigned long long m = pass[r];
-        while (m) {   // bit order = (start, width) order
-            const int bit = __ffsll(static_cast<long long>(m)) - 1;
-            m &= m - 1;
-            if (idx < capacity) {
-                const int code = bit & 7;
-                bfs_cand c;
-                c.mt = tb + (bit >> 3); c.mdt = row0 + r; c.mwidth = MODE == 1 ? code + 1 : code;
-                c.msnr = snr[64 * r + bit];
-                out[idx] = c;
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int w = 0; w < kPairWarps; ++w) {
+                if (w < warp) before[r] += s_warp[r][w];
+                tot[r] += s_warp[r][w];
             }
-            ++idx;
+        if (tot[0] + tot[1] == 0) continue;   // CTA-uniform; its records are zero already
+        if (threadIdx.x == 0) {
+            const unsigned first = atomicAdd(d_count, tot[0] + tot[1]);
+            const size_t rec = static_cast<size_t>(row0) * nwt + wt;
+            rec_first[rec] = first;
+            rec_count[rec] = tot[0];
+            if (has1) {
+                rec_first[rec + nwt] = first + tot[0];
+                rec_count[rec + nwt] = tot[1];
+            }
+            s_first = first;
         }
+        __syncthreads();
+        unsigned idx[2] = {s_first + before[0] + (i01 & 0xffffu) - c0, s_first + tot[0] + before[1] + (i01 >> 16) - c1};
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (!pass[r]) continue;
+#pragma unroll
+            for (int bit = 0; bit < 8 * kPairStarts; ++bit) {   // bit order = (start, width) order
+                if (!(pass[r] >> bit & 1u)) continue;
+                if (idx[r] < capacity) {
+                    bfs_cand c;
+                    c.mt = tb + (bit >> 3); c.mdt = row0 + r; c.mwidth = MODE == 1 ? (bit & 7) + 1 : (bit & 7);
+                    c.msnr = snr[r][bit];
+                    out[idx[r]] = c;
+                }
+                ++idx[r];
+            }
+        }
+    }
+}
+
+// b[k] -> sums j blocks further on (block index lane + 32 k + j)
+template <int K>
+__device__ __forceinline__ void block_shift(float (&o)[K], const float (&b)[K], int j, int lane) {
+    float v[K + 1];
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = __shfl_sync(0xffffffffu, b[k], (lane + j) & 31);
+    v[K] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) o[k] = lane + j < 32 ? v[k] : v[k + 1];
+}
+
+__device__ __forceinline__ float warp_top(float v) {   // largest of non-negative floats
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+
+// Whether some window of a row may pass (warp-uniform), from its blocks'
+// samples q and their mean; bound = thr std.
+template <int WMAX, int K>
+__device__ __forceinline__ bool row_may_pass(const float4 (&q)[K], float m, float bound, const WidthConsts& wc, int lane) {
+    float b[K], big = 0.0f, b4 = 0.0f, b16 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const float x = fmaxf(__fsub_rn(q[k].x, m), 0.0f), y = fmaxf(__fsub_rn(q[k].y, m), 0.0f);
+        const float z = fmaxf(__fsub_rn(q[k].z, m), 0.0f), w = fmaxf(__fsub_rn(q[k].w, m), 0.0f);
+        b[k] = (x + y) + (z + w);
+        big = fmaxf(big, fmaxf(max3f(x, y, z), w));
+        if constexpr (WMAX >= 3) b4 = fmaxf(b4, b[k]);
+        if constexpr (WMAX >= 16) {
+            float s = b[k] + __shfl_xor_sync(0xffffffffu, b[k], 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            b16 = fmaxf(b16, s);
+        }
+    }
+    big = warp_top(big);
+    if (big > bound * wc.cls[0]) return true;
+    if constexpr (WMAX >= 2)
+        if (2.0f * big > bound * wc.cls[1]) return true;
+    if constexpr (WMAX >= 3) {
+        b4 = warp_top(b4);
+        bool near = 2.0f * b4 > bound * wc.cls[2];
+        if constexpr (WMAX >= 6) near |= 3.0f * b4 > bound * wc.cls[3];
+        if constexpr (WMAX >= 16) {
+            b16 = warp_top(b16);
+            near |= 2.0f * b16 > bound * wc.cls[4];
+            if constexpr (WMAX >= 32) near |= 3.0f * b16 > bound * wc.cls[5];
+            if constexpr (WMAX >= 64) near |= 5.0f * b16 > bound * wc.cls[6];
+            if constexpr (WMAX >= 128) near |= 9.0f * b16 > bound * wc.cls[7];
+        }
+        if (!near) return false;
+        bool over = false;
+        float sum[K], t[K];   // sums of 2, 4, 8, .. blocks
+        auto test = [&](int cls) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) over |= t[k] > bound * wc.cls[cls];
+        };
+        auto plus = [&](const float (&x)[K], int j) {   // t = sum + x shifted
+            block_shift<K>(t, x, j, lane);
+#pragma unroll
+            for (int k = 0; k < K; ++k) t[k] += sum[k];
+        };
+        auto keep = [&]() {
+#pragma unroll
+            for (int k = 0; k < K; ++k) sum[k] = t[k];
+        };
+#pragma unroll
+        for (int k = 0; k < K; ++k) sum[k] = b[k];
+        plus(b, 1);
+        test(2);
+        if constexpr (WMAX >= 6) {
+            keep();
+            plus(b, 2);
+            test(3);
+        }
+        if constexpr (WMAX >= 16) {
+            plus(sum, 2);
+            keep();
+            plus(b, 4);
+            test(4);
+        }
+        if constexpr (WMAX >= 32) {
+            plus(sum, 4);
+            keep();
+            plus(b, 8);
+            test(5);
+        }
+        if constexpr (WMAX >= 64) {
+            plus(sum, 8);
+            keep();
+            plus(b, 16);
+            test(6);
+        }
+        if constexpr (WMAX >= 128) {
+            plus(sum, 16);
+            keep();
+#pragma unroll
+            for (int k = 0; k < K; ++k) t[k] = sum[k] + (k + 1 < K ? b[k + 1] : 0.0f);   // 32 blocks further on
+            test(7);
+        }
+        return __any_sync(0xffffffffu, over);
+    }
+    return false;
+}
+
+// One warp per (row pair, warp tile): its records zeroed, and the tile put on
+// the work list when a window of one of its rows may pass (all of them with
+// thr <= 0).  Rows are read in 16-byte pieces of memory: where a row's samples
+// tw.. start `ph` floats into a piece, the samples before tw in it only raise
+// the sums.  Pieces that leave the row are read sample by sample, the mean
+// taken for what lies outside.  HBM-bound: 4096 x 45001 in 141 us (5.2 TB/s)
+// with 56 warps per SM, 178 us with 40; the whole search of that plane took
+// 330 us in one kernel, of a 512 x 32768 plane with 0.3 M candidates 89 us,
+// now 14.5 + 13 us.
+constexpr int kFilterThreads = 128;
+template <int WMAX>
+__global__ void __launch_bounds__(kFilterThreads, WMAX <= 32 ? 14 : 10)
+k_boxcar_filter(const float* __restrict__ plane, int rows, int cols, const float* __restrict__ stats,
+                const float* __restrict__ d_thr, float thr_host, unsigned* __restrict__ rec_count,
+                unsigned* __restrict__ work, unsigned* __restrict__ work_n, const WidthConsts wc) {
+    constexpr int kSpan = (kPairTile + WMAX - 1 + 3) / 4 * 4;
+    constexpr int kBlocks = kSpan / 4 + 1;
+    constexpr int kPer = (kBlocks + 31) / 32;
+    const unsigned nwt = (cols + kPairTile - 1) / kPairTile;
+    const unsigned wt = blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5);
+    if (wt >= nwt) return;   // warp-uniform
+    const int lane = threadIdx.x & 31, tw = static_cast<int>(wt) * kPairTile;
+    const unsigned pt = blockIdx.y * nwt + wt;
+    const int row0 = 2 * static_cast<int>(blockIdx.y);
+    const float thr = d_thr ? __ldg(d_thr) : thr_host;
+    const bool has1 = row0 + 1 < rows;
+    bool may = !(thr > 0.0f);
+    if (!may) {
+        float4 q[2][kPer];
+        float m[2] = {0.0f, 0.0f}, sd[2] = {1.0f, 1.0f};
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (r && !has1) continue;
+            if (stats) { m[r] = __ldg(stats + row0 + r); sd[r] = __ldg(stats + rows + row0 + r); }
+            const float* x = plane + static_cast<size_t>(row0 + r) * cols;
+            const int ph = static_cast<int>((reinterpret_cast<uintptr_t>(x + tw) >> 2) & 3);
+            if ((tw >= 4 || ph == 0) && tw + 4 * kBlocks <= cols) {   // no piece leaves the row
+#pragma unroll
+                for (int k = 0; k < kPer; ++k)
+                    if (k < kPer - 1 || lane + 32 * k < kBlocks)
+                        q[r][k] = __ldg(reinterpret_cast<const float4*>(x + tw + 4 * (lane + 32 * k) - ph));
+                    else
+                        q[r][k] = make_float4(m[r], m[r], m[r], m[r]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < kPer; ++k) {
+                    float f[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int t = tw + 4 * (lane + 32 * k) - ph + j;
+                        f[j] = t >= tw && t < min(cols, tw + kSpan) ? __ldg(x + t) : m[r];
+                    }
+                    q[r][k] = make_float4(f[0], f[1], f[2], f[3]);
+                }
+            }
+        }
+        // std 0 or NaN: every sample is 0; std beyond the bounds' range: not filtered
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+            if (!may && (r == 0 || has1) && sd[r] > 0.0f)
+                may = sd[r] < 1e-30f || sd[r] > 1e30f || row_may_pass<WMAX, kPer>(q[r], m[r], thr * sd[r], wc, lane);
+    }
+    if (lane == 0) {
+        const size_t rec = static_cast<size_t>(row0) * nwt + wt;
+        rec_count[rec] = 0u;
+        if (has1) rec_count[rec + nwt] = 0u;
+        if (may) work[atomicAdd(work_n, 1u)] = pt;
     }
 }
 
@@ -709,30 +861,42 @@ bool boxcar_ordered_supported(int mode, int param) {
 }
 
 long long boxcar_ordered_records(int rows, int cols) {
-    return static_cast<long long>(rows) * ((cols + kPairWarpTile - 1) / kPairWarpTile);
+    return static_cast<long long>(rows) * ((cols + kPairTile - 1) / kPairTile);
 }
 
 // The boxcar with canonical per-tile output (k_boxcar_pair): candidates go to
 // d_out in blocks, one per (row, warp tile), each in canonical order; records
 // rec_first / rec_count (boxcar_ordered_records entries, (row, tile) order)
-// locate the blocks for compact_ordered.
+// locate the blocks for compact_ordered.  work: one entry per row pair and
+// warp tile; *work_n: 0.
 bfs_status launch_boxcar_ordered(const float* d_plane, int rows, int cols, const float* d_stats, float thr,
                                  const float* d_thr, int mode, int param, int snr_fast, bfs_cand* d_out,
                                  unsigned capacity, unsigned* d_count, unsigned* rec_first, unsigned* rec_count,
-                                 cudaStream_t s) {
-    BFS_ARG(d_plane && d_count && rec_first && rec_count, "null argument");
+                                 unsigned* work, unsigned* work_n, cudaStream_t s) {
+    BFS_ARG(d_plane && d_count && rec_first && rec_count && work && work_n, "null argument");
     BFS_ARG(rows >= 1 && cols >= 1, "bad shape %dx%d", rows, cols);
     BFS_ARG((rows + 1) / 2 <= 65535, "rows > 131070 not supported");
     BFS_ARG(capacity == 0 || d_out, "d_out is null");
     BFS_ARG(boxcar_ordered_supported(mode, param), "width set (%d, %d) has no ordered kernel", mode, param);
     const float thr_lo = thr > 0.0f ? thr * 0.99999f : -INFINITY;
-    const int vec = (cols % 4 == 0) && (reinterpret_cast<uintptr_t>(d_plane) % 16 == 0);
     WidthConsts wc;
     for (int w = 0; w <= kRegMaxW; ++w) wc.sq[w] = std::sqrt(static_cast<float>(w));  // IEEE-correct on the host
-    const dim3 grid((cols + kPairTile - 1) / kPairTile, (rows + 1) / 2);
-#define BFS_BOX_PAIR(M, W) k_boxcar_pair<M, W><<<grid, kPairThreads, 0, s>>>(                               \
-        d_plane, rows, cols, d_stats, d_thr, thr, thr_lo, snr_fast, vec, d_out, capacity, d_count, rec_first, \
-        rec_count, wc)
+    for (float& c : wc.cls) c = INFINITY;
+    const int widest = mode == BFS_WIDTHS_POW2 ? 1 << param : param;
+    for (int w = 1; w <= widest; w = mode == BFS_WIDTHS_POW2 ? 2 * w : w + 1)
+        wc.cls[window_class(w)] = std::min(wc.cls[window_class(w)], 0.9999f * wc.sq[w]);
+    const long long pairs = boxcar_ordered_records((rows + 1) / 2, cols);
+    BFS_ARG(pairs < (1ll << 31), "too many boxcar tiles (%lld)", pairs);
+    constexpr int kPerCta = kFilterThreads / 32 * kPairTile;
+    const dim3 fgrid((cols + kPerCta - 1) / kPerCta, (rows + 1) / 2);
+    // the searching kernel's CTAs take the listed tiles in turn
+    const int grid = static_cast<int>(std::min<long long>(pairs, 148LL * 8));
+#define BFS_BOX_PAIR(M, W)                                                                                        \
+    k_boxcar_filter<W><<<fgrid, kFilterThreads, 0, s>>>(d_plane, rows, cols, d_stats, d_thr, thr, rec_count,     \
+                                                        work, work_n, wc);                                        \
+    k_boxcar_pair<M, W><<<grid, kPairThreads, 0, s>>>(d_plane, rows, cols, d_stats, d_thr, thr, thr_lo, snr_fast,  \
+                                                      d_out, capacity, d_count, rec_first, rec_count, work,        \
+                                                      work_n, wc)
     if (mode == BFS_WIDTHS_POW2) {
         switch (param) {
             case 0: BFS_BOX_PAIR(0, 1); break;
@@ -836,16 +1000,16 @@ extern "C" bfs_status bfs_boxcar_gather(const float* d_plane, int rows, int cols
     const bool ordered = boxcar_ordered_supported(widths_mode, param);
     const long long nrec = ordered ? boxcar_ordered_records(rows, cols) : 0;
     unsigned* d_count = nullptr;
-    unsigned* rec = nullptr;   // first[nrec], count[nrec]
-    BFS_TRY_ST(stream_alloc(reinterpret_cast<void**>(&d_count), sizeof(unsigned), s));
-    bfs_status st = ordered ? stream_alloc(reinterpret_cast<void**>(&rec), sizeof(unsigned) * 2 * nrec, s) : BFS_OK;
+    unsigned* rec = nullptr;   // first[nrec], count[nrec], work[nrec]
+    BFS_TRY_ST(stream_alloc(reinterpret_cast<void**>(&d_count), 2 * sizeof(unsigned), s));   // candidates, work entries
+    bfs_status st = ordered ? stream_alloc(reinterpret_cast<void**>(&rec), sizeof(unsigned) * 3 * nrec, s) : BFS_OK;
     if (st == BFS_OK) {
-        cudaError_t e = cudaMemsetAsync(d_count, 0, sizeof(unsigned), s);
+        cudaError_t e = cudaMemsetAsync(d_count, 0, 2 * sizeof(unsigned), s);
         if (e != cudaSuccess) st = fail(BFS_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
     }
     if (st == BFS_OK)
         st = ordered ? launch_boxcar_ordered(d_plane, rows, cols, d_stats, thr, d_thr, widths_mode, param, snr_fast,
-                                             d_out, capacity, d_count, rec, rec + nrec, s)
+                                             d_out, capacity, d_count, rec, rec + nrec, rec + 2 * nrec, d_count + 1, s)
                      : launch_boxcar(d_plane, rows, cols, d_stats, thr, d_thr, widths_mode, param,
                                      snr_fast, d_out, capacity, d_count, s, 0, nullptr);
     unsigned count = 0;
