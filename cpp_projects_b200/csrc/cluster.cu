@@ -208,7 +208,7 @@ bfs_status launch_select_delegates(const bfs_cand* c, const int* perm, unsigned 
     // a thread's positions are a chain of dependent loads: few of them until
     // the blocks fill the chip (0.3 M candidates: 19.5 us with 16)
     auto blocks = [&](unsigned per) { return (n + kLaneThreads * per - 1) / (kLaneThreads * per); };
-    if (blocks(16) >= 8 * 148)
+    if (blocks(16) >= 2 * 148)
         k_delegate_lanes<16><<<blocks(16), kLaneThreads, 0, s>>>(c, perm, static_cast<int>(n), offsets,
                                                                  static_cast<int>(ngroups), slots);
     else
@@ -309,21 +309,43 @@ __device__ __forceinline__ unsigned gap_group(const bfs_cand& c, unsigned g, con
 
 struct GapMaps { GapMap m[3]; };
 
-__global__ void k_gap_mark(const bfs_cand* __restrict__ c, const int* __restrict__ g0, unsigned n, GapMaps maps,
-                           int field, int fmin, int shift, unsigned words, unsigned* __restrict__ bits) {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned p = 0xffffffffu;
-    if (i < n) {
-        const bfs_cand v = c[i];
-        p = gap_cell(v, field, gap_group(v, g0 ? static_cast<unsigned>(__ldg(g0 + i)) : 0u, maps.m, field), fmin, shift);
+// Marks the cells of a CTA's contiguous share of the candidates.  Neighbours
+// lie in few words and the words of a bright pulse are hit by most of the
+// list, so a warp sets a word's bits with one atomic, and only where a small
+// table of the words this CTA has set does not hold them yet (with a look at
+// the word in L2 instead the hot words' lines were the bound: 126 us for 4 M
+// candidates, 13 us for 0.3 M).
+constexpr int kMarkCache = 1024;
+__global__ void __launch_bounds__(256)
+k_gap_mark(const bfs_cand* __restrict__ c, const int* __restrict__ g0, unsigned n, unsigned per_cta, GapMaps maps,
+           int field, int fmin, int shift, unsigned words, unsigned* __restrict__ bits) {
+    __shared__ unsigned long long known[kMarkCache];   // {word + 1, its bits}: one 8-byte access each
+    for (int i = threadIdx.x; i < kMarkCache; i += blockDim.x) known[i] = 0ull;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const unsigned beg = blockIdx.x * per_cta, end = min(n, beg + per_cta);
+    for (unsigned i0 = beg; i0 < end; i0 += blockDim.x) {   // CTA-uniform
+        const unsigned i = i0 + threadIdx.x;
+        unsigned w = 0xffffffffu, b = 0u;
+        if (i < end) {
+            const bfs_cand v = c[i];
+            const unsigned p =
+                gap_cell(v, field, gap_group(v, g0 ? static_cast<unsigned>(__ldg(g0 + i)) : 0u, maps.m, field), fmin, shift);
+            w = p >> 5;
+            b = 1u << (p & 31u);
+        }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {   // the lane's bits and those of the lanes after it in the same word
+            const unsigned uw = __shfl_down_sync(0xffffffffu, w, d), ub = __shfl_down_sync(0xffffffffu, b, d);
+            if (lane + d < 32 && uw == w) b |= ub;
+        }
+        const unsigned left = __shfl_up_sync(0xffffffffu, w, 1);
+        if (w >= words || (lane != 0 && left == w)) continue;
+        const unsigned long long k = *const_cast<volatile unsigned long long*>(known + (w & (kMarkCache - 1)));
+        if ((k >> 32) == w + 1ull && (static_cast<unsigned>(k) & b) == b) continue;
+        const unsigned old = atomicOr(bits + w, b);
+        *const_cast<volatile unsigned long long*>(known + (w & (kMarkCache - 1))) = (w + 1ull) << 32 | (old | b);
     }
-    // one atomic per warp and word (neighbouring candidates lie in few words),
-    // and none where the bits are set already
-    const unsigned w = p >> 5;
-    const unsigned same = __match_any_sync(0xffffffffu, w);
-    const unsigned b = __reduce_or_sync(same, 1u << (p & 31u));
-    if (i >= n || w >= words || (threadIdx.x & 31) != __ffs(same) - 1) return;
-    if ((__ldcg(bits + w) & b) != b) atomicOr(bits + w, b);
 }
 
 // keys of the final order: (group, width), ties by index
@@ -351,13 +373,37 @@ __global__ void k_gap_offsets(const K* __restrict__ keys, unsigned n, int wbits,
     if (i == 0) offsets[ng] = static_cast<int>(n);
 }
 
+// Stream-ordered scratch: pieces of one block allocated up front, more blocks
+// where it runs out.
 struct Scratch {
     cudaStream_t s;
     std::vector<void*> ptrs;
-    bfs_status alloc(void** p, size_t bytes) {
-        bfs_status st = stream_alloc(p, bytes, s);
+    char* at = nullptr;
+    size_t left = 0;
+    bfs_status reserve(size_t bytes) {
+        void* p = nullptr;
+        bfs_status st = stream_alloc(&p, bytes, s);
         if (st != BFS_OK) return st;
-        ptrs.push_back(*p);
+        ptrs.push_back(p);
+        at = static_cast<char*>(p);
+        left = bytes;
+        return BFS_OK;
+    }
+    bfs_status alloc(void** p, size_t bytes) {
+        const size_t need = (bytes + 255) & ~static_cast<size_t>(255);
+        if (need > left) {
+            char* keep = at;
+            const size_t kept = left;
+            bfs_status st = reserve(need);
+            if (st != BFS_OK) return st;
+            *p = at;
+            at = keep;
+            left = kept;
+            return BFS_OK;
+        }
+        *p = at;
+        at += need;
+        left -= need;
         return BFS_OK;
     }
     ~Scratch() { for (void* p : ptrs) cudaFreeAsync(p, s); }
@@ -377,7 +423,7 @@ extern "C" bfs_status bfs_select_delegates(const bfs_cand* d_cands, const int* d
     if (ngroups == 0) return BFS_OK;
     BFS_ARG(n > 0 && n < 0x7fffffffu, "bad candidate count %u", n);
     cudaStream_t s = as_stream(stream);
-    Scratch sc{s, {}};
+    Scratch sc{s};
     unsigned long long* slots;
     BFS_TRY(sc.alloc(reinterpret_cast<void**>(&slots),
                      sizeof(unsigned long long) * kDelegateLanes * ngroups));
@@ -485,7 +531,7 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
     GapMaps maps{};
     unsigned* total;
     BFS_TRY(sc.alloc(reinterpret_cast<void**>(&total), sizeof(unsigned)));
-    const int th = 256, bl = static_cast<int>((n + th - 1) / th);
+    const int th = 256;
     const unsigned long long most = std::max<unsigned long long>(1ull << 20, n);
     unsigned long long groups = groups0;   // before the pass, at most
     bool exact = true;
@@ -497,8 +543,7 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
         while (shift < 32 && (1ll << shift) <= range[f]) ++shift;
         if (!exact && (groups << (shift - 5)) > (1ull << 16)) {
             unsigned have = 0;
-            BFS_CUDA(cudaMemcpyAsync(&have, total, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-            BFS_CUDA(cudaStreamSynchronize(s));
+            BFS_TRY(read_back(&have, total, 1, s));
             groups = have;
             exact = true;
         }
@@ -524,7 +569,9 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
         bits = reinterpret_cast<unsigned*>(piece + at_bits);
         tmp = piece + at_tmp;
         BFS_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned) * words, s));
-        k_gap_mark<<<bl, th, 0, s>>>(d_cands, d_group0, n, maps, f, fmin[f], shift, words, bits);
+        const unsigned per_cta = std::max(1024u, ((n + 148 * 4 - 1) / (148 * 4) + 255u) & ~255u);
+        k_gap_mark<<<(n + per_cta - 1) / per_cta, 256, 0, s>>>(d_cands, d_group0, n, per_cta, maps, f, fmin[f], shift,
+                                                               words, bits);
         BFS_LAUNCH_CHECK("k_gap_mark");
         BFS_CUDA(cub::DeviceScan::ExclusiveScan(tmp, tmp_bytes, Words(Count(0u), GapWord{bits, rule.metric}), state, rule,
                                                 GapState{0u, 0u, 0u, 0u}, static_cast<int>(words), s));
@@ -535,8 +582,7 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
         exact = false;
     }
     unsigned ng = 0;
-    BFS_CUDA(cudaMemcpyAsync(&ng, total, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    BFS_CUDA(cudaStreamSynchronize(s));
+    BFS_TRY(read_back(&ng, total, 1, s));
     BFS_ARG(ng >= 1 && ng <= n, "bad group count %u", ng);
     const int wbits = bits_for(static_cast<unsigned long long>(range[2]));
     const int end_bit = wbits + bits_for(ng - 1);
@@ -570,7 +616,9 @@ extern "C" bfs_status bfs_cluster_grouped(const bfs_cand* d_cands, uint32_t n, c
     BFS_ARG(d_cands && d_perm && d_offsets && d_delegates, "null argument");
     BFS_ARG(n < 0x7fffffffu, "too many candidates");
     cudaStream_t s = as_stream(stream);
-    Scratch sc{s, {}};
+    Scratch sc{s};
+    // keys, values and the sort's own of the gap grouping, and its small tables
+    BFS_TRY(sc.reserve(sizeof(unsigned) * 4 * static_cast<size_t>(n) + (size_t(2) << 20)));
     const int th = 256;
     const int bl = static_cast<int>((n + th - 1) / th);
     // field ranges -> key widths
@@ -584,8 +632,7 @@ extern "C" bfs_status bfs_cluster_grouped(const bfs_cand* d_cands, uint32_t n, c
         const int rb = static_cast<int>((n + kRangeThreads - 1) / kRangeThreads);
         k_field_range<<<std::min(rb, 592), kRangeThreads, 0, s>>>(d_cands, n, range);
         BFS_LAUNCH_CHECK("k_field_range");
-        BFS_CUDA(cudaMemcpyAsync(h_range, range, sizeof(h_range), cudaMemcpyDeviceToHost, s));
-        BFS_CUDA(cudaStreamSynchronize(s));
+        BFS_TRY(read_back(h_range, range, 6, s));
         for (int f = 0; f < 3; ++f) {
             fmin[f] = static_cast<int>(~h_range[2 * f] ^ 0x80000000u);
             frange[f] = static_cast<long long>(static_cast<int>(h_range[2 * f + 1] ^ 0x80000000u)) - fmin[f];
@@ -639,8 +686,7 @@ extern "C" bfs_status bfs_cluster_grouped(const bfs_cand* d_cands, uint32_t n, c
                                                   tmp, tmp_bytes, s, sort_only);
         if (st != BFS_OK) return st;
         if (sort_only) continue;   // same groups, same boundaries (groups stay in gid order)
-        BFS_CUDA(cudaMemcpyAsync(&groups, scan + (n - 1), sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        BFS_CUDA(cudaStreamSynchronize(s));
+        BFS_TRY(read_back(&groups, scan + (n - 1), 1, s));
     }
     BFS_CUDA(cudaMemcpyAsync(d_perm, v_out, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
     k_offsets<<<bl, th, 0, s>>>(flags, scan, n, d_offsets);

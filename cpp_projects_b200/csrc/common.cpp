@@ -58,6 +58,38 @@ bfs_status stream_alloc(void** p, size_t bytes, cudaStream_t s) {
     return BFS_OK;
 }
 
+namespace {
+struct PinnedWords {
+    unsigned* p = nullptr;
+    bool tried = false;
+    ~PinnedWords() {
+        if (p) cudaFreeHost(p);
+    }
+};
+thread_local PinnedWords g_pinned;
+}  // namespace
+
+unsigned* read_back_words() {
+    if (!g_pinned.tried) {
+        g_pinned.tried = true;
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(unsigned) * kReadBackWords, cudaHostAllocPortable) == cudaSuccess)
+            g_pinned.p = static_cast<unsigned*>(p);
+        else
+            cudaGetLastError();
+    }
+    return g_pinned.p;
+}
+
+bfs_status read_back(unsigned* host, const unsigned* d, int n, cudaStream_t s) {
+    unsigned* pin = n <= kReadBackWords ? read_back_words() : nullptr;
+    unsigned* to = pin ? pin : host;
+    BFS_CUDA(cudaMemcpyAsync(to, d, sizeof(unsigned) * n, cudaMemcpyDeviceToHost, s));
+    BFS_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < n && to != host; ++i) host[i] = to[i];
+    return BFS_OK;
+}
+
 }  // namespace bfs
 
 extern "C" const char* bfs_last_error(void) { return bfs::last_error(); }

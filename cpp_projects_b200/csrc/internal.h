@@ -21,6 +21,15 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // cudaMallocAsync from the device's default pool, which keeps freed memory.
 bfs_status stream_alloc(void** p, size_t bytes, cudaStream_t s);
 
+// A few words of pinned host memory of the calling thread, for counts read
+// back from the device (kReadBackWords of them; null when pinning failed: the
+// caller then reads into pageable memory).
+constexpr int kReadBackWords = 16;
+unsigned* read_back_words();
+
+// n words from device memory, waiting for the stream.
+bfs_status read_back(unsigned* host, const unsigned* d, int n, cudaStream_t s);
+
 #define BFS_CUDA(call)                                                                     \
     do {                                                                                   \
         cudaError_t e_ = (call);                                                           \

@@ -940,11 +940,11 @@ bfs_status compact_ordered(const bfs_cand* src, const unsigned* rec_first, const
     const long long blocks = (nrec + th - 1) / th;
     BFS_ARG(blocks < (1ll << 31), "too many boxcar tiles (%lld)", nrec);
     unsigned* pos = nullptr;
-    void* tmp = nullptr;
     size_t tmp_bytes = 0;
     BFS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, rec_count, pos, static_cast<int>(nrec), s));
-    bfs_status st = stream_alloc(reinterpret_cast<void**>(&pos), sizeof(unsigned) * nrec, s);
-    if (st == BFS_OK) st = stream_alloc(&tmp, tmp_bytes ? tmp_bytes : 16, s);
+    const size_t pos_bytes = (sizeof(unsigned) * nrec + 255) & ~static_cast<size_t>(255);
+    bfs_status st = stream_alloc(reinterpret_cast<void**>(&pos), pos_bytes + tmp_bytes, s);
+    void* tmp = reinterpret_cast<char*>(pos) + pos_bytes;
     if (st == BFS_OK) {
         cudaError_t e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, rec_count, pos, static_cast<int>(nrec), s);
         if (e == cudaSuccess) {
@@ -955,7 +955,6 @@ bfs_status compact_ordered(const bfs_cand* src, const unsigned* rec_first, const
         if (e != cudaSuccess) st = fail(BFS_ERR_CUDA, "candidate compaction: %s", cudaGetErrorString(e));
     }
     if (pos) cudaFreeAsync(pos, s);
-    if (tmp) cudaFreeAsync(tmp, s);
     return st;
 }
 
@@ -999,11 +998,12 @@ extern "C" bfs_status bfs_boxcar_gather(const float* d_plane, int rows, int cols
     // others: atomic appends, then a radix sort by the canonical key
     const bool ordered = boxcar_ordered_supported(widths_mode, param);
     const long long nrec = ordered ? boxcar_ordered_records(rows, cols) : 0;
+    // one piece: candidate and work-list counts, first[nrec], count[nrec], work[nrec]
     unsigned* d_count = nullptr;
-    unsigned* rec = nullptr;   // first[nrec], count[nrec], work[nrec]
-    BFS_TRY_ST(stream_alloc(reinterpret_cast<void**>(&d_count), 2 * sizeof(unsigned), s));   // candidates, work entries
-    bfs_status st = ordered ? stream_alloc(reinterpret_cast<void**>(&rec), sizeof(unsigned) * 3 * nrec, s) : BFS_OK;
-    if (st == BFS_OK) {
+    BFS_TRY_ST(stream_alloc(reinterpret_cast<void**>(&d_count), sizeof(unsigned) * (64 + 3 * nrec), s));
+    unsigned* rec = d_count + 64;
+    bfs_status st = BFS_OK;
+    {
         cudaError_t e = cudaMemsetAsync(d_count, 0, 2 * sizeof(unsigned), s);
         if (e != cudaSuccess) st = fail(BFS_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
     }
@@ -1013,13 +1013,7 @@ extern "C" bfs_status bfs_boxcar_gather(const float* d_plane, int rows, int cols
                      : launch_boxcar(d_plane, rows, cols, d_stats, thr, d_thr, widths_mode, param,
                                      snr_fast, d_out, capacity, d_count, s, 0, nullptr);
     unsigned count = 0;
-    if (st == BFS_OK) {
-        cudaError_t e = cudaMemcpyAsync(&count, d_count, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) st = fail(BFS_ERR_CUDA, "reading the candidate count: %s",
-                                        cudaGetErrorString(e));
-    }
-    cudaFreeAsync(d_count, s);
+    if (st == BFS_OK) st = read_back(&count, d_count, 1, s);
     if (st == BFS_OK) {
         *h_count = count;
         const unsigned n = count < capacity ? count : capacity;
@@ -1037,7 +1031,7 @@ extern "C" bfs_status bfs_boxcar_gather(const float* d_plane, int rows, int cols
             st = sort_candidates_canonical(d_out, n, rows, cols, widths_mode, param, s);
         }
     }
-    if (rec) cudaFreeAsync(rec, s);
+    cudaFreeAsync(d_count, s);
     if (st != BFS_OK) return st;
     if (count > capacity)
         return fail(BFS_ERR_OVERFLOW, "%u candidates found, capacity %u", count, capacity);
