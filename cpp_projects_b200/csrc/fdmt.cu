@@ -1187,9 +1187,10 @@ constexpr int kRunCtas = 2 * 148;
 // CTAs per SM.  Large planes take the most rows that fit (4096 x 45001: 40
 // rows 1.05 ms, 32 1.09, 24 1.19, 16 1.43), short ones fewer (256 x 22005: 32
 // rows 36.9 us, 40 41.1; 64 x 1000: 16 rows 12.5 us, 32 16.5).
-static void plan_run(const FdmtPlanHost& h, int l0, int l1, bool from_input, RunPlan* out) {
+static void plan_run(const FdmtPlanHost& h, int l0, int l1, bool from_input, RunPlan* out, int esize = 4) {
     const int m = l1 - l0, s2 = m == 4 ? 2 : 1;
-    const long long tt = (h.ncols + kSegTile - 1) / kSegTile;
+    const int width = esize == 2 ? kRun16Tile : kSegTile;
+    const long long tt = (h.ncols + width - 1) / width;
     std::vector<std::pair<double, int>> order;
     for (int G = 8; G <= 48; G += 4) {
         long long tiles = 0, left = 0;   // the cut of build_run_plan
@@ -1204,7 +1205,7 @@ static void plan_run(const FdmtPlanHost& h, int l0, int l1, bool from_input, Run
     }
     std::sort(order.begin(), order.end());
     for (const auto& o : order)
-        if (build_run_plan(h, l0, l1, o.second, kRunSmem, out, from_input)) return;
+        if (build_run_plan(h, l0, l1, o.second, kRunSmem, out, from_input, esize)) return;
 }
 
 // `tables`: k_fdmt_seg's tables are wanted for passes that run segments serve
@@ -1212,7 +1213,8 @@ static void plan_run(const FdmtPlanHost& h, int l0, int l1, bool from_input, Run
 // The passes after the head (or level 0): levels k+1..niter cut into fused
 // segments of about desc->seg_levels levels (FP32 plans), or one plain merge
 // pass per level; then the ping-pong plane of every level that reaches HBM.
-static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int default_levels, bool tables) {
+static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int default_levels, bool tables,
+                               bool runs16 = false) {
     const FdmtPlanHost& h = p->host;
     const int k = p->fuse_depth;
     const int want = desc->seg_levels == 0 ? default_levels : desc->seg_levels;
@@ -1238,10 +1240,11 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
     // a fused pass runs as a run segment where one fits two CTAs on an SM,
     // unless the description names a CTA size or buffering of k_fdmt_seg
     const bool run_ok = desc->seg_threads == 0 && desc->seg_flags == 0;
+    const int esize = elem_bytes_of(p->precision);
     auto run_alone = [&](int l0, int l1, bool from_input) {
-        if ((tables && !(from_input && h.kind == BFS_PLAN_PRAVIR)) || !run_ok) return false;
+        if ((tables && esize == 4 && !(from_input && h.kind == BFS_PLAN_PRAVIR)) || !run_ok) return false;
         RunPlan rp;
-        plan_run(h, l0, l1, from_input, &rp);
+        plan_run(h, l0, l1, from_input, &rp, esize);
         if (rp.s1 == 0) return false;
         SegPlan sp;
         sp.l0 = l0; sp.l1 = l1; sp.r0c = rp.r0c;
@@ -1251,7 +1254,25 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
         return true;
     };
     const int left = h.niter - k;
-    if (want < 2 || p->precision != BFS_PREC_F32 || left < 2) {
+    if (esize == 2) {
+        // run segments where every row of a level has the scale of its level
+        // (a power-of-two channel count), else one plain pass per level
+        const auto even = [&] {
+            const std::vector<std::vector<int>> ex = row_exponents(h);
+            for (int l = k; l <= h.niter; ++l)
+                for (int e : ex[l])
+                    if (e != l) return false;
+            return true;
+        };
+        const int nseg = runs16 && left >= 2 && even() ? (left + kRunDefaultLevels - 1) / kRunDefaultLevels : 0;
+        int l0 = k;
+        for (int i = 0; i < nseg; ++i) {
+            const int l1 = l0 + left / nseg + (i < left % nseg ? 1 : 0);
+            if (!run_alone(l0, l1, false)) break;
+            l0 = l1;
+        }
+        for (int l = l0 + 1; l <= h.niter; ++l) plain(l);
+    } else if (want < 2 || left < 2) {
         for (int l = k + 1; l <= h.niter; ++l) plain(l);
     } else {
         const int nseg = (left + want - 1) / want;
@@ -1324,7 +1345,9 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
     return BFS_OK;
 }
 
-static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_fdmt_plan>& p, bool tables) {
+// `tuned`: desc is the autotuner's own choice.
+static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_fdmt_plan>& p, bool tables,
+                                 bool tuned = false) {
     BFS_ARG(desc != nullptr, "null argument");
     BFS_ARG(desc->plan_kind == BFS_PLAN_KEITH || desc->plan_kind == BFS_PLAN_PRAVIR,
             "unsupported plan_kind %d", desc->plan_kind);
@@ -1376,7 +1399,9 @@ static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_
             return BFS_OK;
     }
     p->fuse_depth = p->head.depth;
-    return build_passes(desc, p.get(), kSegDefaultLevels, tables);
+    // (16-bit plans: with an explicit depth 0 or one level per pass, plain passes)
+    const bool runs16 = desc->seg_levels == 0 && (tuned || desc->fuse_depth != 0);
+    return build_passes(desc, p.get(), kSegDefaultLevels, tables, runs16);
 }
 
 static inline int bfs_fdmt_plan_depth_of(int d) { return d; }
@@ -1464,6 +1489,8 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
         st = fail(BFS_ERR_ALLOC, "autotune: cannot allocate scratch for a %dx%d FDMT", base.nchan, base.ncols);
     }
     if (st == BFS_OK) cudaMemsetAsync(d_in, 0, in_n * sizeof(float), s);
+    // (16-bit plans: the depth, which decides where values are rounded, is
+    // chosen on one plain pass per level; run segments then serve it)
     for (const Cand& c : cands) {
         if (st != BFS_OK) break;
         bfs_fdmt_desc d = base;
@@ -1509,6 +1536,7 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
     if (e1) cudaEventDestroy(e1);
     cudaGetLastError();
     if (st != BFS_OK) return st;
+    if (base.precision != BFS_PREC_F32) win.seg = 0;
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune[tune_key(base)] = win;
     *best = win;
@@ -1569,7 +1597,7 @@ extern "C" bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc_in, bfs_fdm
     }
     const bfs_fdmt_desc* desc = &tuned;
     std::unique_ptr<bfs_fdmt_plan> p;
-    bfs_status st = plan_host_part(desc, p, desc_in->seg_rows > 0);
+    bfs_status st = plan_host_part(desc, p, desc_in->seg_rows > 0, desc_in->fuse_depth == BFS_FUSE_AUTOTUNE);
     if (st != BFS_OK) return st;
     p->host_only = false;
     BFS_CUDA(cudaGetDevice(&p->device));
@@ -1879,9 +1907,20 @@ static bfs_status fdmt_run16(bfs_fdmt_plan* plan, const float* d_in, float* d_ou
         cudaError_t e = launch_init<S>(d_in, bufs[plan->plane_buf[0]], h, P, b_ones ? 1 : 0, s, plan->d_lvl0);
         if (e != cudaSuccess) return fail(BFS_ERR_CUDA, "k_fdmt_init: %s", cudaGetErrorString(e));
     }
-    for (const SegPlan& sp : plan->passes) {  // 16-bit plans: one plain pass per level
+    for (size_t i = 0; i < plan->passes.size(); ++i) {
+        const SegPlan& sp = plan->passes[i];
         const int l = sp.l1;
         const S* src = bufs[plan->plane_buf[sp.l0]];
+        if (plan->runs[i].s1 > 0) {
+            const bool last = l == h.niter;
+            cudaError_t e = launch_run16<S>(plan->runs[i], src, last ? static_cast<void*>(d_out) : bufs[plan->plane_buf[l]],
+                                            last, plan->d_run_tiles + plan->run_tile0[i],
+                                            reinterpret_cast<const int2*>(plan->d_run_rows + plan->run_row0[i]),
+                                            reinterpret_cast<const int4*>(plan->d_run_ent + plan->run_ent0[i]), T, P,
+                                            last ? T : P, s);
+            if (e != cudaSuccess) return fail(BFS_ERR_CUDA, "k_fdmt_run16 (levels %d..%d): %s", sp.l0 + 1, l, cudaGetErrorString(e));
+            continue;
+        }
         const int4* tab = plan->d_tab + plan->tab_off[l];
         const int rows = h.lv[l].total_rows();
         cudaError_t e = (l == h.niter)

@@ -12,4 +12,10 @@ namespace bfs {
 cudaError_t launch_run(const RunPlan& rp, const float* src, float* dst, const RunTile* tiles, const int2* rows,
                        const int4* ent, int ncols, int in_pitch, int out_pitch, int ones, cudaStream_t s);
 
+// The same over 16-bit planes of a plan whose level-l rows all carry the scale
+// 2^-l: src and, unless out_f32, dst hold S = __half or __nv_bfloat16.
+template <typename S>
+cudaError_t launch_run16(const RunPlan& rp, const S* src, void* dst, bool out_f32, const RunTile* tiles,
+                         const int2* rows, const int4* ent, int ncols, int in_pitch, int out_pitch, cudaStream_t s);
+
 }  // namespace bfs

@@ -294,11 +294,16 @@ bool build_seg_plan(const FdmtPlanHost& p, int l0, int l1, int rows, int tile, s
 // 2, .. per channel): the input rows are channels and an input of stage 1 is
 // a level-0 row of one: entry bits 20.. give its row number r, the
 // running mean over r + 1 samples is formed where it is read.
+// 16-bit plans (esize 2) keep both buffers in 16 bits: offsets and pitches
+// count 2-byte values, tiles have kRun16Tile samples and mid rows kRun16Mid,
+// windows start on 16-byte boundaries (8 samples).
 // ---------------------------------------------------------------------------
 constexpr int kRunMidChunks = 9;                  // 32-column chunks of a mid row
 constexpr int kRunMid = 32 * kRunMidChunks;
 constexpr int kRunOutChunks = kSegTile / 32;
 constexpr int kRunMaxPitch = 384;
+constexpr int kRun16Tile = 2 * kSegTile;          // 16-bit plans: the same bytes per row
+constexpr int kRun16Mid = 2 * kRunMid;
 
 struct RunTile {                 // device-side
     int row;                     // first of the tile's input rows
@@ -311,10 +316,11 @@ struct RunTile {                 // device-side
 struct RunPlan {
     int l0 = 0, l1 = 0;
     int s1 = 0, s2 = 0;          // levels merged by each stage (0: no plan)
+    int esize = 4;               // bytes of a value in the planes and buffers
     int r0c = 0;                 // input segment: most level-0 rows of a channel
     bool positive = false;       // input segment of a Pravir plan: its window sums start at +0,
                                  // so a channel's -0.0 counts as +0
-    int pitch_x = 0;             // floats per row of X
+    int pitch_x = 0;             // values per row of X
     int zero_x = 0, zero_y = 0;  // offsets of the -0.0 rows
     int y0 = 0, ent0 = 0;        // offsets of Y and of the two staged entry buffers
     int max_ent = 0;             // most entries of one tile
@@ -329,6 +335,6 @@ struct RunPlan {
 // the leads of an input segment: a channel's window starts on a 16-byte
 // boundary of the filterbank, whose rows are ncols floats.
 bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int rows, size_t smem_limit, RunPlan* out,
-                    bool from_input);
+                    bool from_input, int esize = 4);
 
 }  // namespace bfs

@@ -395,9 +395,11 @@ static std::vector<std::pair<int, int>> row_cuts(const FdmtLevel& top, int G) {
 }
 
 bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_limit, RunPlan* out,
-                    bool from_input) {
+                    bool from_input, int esize) {
     const int m = l1 - l0;
-    if (m < 2 || m > 4 || l0 < 0 || l1 > p.niter || G < 1) return false;
+    if (m < 2 || m > 4 || l0 < 0 || l1 > p.niter || G < 1 || (from_input && esize != 4)) return false;
+    const int tile = esize == 2 ? kRun16Tile : kSegTile, mid = esize == 2 ? kRun16Mid : kRunMid;
+    const int max_pitch = esize == 2 ? 2 * kRunMaxPitch : kRunMaxPitch, piece = 16 / esize;   // samples of 16 bytes
     const std::vector<int>& ccum = p.lv[0].cum;   // level-0 rows by channel
     int r0c = 0;
     if (from_input) {
@@ -419,7 +421,7 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
     s.positive = from_input && p.kind == BFS_PLAN_PRAVIR;
     const int lm = l1 - s.s2;
     struct Leaf { int row, shift; };             // row -1: the -0.0 row
-    struct Row { int row, lo, hi; };             // needs samples t0 - hi .. t0 + kSegTile - lo
+    struct Row { int row, lo, hi; };             // needs samples t0 - hi .. t0 + tile - lo
     auto leaves = [&](int level, int g, int levels, Leaf (&v)[4]) {
         const FdmtLevel& L = p.lv[level];
         const Leaf a{L.a_row[g], 0};
@@ -435,7 +437,17 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         split(a, v[0], v[1]);
         split(b, v[2], v[3]);
     };
-    auto add = [](std::vector<Row>& v, int row, int lo, int hi) { v.push_back({row, lo, hi}); };
+    // leaf i of consecutive rows is often the same row: extended where it was
+    // added last (at[i]) instead of added again
+    auto add = [](std::vector<Row>& v, int (&at)[4], int i, int row, int lo, int hi) {
+        if (at[i] >= 0 && v[at[i]].row == row) {
+            v[at[i]].lo = std::min(v[at[i]].lo, lo);
+            v[at[i]].hi = std::max(v[at[i]].hi, hi);
+        } else {
+            at[i] = static_cast<int>(v.size());
+            v.push_back({row, lo, hi});
+        }
+    };
     auto unite = [](std::vector<Row>& v) {       // sorted by row, one entry per row
         std::sort(v.begin(), v.end(), [](const Row& a, const Row& b) { return a.row < b.row; });
         size_t k = 0;
@@ -458,12 +470,14 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         Tile t;
         t.g0 = c.first; t.g1 = c.second;
         Leaf v[4];
+        int at[4] = {-1, -1, -1, -1};
         for (int g = t.g0; g < t.g1; ++g) {
             leaves(l1, g, s.s2, v);
-            for (const Leaf& x : v)
-                if (x.row >= 0) add(t.mid, x.row, x.shift, x.shift);
+            for (int i = 0; i < 4; ++i)
+                if (v[i].row >= 0) add(t.mid, at, i, v[i].row, v[i].shift, v[i].shift);
         }
         unite(t.mid);
+        std::fill(at, at + 4, -1);
         // one window per sub-band of the mid level
         for (size_t i = 0; i < t.mid.size();) {
             const int band = static_cast<int>(std::upper_bound(mcum.begin(), mcum.end(), t.mid[i].row) - mcum.begin()) - 1;
@@ -473,45 +487,47 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
                 lo = std::min(lo, t.mid[e].lo);
                 hi = std::max(hi, t.mid[e].hi);
             }
-            if (kSegTile + hi - lo > kRunMid) return false;
+            if (tile + hi - lo > mid) return false;
             for (; i < e; ++i) { t.mid[i].lo = lo; t.mid[i].hi = hi; }
         }
         for (const Row& r : t.mid) {
             leaves(lm, r.row, s.s1, v);
-            for (const Leaf& x : v) {
+            for (int i = 0; i < 4; ++i) {
+                const Leaf& x = v[i];
                 if (x.row < 0) continue;
                 if (from_input) {
                     const int c = chan_of(x.row);
-                    add(t.in, c, r.lo + x.shift, r.hi + x.shift + x.row - ccum[c]);
+                    add(t.in, at, i, c, r.lo + x.shift, r.hi + x.shift + x.row - ccum[c]);
                 } else {
-                    add(t.in, x.row, r.lo + x.shift, r.hi + x.shift);
+                    add(t.in, at, i, x.row, r.lo + x.shift, r.hi + x.shift);
                 }
             }
         }
         unite(t.in);
         for (Row& r : t.in) {
-            // first sample t0 - hi on a 16-byte boundary (t0 a multiple of 4)
+            // first sample t0 - hi on a 16-byte boundary (t0 a multiple of 8)
             const int phase = from_input ? static_cast<int>((static_cast<long long>(r.row) * p.ncols) & 3) : 0;
-            while ((r.hi & 3) != phase) ++r.hi;
+            while ((r.hi & (piece - 1)) != phase) ++r.hi;
             spread = std::max(spread, r.hi - r.lo);
             max_lead = std::max(max_lead, r.hi);
         }
         max_in = std::max(max_in, static_cast<int>(t.in.size()));
         max_mid = std::max(max_mid, static_cast<int>(t.mid.size()));
         s.max_ent = std::max(s.max_ent, static_cast<int>(t.mid.size()) + t.g1 - t.g0);
-        if (4ull * (static_cast<size_t>(max_in) * (kSegTile + spread) + static_cast<size_t>(max_mid) * kRunMid) > smem_limit)
+        if (static_cast<size_t>(esize) * (static_cast<size_t>(max_in) * (tile + spread) + static_cast<size_t>(max_mid) * mid) > smem_limit)
             return false;
         tiles.push_back(std::move(t));
     }
-    s.pitch_x = (kSegTile + spread + 3) & ~3;
-    if (s.pitch_x > kRunMaxPitch) return false;
+    s.esize = esize;
+    s.pitch_x = (tile + spread + piece - 1) & ~(piece - 1);
+    if (s.pitch_x > max_pitch) return false;
     s.zero_x = max_in * s.pitch_x;
-    s.y0 = s.zero_x + kRunMid;
-    s.zero_y = s.y0 + max_mid * kRunMid;
-    s.ent0 = s.zero_y + kSegTile;
+    s.y0 = s.zero_x + mid;
+    s.zero_y = s.y0 + max_mid * mid;
+    s.ent0 = s.zero_y + tile;
     s.edge = max_lead + r0c;
     ++s.max_ent;   // (the kernel reads one entry ahead)
-    s.smem_bytes = static_cast<size_t>(s.ent0) * sizeof(float) + 2 * static_cast<size_t>(s.max_ent) * 16;
+    s.smem_bytes = static_cast<size_t>(s.ent0) * esize + 2 * static_cast<size_t>(s.max_ent) * 16;
     if (s.smem_bytes > smem_limit) return false;
     auto slot_of = [](const std::vector<Row>& v, int row) {
         return static_cast<int>(std::lower_bound(v.begin(), v.end(), row, [](const Row& w, int r) { return w.row < r; }) -
@@ -523,13 +539,13 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         Leaf v[4];
         leaves(level, row, levels, v);
         for (int i = 0; i < 4; ++i) {
-            int e = zero * 4;
+            int e = zero * esize;
             if (v[i].row >= 0) {
                 const int src = chan ? chan_of(v[i].row) : v[i].row, r = chan ? v[i].row - ccum[src] : 0;
                 const int j = slot_of(from, src);
                 const int off = from[j].hi - hi - v[i].shift;
-                if (off < r || off + kSegTile > pitch) return false;
-                e = (base + j * pitch + off) * 4 | (r << 20);
+                if (off < r || off + tile > pitch) return false;
+                e = (base + j * pitch + off) * esize | (r << 20);
             }
             s.ent.push_back(e | (e != prev[i] ? 1 : 0));
             prev[i] = e;
@@ -550,7 +566,7 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
             if (!entries(lm, s.s1, t.in, 0, s.pitch_x, s.zero_x, from_input, w.row, w.hi, prev)) return false;
         for (int& x : prev) x = -1;
         for (int g = t.g0; g < t.g1; ++g)
-            if (!entries(l1, s.s2, t.mid, s.y0, kRunMid, s.zero_y, false, g, 0, prev)) return false;
+            if (!entries(l1, s.s2, t.mid, s.y0, mid, s.zero_y, false, g, 0, prev)) return false;
         s.tiles.push_back(r);
     }
     *out = std::move(s);

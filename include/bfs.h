@@ -88,8 +88,10 @@ typedef struct bfs_fdmt_desc {
     int dt_min;        /* BFS_PLAN_PRAVIR: smallest delay of the grid (0)              */
     int dt_step;       /* BFS_PLAN_PRAVIR: grid step (0 is taken as 1)                 */
     float tsamp;       /* BFS_PLAN_PRAVIR: sample time (s), for the DM grid only       */
-    int seg_levels;    /* merge levels fused per HBM pass after the head (FP32 plans):
-                          0: 3; 1: one pass per level; 2..6                              */
+    int seg_levels;    /* merge levels fused per HBM pass after the head: FP32 plans 0: 3;
+                          1: one pass per level; 2..6.  16-bit plans 0: up to 4 with a
+                          head or the default schedule, where every row of a level sums
+                          equally many channels, else one; 1: one pass per level         */
     int seg_rows;      /* output rows per tile of a fused pass (0: the most that keep
                           two CTAs per SM, of 64 / 32 / 16; run segments choose theirs) */
     int seg_threads;   /* 0 with seg_flags 0: passes of 2..4 levels are run segments
