@@ -28,6 +28,7 @@
 // reference's sizes.
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <memory>
 #include <vector>
@@ -44,20 +45,23 @@ struct bfs_chunk {
     bfs_fdmt_plan* fdmt = nullptr;
     float2* volt = nullptr;  // chirped spectrum, then voltages, per DM
     float* plane = nullptr;  // rows x msamp FDMT input
-    float* mask = nullptr;   // rows x msamp normalisation input
-    float* norm = nullptr;   // max_dt x msamp FDMT of the mask
+    float* mask = nullptr;   // rows kept (1) or zapped (0)
     float* buff = nullptr;   // 4 + 2 rows statistics
     int* d_shift = nullptr;  // rows dedispersion shifts
     // chirp factors per coherent DM ([chan][sub-band][mbin]) for the own
     // sub-band transforms, the most recent kChirpCache DMs
     std::vector<std::pair<double, float2*>> chirps;
+    // other geometries: the factors of the DM loop's first kept_max DMs
+    std::vector<double> kept;
+    size_t kept_max = 0;
+    float2* kept_tab = nullptr;
     ~bfs_chunk() {
         if (have_fwd) cufftDestroy(fwd);
         if (have_inv) cufftDestroy(inv);
         if (fdmt) bfs_fdmt_plan_destroy(fdmt);
         for (auto& c : chirps) cudaFree(c.second);
         for (void* p : {static_cast<void*>(volt), static_cast<void*>(plane), static_cast<void*>(mask),
-                        static_cast<void*>(norm), static_cast<void*>(buff), static_cast<void*>(d_shift)})
+                        static_cast<void*>(buff), static_cast<void*>(d_shift), static_cast<void*>(kept_tab)})
             if (p) cudaFree(p);
     }
 };
@@ -115,13 +119,21 @@ __device__ __forceinline__ float2 chirp_factor(double dm, int ichan, int isft, i
 // Chirp: one thread per (bin of the mbin sub-band, sub-band, coarse channel);
 // the factor is applied to every polarisation and FFT segment at the
 // fft-shifted position of the nbin spectrum.
-__global__ void k_chirp(const float2* __restrict__ in, float2* __restrict__ out, double dm, int nchan,
-                        int len_sft, int mbin, int nbin, int nseg, double fmin, double bw_sub,
-                        double bw_chan) {
+// tab: a table of the factors, to be read (known) or to receive them.
+__global__ void k_chirp(const float2* __restrict__ in, float2* __restrict__ out, float2* __restrict__ tab, int known,
+                        double dm, int nchan, int len_sft, int mbin, int nbin, int nseg, double fmin,
+                        double bw_sub, double bw_chan) {
     const int ibin = blockIdx.x * blockDim.x + threadIdx.x;
     if (ibin >= mbin) return;
     const int isft = blockIdx.y, ichan = blockIdx.z;
-    const float2 cf = chirp_factor(dm, ichan, isft, ibin, len_sft, mbin, nbin, fmin, bw_sub, bw_chan);
+    const size_t at = (static_cast<size_t>(ichan) * len_sft + isft) * mbin + ibin;
+    float2 cf;
+    if (known) {
+        cf = tab[at];
+    } else {
+        cf = chirp_factor(dm, ichan, isft, ibin, len_sft, mbin, nbin, fmin, bw_sub, bw_chan);
+        if (tab) tab[at] = cf;
+    }
     const size_t pos = static_cast<size_t>(ichan) * nbin + (isft * mbin + ibin + nbin / 2) % nbin;
     const size_t stride = static_cast<size_t>(nbin) * nchan;
     for (int i = 0; i < nseg; ++i) {
@@ -277,10 +289,20 @@ extern "C" bfs_status bfs_chunk_create(const bfs_chunk_desc* desc, bfs_chunk** o
     if (st != BFS_OK) return st;
     BFS_CUDA(cudaMalloc(&c->volt, sizeof(float2) * c->cplx_len));
     BFS_CUDA(cudaMalloc(&c->plane, sizeof(float) * static_cast<size_t>(c->rows) * c->msamp));
-    BFS_CUDA(cudaMalloc(&c->mask, sizeof(float) * static_cast<size_t>(c->rows) * c->msamp));
-    BFS_CUDA(cudaMalloc(&c->norm, sizeof(float) * static_cast<size_t>(max_dt) * c->msamp));
+    BFS_CUDA(cudaMalloc(&c->mask, sizeof(float) * c->rows));
     BFS_CUDA(cudaMalloc(&c->buff, sizeof(float) * (4 + 2 * static_cast<size_t>(c->rows))));
     BFS_CUDA(cudaMalloc(&c->d_shift, sizeof(int) * c->rows));
+    if (!subband_ifft_supported(d.nbin, d.len_sft, d.npol)) {
+        // up to four tables in about half the plane's memory, at least one;
+        // without the memory for them none
+        const size_t n = static_cast<size_t>(d.nchan) * d.nbin;
+        c->kept_max = std::min<size_t>(4, std::max<size_t>(1, static_cast<size_t>(c->rows) * c->msamp / (2 * n)));
+        if (cudaMalloc(&c->kept_tab, sizeof(float2) * n * c->kept_max) != cudaSuccess) {
+            cudaGetLastError();
+            c->kept_tab = nullptr;
+            c->kept_max = 0;
+        }
+    }
     *out = c.release();
     return BFS_OK;
 }
@@ -356,8 +378,11 @@ static bfs_status chirp_table(bfs_chunk* c, double dm, const float2** out, cudaS
     return BFS_OK;
 }
 
+// loop: from the DM loop, which keeps its first DMs' factors: their FP64 powers
+// and sines cost more than the pass over the spectra (16 x 2 x 2^16, two
+// polarisations: 25.0 us, with the table 9.9).
 static bfs_status chunk_voltages(bfs_chunk* c, const void* d_spec, double dm, float2* d_volt,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, bool loop = false) {
     const bfs_chunk_desc& d = c->d;
     // (the first pass reads all of a sub-band while writing it: not in place)
     const char* sp = static_cast<const char*>(d_spec);
@@ -377,7 +402,17 @@ static bfs_status chunk_voltages(bfs_chunk* c, const void* d_spec, double dm, fl
     const double bw_chan = bw_sub / d.len_sft;
     dim3 grid((c->mbin + 255) / 256, d.len_sft, d.nchan);
     BFS_ARG(grid.y <= 65535 && grid.z <= 65535, "too many sub-bands or channels");
-    k_chirp<<<grid, 256, 0, s>>>(static_cast<const float2*>(d_spec), d_volt, dm, d.nchan, d.len_sft,
+    float2* tab = nullptr;
+    int known = 0;
+    if (loop) {
+        const size_t n = static_cast<size_t>(d.nchan) * d.nbin;
+        size_t i = 0;
+        while (i < c->kept.size() && c->kept[i] != dm) ++i;
+        known = i < c->kept.size();
+        if (i < c->kept_max) tab = c->kept_tab + i * n;
+        if (tab && !known) c->kept.push_back(dm);
+    }
+    k_chirp<<<grid, 256, 0, s>>>(static_cast<const float2*>(d_spec), d_volt, tab, known, dm, d.nchan, d.len_sft,
                                  c->mbin, d.nbin, d.nfft * d.npol / 2, static_cast<double>(d.fmin),
                                  bw_sub, bw_chan);
     BFS_LAUNCH_CHECK("k_chirp");
@@ -439,7 +474,7 @@ static bfs_status chunk_detect(bfs_chunk* c, const float2* d_volt, double dm, fl
 static bfs_status chunk_detect_spectrum(bfs_chunk* c, const void* d_spec, double dm, float* d_plane,
                                         cudaStream_t s) {
     if (!own_subband(c, d_spec)) {
-        bfs_status st = chunk_voltages(c, d_spec, dm, c->volt, s);
+        bfs_status st = chunk_voltages(c, d_spec, dm, c->volt, s, true);
         if (st != BFS_OK) return st;
         return chunk_detect(c, c->volt, dm, d_plane, s);
     }
@@ -499,16 +534,17 @@ static bfs_status chunk_dm_loop(bfs_chunk* c, const void* d_cplx, const double* 
     for (int i = 0; i < ndm; ++i) {
         st = chunk_detect_spectrum(c, d_cplx, dms[i], c->plane, s);
         if (st != BFS_OK) return st;
-        st = bfs_preproc_calc_fdmt_inputs(c->plane, c->rows, c->msamp, c->buff, c->mask, stream);
+        st = clean_rows(c->plane, c->rows, c->msamp, c->buff, c->mask, s);
         if (st != BFS_OK) return st;
-        // FDMT of the mask: its rows are all 0 or all 1 (calc_fdmt_inputs zaps
-        // whole rows), so the channel-count form gives the same bits in one pass
-        st = bfs_fdmt_execute_row_mask(c->fdmt, c->mask, c->msamp, c->norm, stream);
+        // FDMT of the mask: its rows are all 0 or all 1 (whole rows are zapped),
+        // so the channel-count form gives its bits, one row of them at a time,
+        // where they divide
+        st = row_mask_ready(c->fdmt);
         if (st != BFS_OK) return st;
         float* out = d_out + i * plane_out;
         st = bfs_fdmt_execute(c->fdmt, c->plane, out, 0, stream);
         if (st != BFS_OK) return st;
-        st = bfs_fdmt_normalize(out, c->norm, static_cast<int64_t>(plane_out), out, stream);
+        st = row_mask_normalize(c->fdmt, c->mask, out, s);
         if (st != BFS_OK) return st;
     }
     return BFS_OK;

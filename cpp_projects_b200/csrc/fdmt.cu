@@ -242,11 +242,9 @@ cudaError_t launch_init(const float* d_in, D* dst, const FdmtPlanHost& h, int P,
 // the row written once.  L = max tau + 1 histogram entries.
 constexpr int kOnesThreads = 256;
 
-__global__ void __launch_bounds__(kOnesThreads)
-k_fdmt_ones(float* __restrict__ out, int out_pitch, const int* __restrict__ tau,
-            const float* __restrict__ w, int w_stride, int nchan, int ncols, int L) {
-    extern __shared__ float hist[];
-    const int d = blockIdx.x;
+// hist[i] = channels of output row d with delay <= i (i < L), by the whole CTA.
+__device__ __forceinline__ void ones_counts(float* hist, int d, const int* __restrict__ tau,
+                                            const float* __restrict__ w, int w_stride, int nchan, int L) {
     for (int i = threadIdx.x; i < L; i += blockDim.x) hist[i] = 0.0f;
     __syncthreads();
     const int* tr = tau + static_cast<size_t>(d) * nchan;
@@ -255,28 +253,85 @@ k_fdmt_ones(float* __restrict__ out, int out_pitch, const int* __restrict__ tau,
         if (on) atomicAdd(&hist[__ldg(tr + c)], 1.0f);
     }
     __syncthreads();
-    if (threadIdx.x < 32) {  // inclusive scan by one warp: a segment per lane
-        const int lane = threadIdx.x;
-        const int seg = (L + 31) / 32;
-        const int b0 = min(L, lane * seg), b1 = min(L, b0 + seg);
-        float sum = 0.0f;
-        for (int i = b0; i < b1; ++i) sum += hist[i];
-        float pre = sum;  // inclusive scan of the segment totals
+    // inclusive scan, a segment per thread (whole numbers: exact in any order)
+    __shared__ float warp_sum[kOnesThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int seg = (L + kOnesThreads - 1) / kOnesThreads;
+    const int b0 = min(L, static_cast<int>(threadIdx.x) * seg), b1 = min(L, b0 + seg);
+    float sum = 0.0f;
+    for (int i = b0; i < b1; ++i) sum += hist[i];
+    float pre = sum;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float v = __shfl_up_sync(0xffffffffu, pre, o);
-            if (lane >= o) pre += v;
-        }
-        float run = pre - sum;
-        for (int i = b0; i < b1; ++i) {
-            run += hist[i];
-            hist[i] = run;
-        }
+    for (int o = 1; o < 32; o <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += v;
+    }
+    if (lane == 31) warp_sum[warp] = pre;
+    __syncthreads();
+    float run = pre - sum;
+    for (int i = 0; i < warp; ++i) run += warp_sum[i];
+    for (int i = b0; i < b1; ++i) {
+        run += hist[i];
+        hist[i] = run;
     }
     __syncthreads();
+}
+
+__global__ void __launch_bounds__(kOnesThreads)
+k_fdmt_ones(float* __restrict__ out, int out_pitch, const int* __restrict__ tau,
+            const float* __restrict__ w, int w_stride, int nchan, int ncols, int L) {
+    extern __shared__ float hist[];
+    const int d = blockIdx.x;
+    ones_counts(hist, d, tau, w, w_stride, nchan, L);
     float* o = out + static_cast<size_t>(d) * out_pitch;
     const float last = hist[L - 1];
     for (int t = threadIdx.x; t < ncols; t += blockDim.x) o[t] = t < L ? hist[t] : last;
+}
+
+// x /= sqrt(counts + 1e-8), row d of x by gridDim.y CTAs.  The counts change
+// only below L, so the square roots are formed once per row (in place of the
+// counts) and a row is read and written once: 1024 x 129024 in 180 us, HBM-bound (5.9 TB/s);
+// as a plane of counts and a pass over both 109 + 244 us.  VEC: every row
+// starts on a 16-byte boundary (ncols a multiple of 4).
+template <bool VEC>
+__global__ void __launch_bounds__(kOnesThreads)
+k_fdmt_ones_divide(float* __restrict__ x, const int* __restrict__ tau, const float* __restrict__ w, int nchan,
+                   int ncols, int L) {
+    extern __shared__ float hist[];
+    const int d = blockIdx.x;
+    ones_counts(hist, d, tau, w, 1, nchan, L);
+    for (int i = threadIdx.x; i < L; i += kOnesThreads)
+        hist[i] = __fsqrt_rn(__double2float_rn(static_cast<double>(hist[i]) + 1.0e-8));
+    __syncthreads();
+    const float last = hist[L - 1];
+    float* row = x + static_cast<size_t>(d) * ncols;
+    auto div = [&](float v, int t) { return __fdiv_rn(v, t < L ? hist[t] : last); };
+    if constexpr (VEC) {
+        constexpr int kDeep = 4;   // loads in flight per thread
+        float4* r4 = reinterpret_cast<float4*>(row);
+        const int n4 = ncols >> 2, step = kOnesThreads * gridDim.y;
+        for (int i = blockIdx.y * kOnesThreads + threadIdx.x; i < n4; i += kDeep * step) {
+            float4 v[kDeep];
+#pragma unroll
+            for (int k = 0; k < kDeep; ++k)
+                if (i + k * step < n4) v[k] = r4[i + k * step];
+#pragma unroll
+            for (int k = 0; k < kDeep; ++k) {
+                const int t = 4 * (i + k * step);
+                if (i + k * step >= n4) break;
+                if (t >= L) {
+                    v[k] = make_float4(__fdiv_rn(v[k].x, last), __fdiv_rn(v[k].y, last), __fdiv_rn(v[k].z, last),
+                                       __fdiv_rn(v[k].w, last));
+                } else {
+                    v[k] = make_float4(div(v[k].x, t), div(v[k].y, t + 1), div(v[k].z, t + 2), div(v[k].w, t + 3));
+                }
+                r4[i + k * step] = v[k];
+            }
+        }
+    } else {
+        for (int t = blockIdx.y * kOnesThreads + threadIdx.x; t < ncols; t += kOnesThreads * gridDim.y)
+            row[t] = div(row[t], t);
+    }
 }
 
 // One merge level.  The input plane is always a workspace plane (128-byte
@@ -1884,6 +1939,29 @@ static bfs_status launch_ones(bfs_fdmt_plan* plan, const float* d_w, int w_strid
     return BFS_OK;
 }
 
+bfs_status bfs::row_mask_ready(bfs_fdmt_plan* plan) {
+    BFS_ARG(plan->precision == BFS_PREC_F32, "the row-mask FDMT is implemented for FP32 plans");
+    bool usable = false;
+    bfs_status st = ensure_ones(plan, &usable);
+    if (st != BFS_OK) return st;
+    BFS_ARG(usable, "the plan's delays exceed the row-mask histogram (%d)", kOnesMaxHist);
+    return BFS_OK;
+}
+
+bfs_status bfs::row_mask_normalize(bfs_fdmt_plan* plan, const float* row_mask, float* out, cudaStream_t s) {
+    bfs_status st = row_mask_ready(plan);
+    if (st != BFS_OK) return st;
+    const FdmtPlanHost& h = plan->host;
+    const int rows = h.out_rows(), L = plan->ones_max_tau + 1;
+    // few rows: a row's columns over several CTAs, of 16 or more columns per thread
+    const int parts = std::max(1, std::min({(2 * 8 * 148 + rows - 1) / rows, h.ncols / (16 * kOnesThreads), 65535}));
+    const bool vec = h.ncols % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
+    auto* kern = vec ? k_fdmt_ones_divide<true> : k_fdmt_ones_divide<false>;
+    kern<<<dim3(rows, parts), kOnesThreads, L * sizeof(float), s>>>(out, plan->d_ones_tau, row_mask, h.nchan, h.ncols, L);
+    BFS_LAUNCH_CHECK("k_fdmt_ones_divide");
+    return BFS_OK;
+}
+
 // The same schedule over 16-bit planes (storage type S).
 template <typename S>
 static bfs_status fdmt_run16(bfs_fdmt_plan* plan, const float* d_in, float* d_out, int b_ones,
@@ -2023,11 +2101,8 @@ extern "C" bfs_status bfs_fdmt_execute_row_mask(bfs_fdmt_plan* plan, const float
                                                 float* d_out, void* stream) {
     BFS_ARG(plan != nullptr && d_mask != nullptr && d_out != nullptr, "null argument");
     BFS_ARG(!plan->host_only, "plan was created with bfs_fdmt_plan_create_host");
-    BFS_ARG(plan->precision == BFS_PREC_F32, "the row-mask FDMT is implemented for FP32 plans");
-    bool usable = false;
-    bfs_status st = ensure_ones(plan, &usable);
+    bfs_status st = row_mask_ready(plan);
     if (st != BFS_OK) return st;
-    BFS_ARG(usable, "the plan's delays exceed the row-mask histogram (%d)", kOnesMaxHist);
     return launch_ones(plan, d_mask, mask_pitch, d_out, as_stream(stream));
 }
 

@@ -337,4 +337,12 @@ struct RunPlan {
 bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int rows, size_t smem_limit, RunPlan* out,
                     bool from_input, int esize = 4);
 
+// bfs_preproc_calc_fdmt_inputs with the mask as one value (0 or 1) per row.
+bfs_status clean_rows(float* x, int nrows, int ncols, float* buff, float* row_mask, cudaStream_t s);
+// Whether the plan's row-mask FDMT can run (its delay table built on first
+// use), and out /= sqrt(row-mask FDMT + 1e-8) in place, as
+// bfs_fdmt_execute_row_mask and bfs_fdmt_normalize form it.
+bfs_status row_mask_ready(bfs_fdmt_plan* plan);
+bfs_status row_mask_normalize(bfs_fdmt_plan* plan, const float* row_mask, float* out, cudaStream_t s);
+
 }  // namespace bfs

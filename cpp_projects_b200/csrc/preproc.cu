@@ -65,7 +65,9 @@ __device__ __forceinline__ float clean_sample(float v, float mf, float sf) {
 }
 
 // VEC: cols % 4 == 0 and 16-byte aligned planes, so every row moves as float4s.
-template <bool VEC>
+// ROWS: mask holds one value per row instead of a plane of them (a third of the
+// pass's traffic: 1024 x 129024, 229 against 162 us).
+template <bool VEC, bool ROWS>
 __global__ void k_clean_normalize(float* __restrict__ x, float* __restrict__ mask, int rows, int cols,
                                   const float* __restrict__ buff) {
     const int row = blockIdx.y;
@@ -73,30 +75,31 @@ __global__ void k_clean_normalize(float* __restrict__ x, float* __restrict__ mas
     const float mf = g[0], sf = g[1], dmf = g[2], dsf = g[3];
     const bool zap = static_cast<double>(fabsf(buff[rows + row] - dmf)) > 4.0 * static_cast<double>(dsf);
     const size_t base = static_cast<size_t>(row) * cols;
+    if (ROWS && blockIdx.x == 0 && threadIdx.x == 0) mask[row] = zap ? 0.0f : 1.0f;
     if constexpr (VEC) {
         float4* xr = reinterpret_cast<float4*>(x + base);
-        float4* mr = reinterpret_cast<float4*>(mask + base);
+        float4* mr = reinterpret_cast<float4*>(mask + (ROWS ? 0 : base));
         const int n4 = cols >> 2;
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
         for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += gridDim.x * blockDim.x) {
             if (zap) {
                 xr[q] = z;
-                mr[q] = z;
+                if (!ROWS) mr[q] = z;
             } else {
                 const float4 v = xr[q];
                 xr[q] = make_float4(clean_sample(v.x, mf, sf), clean_sample(v.y, mf, sf),
                                     clean_sample(v.z, mf, sf), clean_sample(v.w, mf, sf));
-                mr[q] = one;
+                if (!ROWS) mr[q] = one;
             }
         }
     } else {
         for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cols; t += gridDim.x * blockDim.x) {
             if (zap) {
                 x[base + t] = 0.0f;
-                mask[base + t] = 0.0f;
+                if (!ROWS) mask[base + t] = 0.0f;
             } else {
                 x[base + t] = clean_sample(x[base + t], mf, sf);
-                mask[base + t] = 1.0f;
+                if (!ROWS) mask[base + t] = 1.0f;
             }
         }
     }
@@ -143,27 +146,35 @@ __global__ void k_fdmt_normalize(const float* __restrict__ f, const float* __res
 
 using namespace bfs;
 
+template <bool ROWS>
+static bfs_status clean(float* x, int nrows, int ncols, float* buff, float* mask, cudaStream_t s) {
+    BFS_ARG(nrows >= 1 && ncols >= 1 && nrows <= 65535, "bad shape %dx%d", nrows, ncols);
+    bfs_status st = launch_row_stats(x, nrows, ncols, buff, 1, s);
+    if (st != BFS_OK) return st;
+    k_global_stats<<<1, kGlobalThreads, 0, s>>>(buff, nrows);
+    BFS_LAUNCH_CHECK("k_global_stats");
+    const bool vec = (ncols % 4 == 0) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+                     (ROWS || (reinterpret_cast<uintptr_t>(mask) & 15) == 0);
+    if (vec) {
+        dim3 grid(std::min((ncols / 4 + 255) / 256, 64), nrows);
+        k_clean_normalize<true, ROWS><<<grid, 256, 0, s>>>(x, mask, nrows, ncols, buff);
+    } else {
+        dim3 grid(std::min((ncols + 255) / 256, 64), nrows);
+        k_clean_normalize<false, ROWS><<<grid, 256, 0, s>>>(x, mask, nrows, ncols, buff);
+    }
+    BFS_LAUNCH_CHECK("k_clean_normalize");
+    return BFS_OK;
+}
+
 extern "C" bfs_status bfs_preproc_calc_fdmt_inputs(float* d_inout, int nrows, int ncols,
                                                    float* d_buff, float* d_norm_input,
                                                    void* stream) {
     BFS_ARG(d_inout && d_buff && d_norm_input, "null argument");
-    BFS_ARG(nrows >= 1 && ncols >= 1 && nrows <= 65535, "bad shape %dx%d", nrows, ncols);
-    cudaStream_t s = as_stream(stream);
-    bfs_status st = launch_row_stats(d_inout, nrows, ncols, d_buff, 1, s);
-    if (st != BFS_OK) return st;
-    k_global_stats<<<1, kGlobalThreads, 0, s>>>(d_buff, nrows);
-    BFS_LAUNCH_CHECK("k_global_stats");
-    const bool vec = (ncols % 4 == 0) && (reinterpret_cast<uintptr_t>(d_inout) & 15) == 0 &&
-                     (reinterpret_cast<uintptr_t>(d_norm_input) & 15) == 0;
-    if (vec) {
-        dim3 grid(std::min((ncols / 4 + 255) / 256, 64), nrows);
-        k_clean_normalize<true><<<grid, 256, 0, s>>>(d_inout, d_norm_input, nrows, ncols, d_buff);
-    } else {
-        dim3 grid(std::min((ncols + 255) / 256, 64), nrows);
-        k_clean_normalize<false><<<grid, 256, 0, s>>>(d_inout, d_norm_input, nrows, ncols, d_buff);
-    }
-    BFS_LAUNCH_CHECK("k_clean_normalize");
-    return BFS_OK;
+    return clean<false>(d_inout, nrows, ncols, d_buff, d_norm_input, as_stream(stream));
+}
+
+bfs_status bfs::clean_rows(float* x, int nrows, int ncols, float* buff, float* row_mask, cudaStream_t s) {
+    return clean<true>(x, nrows, ncols, buff, row_mask, s);
 }
 
 extern "C" bfs_status bfs_fdmt_normalize(const float* d_fdmt, const float* d_norm, int64_t n,
