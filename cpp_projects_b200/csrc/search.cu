@@ -191,7 +191,8 @@ inline int window_class(int w) {
 constexpr int kPairStarts = 2;                            // starts per lane
 constexpr int kPairWarps = 4;
 constexpr int kPairThreads = 32 * kPairWarps;
-constexpr int kPairTile = kPairThreads * kPairStarts;     // starts per tile (256)
+constexpr int kPairWarpTile = 32 * kPairStarts;           // starts per warp
+constexpr int kPairTile = kPairWarps * kPairWarpTile;     // starts per tile (256)
 
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
     unsigned long long d;
