@@ -18,7 +18,8 @@
 //
 // Reduced precision (opt-in, BFS_PREC_F16 / BFS_PREC_BF16): the planes that
 // reach HBM between levels are stored as 16-bit values with a 128-byte row
-// pitch; every sum is still formed in FP32 and the last level writes FP32.
+// pitch; every stored value is an FP32 sum rounded once (fdmt_run16.cu forms
+// the same bits in 16 bits) and the last level writes FP32.
 // Row g of a stored plane holds v_g * 2^-e_g, e_g = ceil(log2(channels summed
 // into row g)): a power-of-two per-row scale (exact, so it adds no rounding)
 // that keeps the stored value within the input's own range (the row's channel

@@ -14,10 +14,12 @@
 // (a prefix-sum difference rounds differently and would flip candidates at
 // the threshold).
 //
-// Compaction: lanes that pass a test are appended with one atomicAdd per warp
-// (ballot + popc); the set of candidates is deterministic, their order is not,
-// so the list is then sorted by the canonical key (mdt, mt, width) — the
-// reference's heap order — with a stable device radix sort.
+// Compaction, in the canonical order (mdt, mt, width), the reference's heap
+// order.  Width sets of k_boxcar_pair: a filter lists the tiles that can hold a
+// candidate, each tile's candidates are one block in that order and a scan
+// places the blocks.  Other width sets (k_boxcar): lanes that pass a test are
+// appended with one atomicAdd per warp, and the list is sorted by the key with a
+// stable device radix sort.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 

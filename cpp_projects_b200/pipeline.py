@@ -23,9 +23,9 @@ from .fdmt import CFdmtGpu
 
 
 def fdmt_launches(plan: CFdmtGpu) -> int:
-    """Kernels one FDMT launches: level 0 (or the fused head over the first
-    ``depth`` levels), then one per merge pass (a plain level or a fused
-    segment of several levels)."""
+    """Kernels one FDMT launches, at most: level 0 (or the fused head over the
+    first ``depth`` levels; none where the first segment forms level 0), then
+    one per merge pass (a plain level or a segment of several levels)."""
     return 1 + plan.info.hbm_passes
 
 
@@ -121,8 +121,8 @@ class SearchPipeline:
         search.launch_row_stats(plane, stats)
         cands, n = search.boxcar_gather(plane, self.thr, self.widths_mode, self.param,
                                         stats=stats, out=self.cands)
-        # FDMT, row statistics, boxcar, canonical sort (keys + gather),
-        # clustering (3 passes x keys/flags/scatter, offsets, delegates, delegate keys)
+        # FDMT, row statistics, boxcar filter and search, compaction, clustering
+        # (3 passes x marks/table, keys, offsets, delegates, delegate keys)
         self.launches += fdmt_launches(self.plans[i]) + 2 + (2 if n >= 2 else 0) + (12 if n else 0)
         if n == 0:
             return BeamResult(0, np.zeros(0, search.CAND_DTYPE), np.zeros(0, np.int64))
@@ -186,10 +186,10 @@ class BatchedSearch:
 
     def launches_per_run(self, n_candidates: int) -> int:
         """Kernels of this library one run launches (CUB's not counted): per
-        beam the FDMT, row statistics and boxcar; then the tagged sort (keys
-        + gather), clustering (3 passes x keys/flags/scatter, offsets,
-        delegate lanes/tree, delegate keys) and the per-beam split (inverse
-        permutation, delegate info, permutation, beam bounds)."""
+        beam the FDMT, row statistics and boxcar search; then the records'
+        compaction, clustering (3 passes, offsets, delegate lanes/tree,
+        delegate keys) and the per-beam split (inverse permutation, delegate
+        info, permutation, beam bounds)."""
         import ctypes
         k = 0
         for d in self._descs:

@@ -64,8 +64,8 @@ bfs_status bfs_trim_scratch(void);
 enum { BFS_PLAN_KEITH = 0, BFS_PLAN_PRAVIR = 1 };
 /* Storage of the FDMT planes between levels (no reference counterpart: the
  * reference is FP32 throughout).  F16 / BF16 store those planes as 16-bit
- * values, row g scaled by 2^-ceil(log2(channels summed into g)); sums are
- * formed in FP32 and the output is FP32.  F32 is the default and the only
+ * values, row g scaled by 2^-ceil(log2(channels summed into g)); every stored
+ * value is the FP32 sum's, rounded to 16 bits, and the output is FP32.  F32 is the default and the only
  * precision bit-identical to the reference. */
 enum { BFS_PREC_F32 = 0, BFS_PREC_F16 = 1, BFS_PREC_BF16 = 2 };
 enum { BFS_FDMT_EXTERNAL_WS = 1 };
