@@ -437,30 +437,23 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         split(a, v[0], v[1]);
         split(b, v[2], v[3]);
     };
-    // leaf i of consecutive rows is often the same row: extended where it was
-    // added last (at[i]) instead of added again
-    auto add = [](std::vector<Row>& v, int (&at)[4], int i, int row, int lo, int hi) {
-        if (at[i] >= 0 && v[at[i]].row == row) {
-            v[at[i]].lo = std::min(v[at[i]].lo, lo);
-            v[at[i]].hi = std::max(v[at[i]].hi, hi);
+    // each row once: at[row] = its place, -1 where there is none yet
+    auto add = [](std::vector<Row>& v, std::vector<int>& at, int row, int lo, int hi) {
+        if (at[row] >= 0) {
+            Row& r = v[at[row]];
+            r.lo = std::min(r.lo, lo);
+            r.hi = std::max(r.hi, hi);
         } else {
-            at[i] = static_cast<int>(v.size());
+            at[row] = static_cast<int>(v.size());
             v.push_back({row, lo, hi});
         }
     };
-    auto unite = [](std::vector<Row>& v) {       // sorted by row, one entry per row
+    auto sorted = [](std::vector<Row>& v, std::vector<int>& at) {
+        for (const Row& r : v) at[r.row] = -1;
         std::sort(v.begin(), v.end(), [](const Row& a, const Row& b) { return a.row < b.row; });
-        size_t k = 0;
-        for (size_t i = 0; i < v.size(); ++i) {
-            if (k && v[k - 1].row == v[i].row) {
-                v[k - 1].lo = std::min(v[k - 1].lo, v[i].lo);
-                v[k - 1].hi = std::max(v[k - 1].hi, v[i].hi);
-            } else {
-                v[k++] = v[i];
-            }
-        }
-        v.resize(k);
     };
+    std::vector<int> at_mid(p.lv[lm].total_rows(), -1);
+    std::vector<int> at_in(from_input ? p.nchan : p.lv[l0].total_rows(), -1);
     const std::vector<std::pair<int, int>> cuts = row_cuts(p.lv[l1], G);
     struct Tile { int g0, g1; std::vector<Row> mid, in; };
     std::vector<Tile> tiles;
@@ -470,14 +463,12 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         Tile t;
         t.g0 = c.first; t.g1 = c.second;
         Leaf v[4];
-        int at[4] = {-1, -1, -1, -1};
         for (int g = t.g0; g < t.g1; ++g) {
             leaves(l1, g, s.s2, v);
-            for (int i = 0; i < 4; ++i)
-                if (v[i].row >= 0) add(t.mid, at, i, v[i].row, v[i].shift, v[i].shift);
+            for (const Leaf& x : v)
+                if (x.row >= 0) add(t.mid, at_mid, x.row, x.shift, x.shift);
         }
-        unite(t.mid);
-        std::fill(at, at + 4, -1);
+        sorted(t.mid, at_mid);
         // one window per sub-band of the mid level
         for (size_t i = 0; i < t.mid.size();) {
             const int band = static_cast<int>(std::upper_bound(mcum.begin(), mcum.end(), t.mid[i].row) - mcum.begin()) - 1;
@@ -492,18 +483,17 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         }
         for (const Row& r : t.mid) {
             leaves(lm, r.row, s.s1, v);
-            for (int i = 0; i < 4; ++i) {
-                const Leaf& x = v[i];
+            for (const Leaf& x : v) {
                 if (x.row < 0) continue;
                 if (from_input) {
                     const int c = chan_of(x.row);
-                    add(t.in, at, i, c, r.lo + x.shift, r.hi + x.shift + x.row - ccum[c]);
+                    add(t.in, at_in, c, r.lo + x.shift, r.hi + x.shift + x.row - ccum[c]);
                 } else {
-                    add(t.in, at, i, x.row, r.lo + x.shift, r.hi + x.shift);
+                    add(t.in, at_in, x.row, r.lo + x.shift, r.hi + x.shift);
                 }
             }
         }
-        unite(t.in);
+        sorted(t.in, at_in);
         for (Row& r : t.in) {
             // first sample t0 - hi on a 16-byte boundary (t0 a multiple of 8)
             const int phase = from_input ? static_cast<int>((static_cast<long long>(r.row) * p.ncols) & 3) : 0;
@@ -529,12 +519,11 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
     ++s.max_ent;   // (the kernel reads one entry ahead)
     s.smem_bytes = static_cast<size_t>(s.ent0) * esize + 2 * static_cast<size_t>(s.max_ent) * 16;
     if (s.smem_bytes > smem_limit) return false;
-    auto slot_of = [](const std::vector<Row>& v, int row) {
-        return static_cast<int>(std::lower_bound(v.begin(), v.end(), row, [](const Row& w, int r) { return w.row < r; }) -
-                                v.begin());
+    auto place = [](const std::vector<Row>& v, std::vector<int>& at) {
+        for (size_t j = 0; j < v.size(); ++j) at[v[j].row] = static_cast<int>(j);
     };
     // one stage's entries; prev = the inputs of the row before
-    auto entries = [&](int level, int levels, const std::vector<Row>& from, int base, int pitch, int zero, bool chan,
+    auto entries = [&](int level, int levels, const std::vector<Row>& from, const std::vector<int>& at, int base, int pitch, int zero, bool chan,
                        int row, int hi, int (&prev)[4]) {
         Leaf v[4];
         leaves(level, row, levels, v);
@@ -542,7 +531,7 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
             int e = zero * esize;
             if (v[i].row >= 0) {
                 const int src = chan ? chan_of(v[i].row) : v[i].row, r = chan ? v[i].row - ccum[src] : 0;
-                const int j = slot_of(from, src);
+                const int j = at[src];
                 const int off = from[j].hi - hi - v[i].shift;
                 if (off < r || off + tile > pitch) return false;
                 e = (base + j * pitch + off) * esize | (r << 20);
@@ -562,11 +551,13 @@ bool build_run_plan(const FdmtPlanHost& p, int l0, int l1, int G, size_t smem_li
         r.out0 = t.g0;
         for (const Row& w : t.in) s.rows.insert(s.rows.end(), {w.row, w.hi});
         int prev[4] = {-1, -1, -1, -1};
+        place(t.in, at_in);
+        place(t.mid, at_mid);
         for (const Row& w : t.mid)
-            if (!entries(lm, s.s1, t.in, 0, s.pitch_x, s.zero_x, from_input, w.row, w.hi, prev)) return false;
+            if (!entries(lm, s.s1, t.in, at_in, 0, s.pitch_x, s.zero_x, from_input, w.row, w.hi, prev)) return false;
         for (int& x : prev) x = -1;
         for (int g = t.g0; g < t.g1; ++g)
-            if (!entries(l1, s.s2, t.mid, s.y0, mid, s.zero_y, false, g, 0, prev)) return false;
+            if (!entries(l1, s.s2, t.mid, at_mid, s.y0, mid, s.zero_y, false, g, 0, prev)) return false;
         s.tiles.push_back(r);
     }
     *out = std::move(s);
