@@ -20,6 +20,7 @@ BFS_WIDTHS_POW2, BFS_WIDTHS_ALL = 0, 1
 BFS_FDMT_EXTERNAL_WS = 1
 BFS_FUSE_AUTOTUNE = -2
 BFS_SEG_SINGLE_BUFFER = 1
+BFS_SEG_RUN16 = 2
 BFS_PREC_F32, BFS_PREC_F16, BFS_PREC_BF16 = 0, 1, 2
 BFS_PLAN_KEITH, BFS_PLAN_PRAVIR = 0, 1
 

@@ -35,6 +35,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <tuple>
 
 #include "divide.cuh"
@@ -1278,7 +1279,9 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
             kSegMaxLevels);
     BFS_ARG(desc->seg_rows >= 0, "seg_rows %d is negative", desc->seg_rows);
     const bool explicit_seg = desc->seg_levels >= 2 || desc->seg_rows > 0;
-    BFS_ARG((desc->seg_flags & ~BFS_SEG_SINGLE_BUFFER) == 0, "unknown seg_flags 0x%x", desc->seg_flags);
+    BFS_ARG((desc->seg_flags & ~(BFS_SEG_SINGLE_BUFFER | BFS_SEG_RUN16)) == 0, "unknown seg_flags 0x%x", desc->seg_flags);
+    BFS_ARG((desc->seg_flags & BFS_SEG_RUN16) == 0 || (p->precision != BFS_PREC_F32 && desc->seg_levels == 0),
+            "BFS_SEG_RUN16 is for 16-bit plans with seg_levels 0");
     const bool single = (desc->seg_flags & BFS_SEG_SINGLE_BUFFER) != 0;
     BFS_ARG(desc->seg_threads == 0 || desc->seg_threads == 256 || desc->seg_threads == 512 ||
                 desc->seg_threads == 1024,
@@ -1295,7 +1298,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
     };
     // a fused pass runs as a run segment where one fits two CTAs on an SM,
     // unless the description names a CTA size or buffering of k_fdmt_seg
-    const bool run_ok = desc->seg_threads == 0 && desc->seg_flags == 0;
+    const bool run_ok = desc->seg_threads == 0 && !single;
     const int esize = elem_bytes_of(p->precision);
     auto run_alone = [&](int l0, int l1, bool from_input) {
         if ((tables && esize == 4 && !(from_input && h.kind == BFS_PLAN_PRAVIR)) || !run_ok) return false;
@@ -1401,9 +1404,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
     return BFS_OK;
 }
 
-// `tuned`: desc is the autotuner's own choice.
-static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_fdmt_plan>& p, bool tables,
-                                 bool tuned = false) {
+static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_fdmt_plan>& p, bool tables) {
     BFS_ARG(desc != nullptr, "null argument");
     BFS_ARG(desc->plan_kind == BFS_PLAN_KEITH || desc->plan_kind == BFS_PLAN_PRAVIR,
             "unsupported plan_kind %d", desc->plan_kind);
@@ -1455,12 +1456,10 @@ static bfs_status plan_host_part(const bfs_fdmt_desc* desc, std::unique_ptr<bfs_
             return BFS_OK;
     }
     p->fuse_depth = p->head.depth;
-    // (16-bit plans: with an explicit depth 0 or one level per pass, plain passes)
-    const bool runs16 = desc->seg_levels == 0 && (tuned || desc->fuse_depth != 0);
+    // (16-bit plans: one level per pass, or an explicit depth 0 that does not ask for them, plain passes)
+    const bool runs16 = desc->seg_levels == 0 && (desc->fuse_depth != 0 || (desc->seg_flags & BFS_SEG_RUN16) != 0);
     return build_passes(desc, p.get(), kSegDefaultLevels, tables, runs16);
 }
-
-static inline int bfs_fdmt_plan_depth_of(int d) { return d; }
 
 // ---------------------------------------------------------------------------
 // Autotuner: head depth and tile, or the first segment forming level 0, then
@@ -1508,7 +1507,8 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
     bfs_fdmt_desc d0 = base;
     d0.fuse_depth = -1;
     d0.head_tile = d0.seg_levels = d0.seg_rows = d0.seg_threads = d0.seg_flags = 0;
-    const bool runs = plan_host_part(&d0, probe, false) == BFS_OK && !probe->runs.empty() && probe->runs[0].s1 > 0;
+    const bool runs = base.precision == BFS_PREC_F32 && plan_host_part(&d0, probe, false) == BFS_OK &&
+                      !probe->runs.empty() && probe->runs[0].s1 > 0;
     if (runs) {
         for (int seg : {4, 3, 2}) cands.push_back({0, 0, seg, 32, 0});
     } else {
@@ -1545,33 +1545,25 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
         st = fail(BFS_ERR_ALLOC, "autotune: cannot allocate scratch for a %dx%d FDMT", base.nchan, base.ncols);
     }
     if (st == BFS_OK) cudaMemsetAsync(d_in, 0, in_n * sizeof(float), s);
-    // (16-bit plans: the depth, which decides where values are rounded, is
-    // chosen on one plain pass per level; run segments then serve it)
-    for (const Cand& c : cands) {
-        if (st != BFS_OK) break;
-        bfs_fdmt_desc d = base;
-        d.fuse_depth = c.depth;
-        d.head_tile = c.tile;
-        d.seg_levels = c.seg;
-        d.seg_rows = c.rows;
-        d.seg_threads = 0;
-        d.seg_flags = c.flags;
-        d.flags = BFS_FDMT_EXTERNAL_WS;
+    // ms of one schedule of this shape; no value where it cannot be created or run
+    auto time_desc = [&](const bfs_fdmt_desc& d, bool fused_only) -> std::optional<float> {
         bfs_fdmt_plan* p = nullptr;
-        if (bfs_fdmt_plan_create(&d, &p) != BFS_OK) continue;  // depth/tile not usable here
+        if (bfs_fdmt_plan_create(&d, &p) != BFS_OK) return {};   // depth/tile not usable here
+        std::unique_ptr<bfs_fdmt_plan, bfs_status (*)(bfs_fdmt_plan*)> own(p, bfs_fdmt_plan_destroy);
         size_t need = 0;
         bfs_fdmt_workspace_size(p, &need);
         if (need > ws_bytes) {
             if (ws) cudaFree(ws);
             ws = nullptr;
-            if (cudaMalloc(&ws, need) != cudaSuccess) { bfs_fdmt_plan_destroy(p); ws_bytes = 0; continue; }
+            ws_bytes = 0;
+            if (cudaMalloc(&ws, need) != cudaSuccess) return {};
             ws_bytes = need;
         }
-        float ms = 1e30f;
         // a segment length that fell back to plain levels duplicates seg = 1
         bool fused = false;
         for (const SegPlan& sp : p->passes) fused |= !sp.tiles.empty();
-        if (c.seg > 1 && !fused) { bfs_fdmt_plan_destroy(p); continue; }
+        if (fused_only && !fused) return {};
+        float ms = 1e30f;
         bool ok = bfs_fdmt_execute_ws(p, d_in, d_out, 0, ws, ws_bytes, s) == BFS_OK;
         for (int rep = 0; rep < 2 && ok; ++rep) {
             cudaEventRecord(e0, s);
@@ -1582,8 +1574,42 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
             cudaEventElapsedTime(&t, e0, e1);
             ms = std::min(ms, t);
         }
-        bfs_fdmt_plan_destroy(p);
-        if (ok && ms < win.ms) win = TuneVal{bfs_fdmt_plan_depth_of(c.depth), c.tile, c.seg, c.rows, c.flags, ms};
+        if (!ok) return {};
+        return ms;
+    };
+    auto desc_of = [&](const TuneVal& c) {
+        bfs_fdmt_desc d = base;
+        d.fuse_depth = c.depth;
+        d.head_tile = c.tile;
+        d.seg_levels = c.seg;
+        d.seg_rows = c.rows;
+        d.seg_threads = 0;
+        d.seg_flags = c.flags;
+        d.flags = BFS_FDMT_EXTERNAL_WS;
+        return d;
+    };
+    bool timed = false;
+    for (const Cand& c : cands) {
+        if (st != BFS_OK) break;
+        TuneVal v{c.depth, c.tile, c.seg, c.rows, c.flags, 1e30f};
+        const std::optional<float> ms = time_desc(desc_of(v), c.seg > 1);
+        if (!ms) continue;
+        timed = true;
+        v.ms = *ms;
+        if (v.ms < win.ms) win = v;
+    }
+    // 16-bit plans: the depth decides where values are rounded, so it is the
+    // plain passes' (one per level) best; run segments give their bits and
+    // serve it where they are the faster ones
+    if (timed && base.precision != BFS_PREC_F32) {
+        TuneVal v = win;
+        v.seg = 0;
+        v.flags = BFS_SEG_RUN16;
+        const std::optional<float> ms = time_desc(desc_of(v), false);
+        if (ms && *ms < win.ms) {
+            v.ms = *ms;
+            win = v;
+        }
     }
     if (ws) cudaFree(ws);
     if (d_in) cudaFree(d_in);
@@ -1592,10 +1618,10 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
     if (e1) cudaEventDestroy(e1);
     cudaGetLastError();
     if (st != BFS_OK) return st;
-    if (base.precision != BFS_PREC_F32) win.seg = 0;
+    *best = win;
+    if (!timed) return BFS_OK;   // (no memory for any: one plain pass per level, not kept)
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune[tune_key(base)] = win;
-    *best = win;
     return BFS_OK;
 }
 
@@ -1653,7 +1679,7 @@ extern "C" bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc_in, bfs_fdm
     }
     const bfs_fdmt_desc* desc = &tuned;
     std::unique_ptr<bfs_fdmt_plan> p;
-    bfs_status st = plan_host_part(desc, p, desc_in->seg_rows > 0, desc_in->fuse_depth == BFS_FUSE_AUTOTUNE);
+    bfs_status st = plan_host_part(desc, p, desc_in->seg_rows > 0);
     if (st != BFS_OK) return st;
     p->host_only = false;
     BFS_CUDA(cudaGetDevice(&p->device));

@@ -20,9 +20,9 @@ from ._tensors import dev_ptr, stream_handle
 
 
 def autotune(Fmin: float, Fmax: float, nchan: int, cols: int, imaxDt: int) -> tuple[int, int, float]:
-    """Time the fused-head depths, tile widths and merge-segment lengths for
-    this shape on the current device (cached per shape): returns
-    (fuse_depth, head_tile, ms)."""
+    """Time the schedules of this shape on the current device (run segments of
+    2-4 levels; without them fused-head depths, tile widths and segment
+    lengths; cached per shape): returns (fuse_depth, head_tile, ms)."""
     desc = _capi.FdmtDesc(fmin=float(Fmin), fmax=float(Fmax), nchan=int(nchan), ncols=int(cols),
                           max_dt=int(imaxDt))
     depth, tile, ms = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_float(0)
@@ -32,7 +32,7 @@ def autotune(Fmin: float, Fmax: float, nchan: int, cols: int, imaxDt: int) -> tu
 
 
 def autotune_desc(desc: "_capi.FdmtDesc") -> tuple["_capi.FdmtDesc", float]:
-    """The tuned description (fuse_depth, head_tile, seg_levels, seg_rows
+    """The tuned description (fuse_depth, head_tile and the seg_ fields
     filled in) of `desc` on the current device, and its time in ms."""
     out = _capi.FdmtDesc()
     ms = ctypes.c_float(0)

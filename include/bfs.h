@@ -90,8 +90,9 @@ typedef struct bfs_fdmt_desc {
     float tsamp;       /* BFS_PLAN_PRAVIR: sample time (s), for the DM grid only       */
     int seg_levels;    /* merge levels fused per HBM pass after the head: FP32 plans 0: 3;
                           1: one pass per level; 2..6.  16-bit plans 0: up to 4 with a
-                          head or the default schedule, where every row of a level sums
-                          equally many channels, else one; 1: one pass per level         */
+                          head, the default schedule or BFS_SEG_RUN16, where every row of
+                          a level sums equally many channels, else one; 1: one pass per
+                          level                                                          */
     int seg_rows;      /* output rows per tile of a fused pass (0: the most that keep
                           two CTAs per SM, of 64 / 32 / 16; run segments choose theirs) */
     int seg_threads;   /* 0 with seg_flags 0: passes of 2..4 levels are run segments
@@ -100,9 +101,11 @@ typedef struct bfs_fdmt_desc {
     int seg_flags;     /* BFS_SEG_SINGLE_BUFFER: the one-level-at-a-time segment kernel
                           with one input buffer per CTA (the next
                           tile loads after the current one is merged; half the shared
-                          memory, so two CTAs fit an SM)                                 */
+                          memory, so two CTAs fit an SM).  BFS_SEG_RUN16: 16-bit plans
+                          with seg_levels 0 run up to 4 levels per pass with an explicit
+                          fuse_depth 0 too (the same bits)                               */
 } bfs_fdmt_desc;
-enum { BFS_SEG_SINGLE_BUFFER = 1 };
+enum { BFS_SEG_SINGLE_BUFFER = 1, BFS_SEG_RUN16 = 2 };
 
 typedef struct bfs_fdmt_plan bfs_fdmt_plan;
 
@@ -126,11 +129,14 @@ bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc, bfs_fdmt_plan** plan)
  * 3 and 4 levels (plans without them: fusion depths {0,2,3,4,5} x
  * head tiles {256,512} x merge segments of 1..4 levels) on this shape with
  * zero input (the kernels' cost does not depend on the values) and returns the fastest;
- * results are cached per (nchan, max_dt, band, ncols rounded up to 2^k). */
+ * results are cached per (nchan, max_dt, band, ncols rounded up to 2^k).  16-bit plans:
+ * depth and tile are the fastest with one plain pass per level (the depth decides where
+ * values are rounded); run segments are chosen where they then are faster. */
 bfs_status bfs_fdmt_autotune(const bfs_fdmt_desc* desc, int* depth, int* head_tile, float* ms);
 /* The same measurement over fusion depth, head tile and fused merge-segment
- * length (1..4 levels per HBM pass, FP32): *tuned = *desc with fuse_depth,
- * head_tile, seg_levels and seg_rows set to the fastest (cached per shape). */
+ * length (1..4 levels per HBM pass): *tuned = *desc with fuse_depth,
+ * head_tile and the seg_ fields set to the fastest, which give the schedule that
+ * BFS_FUSE_AUTOTUNE runs (cached per shape). */
 bfs_status bfs_fdmt_autotune_desc(const bfs_fdmt_desc* desc, bfs_fdmt_desc* tuned, float* ms);
 /* Same plan without device resources (introspection only; execute fails). */
 bfs_status bfs_fdmt_plan_create_host(const bfs_fdmt_desc* desc, bfs_fdmt_plan** plan);
