@@ -1299,9 +1299,12 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
     // a fused pass runs as a run segment where one fits two CTAs on an SM,
     // unless the description names a CTA size or buffering of k_fdmt_seg
     const bool run_ok = desc->seg_threads == 0 && !single;
+    // where k_fdmt_seg's tables do not fit, a pass is still a run segment, as
+    // it is without them, unless the description names the rows of its tiles
+    const bool no_tables_ok = tables && desc->seg_rows == 0;
     const int esize = elem_bytes_of(p->precision);
-    auto run_alone = [&](int l0, int l1, bool from_input) {
-        if ((tables && esize == 4 && !(from_input && h.kind == BFS_PLAN_PRAVIR)) || !run_ok) return false;
+    auto run_alone = [&](int l0, int l1, bool from_input, bool want_tables) {
+        if ((want_tables && esize == 4 && !(from_input && h.kind == BFS_PLAN_PRAVIR)) || !run_ok) return false;
         RunPlan rp;
         plan_run(h, l0, l1, from_input, &rp, esize);
         if (rp.s1 == 0) return false;
@@ -1327,7 +1330,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
         int l0 = k;
         for (int i = 0; i < nseg; ++i) {
             const int l1 = l0 + left / nseg + (i < left % nseg ? 1 : 0);
-            if (!run_alone(l0, l1, false)) break;
+            if (!run_alone(l0, l1, false, tables)) break;
             l0 = l1;
         }
         for (int l = l0 + 1; l <= h.niter; ++l) plain(l);
@@ -1341,7 +1344,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
             // no head: the first segment reads the channels and forms level 0
             // itself (no level-0 plane), where the plan's level 0 allows it
             if (i == 0 && k == 0 && l1 >= 2) {
-                bool ok = run_alone(0, l1, true);
+                bool ok = run_alone(0, l1, true, tables);
                 for (int G : {desc->seg_rows > 0 ? desc->seg_rows : 32, 16}) {
                     for (size_t limit : {kHeadSmemTwoPerSm, kHeadSmemMax}) {
                         SegPlan sp;
@@ -1351,6 +1354,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
                         }
                     }
                 }
+                if (!ok && no_tables_ok) ok = run_alone(0, l1, true, false);
                 if (ok) {
                     l0 = l1;
                     continue;
@@ -1358,7 +1362,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
             }
             if (l1 == l0 + 1) {
                 plain(l1);
-            } else if (!run_alone(l0, l1, false)) {
+            } else if (!run_alone(l0, l1, false, tables)) {
                 // rows per tile: the most that keep two CTAs per SM, else one
                 std::vector<std::pair<int, size_t>> rows_try = {
                     {64, kHeadSmemTwoPerSm}, {32, kHeadSmemTwoPerSm}, {16, kHeadSmemTwoPerSm},
@@ -1373,6 +1377,7 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
                         break;
                     }
                 }
+                if (!ok && no_tables_ok) ok = run_alone(l0, l1, false, false);
                 BFS_ARG(ok || !explicit_seg, "seg_levels %d / seg_rows %d are not usable for this plan",
                         desc->seg_levels, desc->seg_rows);
                 if (!ok)
@@ -1510,8 +1515,24 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
     const bool runs = base.precision == BFS_PREC_F32 && plan_host_part(&d0, probe, false) == BFS_OK &&
                       !probe->runs.empty() && probe->runs[0].s1 > 0;
     if (runs) {
-        for (int seg : {4, 3, 2}) cands.push_back({0, 0, seg, 32, 0});
-    } else {
+        // (named with 32 rows as before where that description is accepted;
+        // run segments choose their own)
+        for (int seg : {4, 3, 2})
+            for (int rows : {32, 0}) {
+                bfs_fdmt_desc d = d0;
+                d.fuse_depth = 0;
+                d.seg_levels = seg;
+                d.seg_rows = rows;
+                if (plan_host_part(&d, probe, true) != BFS_OK) continue;
+                cands.push_back({0, 0, seg, rows, 0});
+                // small planes, whose passes cost little more than their launches: after a head, too
+                // (128 x 4000, max delay 32: 13.0 us after three levels, 14.0 without a head)
+                if (seg == 4 && static_cast<long long>(base.nchan) * base.ncols <= (1 << 20) && base.plan_kind == BFS_PLAN_KEITH)
+                    for (int k : {2, 3, 4}) cands.push_back({k, 256, seg, rows, 0});
+                break;
+            }
+    }
+    if (cands.empty()) {
     // one merge pass per level: head depth x head tile
     cands.push_back({0, 0, 1, 0, 0});
     for (int k : {2, 3, 4, 5})
@@ -1552,6 +1573,7 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
         std::unique_ptr<bfs_fdmt_plan, bfs_status (*)(bfs_fdmt_plan*)> own(p, bfs_fdmt_plan_destroy);
         size_t need = 0;
         bfs_fdmt_workspace_size(p, &need);
+        need = std::max<size_t>(need, 256);   // (a plan of one pass needs none, bfs_fdmt_execute_ws wants an address)
         if (need > ws_bytes) {
             if (ws) cudaFree(ws);
             ws = nullptr;
@@ -1561,7 +1583,7 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
         }
         // a segment length that fell back to plain levels duplicates seg = 1
         bool fused = false;
-        for (const SegPlan& sp : p->passes) fused |= !sp.tiles.empty();
+        for (size_t i = 0; i < p->passes.size(); ++i) fused |= !p->passes[i].tiles.empty() || p->runs[i].s1 > 0;
         if (fused_only && !fused) return {};
         float ms = 1e30f;
         bool ok = bfs_fdmt_execute_ws(p, d_in, d_out, 0, ws, ws_bytes, s) == BFS_OK;
