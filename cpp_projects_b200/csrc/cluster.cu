@@ -481,11 +481,13 @@ static bfs_status finish_delegates(const bfs_cand* d_cands, const int* d_perm, u
     BFS_LAUNCH_CHECK("k_delegate_keys");
     size_t b = 0;
     unsigned* dl = reinterpret_cast<unsigned*>(d_delegates);
-    BFS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b, u, u, u, dl, static_cast<int>(ng), 0, tbits, s));
+    // (one start for all: CUB still sorts a bit, and its scratch is asked for with the same bits)
+    const int bits = std::max(tbits, 1);
+    BFS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b, u, u, u, dl, static_cast<int>(ng), 0, bits, s));
     void* tmp;
     BFS_TRY(sc.alloc(&tmp, b));
     BFS_CUDA(cub::DeviceRadixSort::SortPairs(tmp, b, u, u + ng, u + 2 * static_cast<size_t>(ng), dl, static_cast<int>(ng),
-                                             0, tbits > 0 ? tbits : 1, s));
+                                             0, bits, s));
     return BFS_OK;
 }
 
