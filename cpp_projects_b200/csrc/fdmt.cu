@@ -255,27 +255,32 @@ __device__ __forceinline__ void ones_counts(float* hist, int d, const int* __res
         if (on) atomicAdd(&hist[__ldg(tr + c)], 1.0f);
     }
     __syncthreads();
-    // inclusive scan, a segment per thread (whole numbers: exact in any order)
-    __shared__ float warp_sum[kOnesThreads / 32];
+    // inclusive scan, a segment per thread (whole numbers: exact in any order),
+    // first within a warp's segments; it has no shared memory but the
+    // histogram, which may be the 48 KB a kernel has without opting in
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int seg = (L + kOnesThreads - 1) / kOnesThreads;
     const int b0 = min(L, static_cast<int>(threadIdx.x) * seg), b1 = min(L, b0 + seg);
     float sum = 0.0f;
     for (int i = b0; i < b1; ++i) sum += hist[i];
-    float pre = sum;
+    float run = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const float v = __shfl_up_sync(0xffffffffu, pre, o);
-        if (lane >= o) pre += v;
+        const float v = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += v;
     }
-    if (lane == 31) warp_sum[warp] = pre;
-    __syncthreads();
-    float run = pre - sum;
-    for (int i = 0; i < warp; ++i) run += warp_sum[i];
+    run -= sum;
     for (int i = b0; i < b1; ++i) {
         run += hist[i];
         hist[i] = run;
     }
+    __syncthreads();
+    // the warps before end with their totals (a thread with a segment has only full ones before it)
+    float before = 0.0f;
+    if (b0 < b1)
+        for (int w = 1; w <= warp; ++w) before += hist[32 * seg * w - 1];
+    __syncthreads();
+    for (int i = b0; i < b1; ++i) hist[i] += before;
     __syncthreads();
 }
 
@@ -1958,7 +1963,7 @@ extern "C" bfs_status bfs_fdmt_workspace_size(const bfs_fdmt_plan* plan, size_t*
     return BFS_OK;
 }
 
-constexpr int kOnesMaxHist = 12 * 1024;  // shared-memory histogram entries (48 KB)
+constexpr int kOnesMaxHist = 12 * 1024;  // shared-memory histogram entries (48 KB: all a kernel has without opting in)
 
 // Uploads the plan's delay table for 0/1 rows on first use; false when the
 // fast path does not apply (histogram too long).
