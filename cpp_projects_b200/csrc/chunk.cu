@@ -50,7 +50,8 @@ struct bfs_chunk {
     int* d_shift = nullptr;  // rows dedispersion shifts
     // chirp factors per coherent DM ([chan][sub-band][mbin]) for the own
     // sub-band transforms, the most recent kChirpCache DMs
-    std::vector<std::pair<double, float2*>> chirps;
+    struct Chirp { double dm; float2* tab; bool filled; };
+    std::vector<Chirp> chirps;
     // other geometries: the factors of the DM loop's first kept_max DMs
     std::vector<double> kept;
     size_t kept_max = 0;
@@ -59,7 +60,7 @@ struct bfs_chunk {
         if (have_fwd) cufftDestroy(fwd);
         if (have_inv) cufftDestroy(inv);
         if (fdmt) bfs_fdmt_plan_destroy(fdmt);
-        for (auto& c : chirps) cudaFree(c.second);
+        for (auto& c : chirps) cudaFree(c.tab);
         for (void* p : {static_cast<void*>(volt), static_cast<void*>(plane), static_cast<void*>(mask),
                         static_cast<void*>(buff), static_cast<void*>(d_shift), static_cast<void*>(kept_tab)})
             if (p) cudaFree(p);
@@ -293,8 +294,8 @@ extern "C" bfs_status bfs_chunk_create(const bfs_chunk_desc* desc, bfs_chunk** o
     BFS_CUDA(cudaMalloc(&c->buff, sizeof(float) * (4 + 2 * static_cast<size_t>(c->rows))));
     BFS_CUDA(cudaMalloc(&c->d_shift, sizeof(int) * c->rows));
     if (!subband_ifft_supported(d.nbin, d.len_sft, d.npol)) {
-        // up to four tables in about half the plane's memory, at least one;
-        // without the memory for them none
+        // up to four tables (8 bytes a factor) in about the plane's memory, at
+        // least one; without the memory for them none
         const size_t n = static_cast<size_t>(d.nchan) * d.nbin;
         c->kept_max = std::min<size_t>(4, std::max<size_t>(1, static_cast<size_t>(c->rows) * c->msamp / (2 * n)));
         if (cudaMalloc(&c->kept_tab, sizeof(float2) * n * c->kept_max) != cudaSuccess) {
@@ -351,21 +352,35 @@ static bool own_subband(const bfs_chunk* c, const void* d_spec) {
            reinterpret_cast<uintptr_t>(d_spec) % 16 == 0;
 }
 
+// Whether what was just launched on s runs, and is not merely recorded by a
+// stream capture that may never be replayed.
+static bool runs_now(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusActive;
+    const bool ok = cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
 // The chirp table of one coherent DM (computed on first use, kept for the
-// chunk's most recent DMs).
+// chunk's most recent DMs; filled once its kernel has been launched).
 static bfs_status chirp_table(bfs_chunk* c, double dm, const float2** out, cudaStream_t s) {
-    for (auto& e : c->chirps)
-        if (e.first == dm) { *out = e.second; return BFS_OK; }
+    size_t at = 0;
+    while (at < c->chirps.size() && c->chirps[at].dm != dm) ++at;
+    if (at < c->chirps.size() && c->chirps[at].filled) { *out = c->chirps[at].tab; return BFS_OK; }
     const bfs_chunk_desc& d = c->d;
-    float2* tab = nullptr;
-    if (c->chirps.size() >= kChirpCache) {   // reuse the oldest table's memory
-        BFS_CUDA(cudaStreamSynchronize(s));
-        tab = c->chirps.front().second;
-        c->chirps.erase(c->chirps.begin());
-    } else {
-        BFS_CUDA(cudaMalloc(&tab, sizeof(float2) * static_cast<size_t>(d.nchan) * d.len_sft * c->mbin));
+    if (at == c->chirps.size()) {
+        float2* mem = nullptr;
+        if (c->chirps.size() >= kChirpCache) {   // reuse the oldest table's memory
+            BFS_CUDA(cudaStreamSynchronize(s));
+            mem = c->chirps.front().tab;
+            c->chirps.erase(c->chirps.begin());
+        } else {
+            BFS_CUDA(cudaMalloc(&mem, sizeof(float2) * static_cast<size_t>(d.nchan) * d.len_sft * c->mbin));
+        }
+        c->chirps.push_back({dm, mem, false});
+        at = c->chirps.size() - 1;
     }
-    c->chirps.emplace_back(dm, tab);
+    float2* tab = c->chirps[at].tab;
     const double bw = static_cast<double>(d.fmax - d.fmin);
     const double bw_sub = bw / d.nchan;
     const double bw_chan = bw_sub / d.len_sft;
@@ -374,6 +389,7 @@ static bfs_status chirp_table(bfs_chunk* c, double dm, const float2** out, cudaS
     k_chirp_table<<<grid, 256, 0, s>>>(tab, dm, d.len_sft, c->mbin, d.nbin, static_cast<double>(d.fmin), bw_sub,
                                        bw_chan);
     BFS_LAUNCH_CHECK("k_chirp_table");
+    c->chirps[at].filled = runs_now(s);
     *out = tab;
     return BFS_OK;
 }
@@ -410,12 +426,12 @@ static bfs_status chunk_voltages(bfs_chunk* c, const void* d_spec, double dm, fl
         while (i < c->kept.size() && c->kept[i] != dm) ++i;
         known = i < c->kept.size();
         if (i < c->kept_max) tab = c->kept_tab + i * n;
-        if (tab && !known) c->kept.push_back(dm);
     }
     k_chirp<<<grid, 256, 0, s>>>(static_cast<const float2*>(d_spec), d_volt, tab, known, dm, d.nchan, d.len_sft,
                                  c->mbin, d.nbin, d.nfft * d.npol / 2, static_cast<double>(d.fmin),
                                  bw_sub, bw_chan);
     BFS_LAUNCH_CHECK("k_chirp");
+    if (tab && !known && runs_now(s)) c->kept.push_back(dm);   // (its table is filled by this launch)
     bfs_status st = cufft_check(cufftSetStream(c->inv, s), "cufftSetStream");
     if (st != BFS_OK) return st;
     return cufft_check(cufftExecC2C(c->inv, reinterpret_cast<cufftComplex*>(d_volt),
