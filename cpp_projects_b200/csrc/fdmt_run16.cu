@@ -150,9 +150,18 @@ __global__ void __launch_bounds__(kThreads16, 2) k_fdmt_run16(const Run16Args a)
             const unsigned dst = sbase + 2u * (j * a.pitch_x);
             for (int c = lane; c < pieces; c += 32) {
                 const int at = ts + 8 * c;
-                if (at >= 0 && at < a.ncols) copy16(dst + 16u * c, src + 8 * c);
-                else *reinterpret_cast<uint4*>(sm16 + 2 * (j * a.pitch_x) + 16 * c) =
-                    at < 0 ? make_uint4(kNegZero, kNegZero, kNegZero, kNegZero) : make_uint4(0u, 0u, 0u, 0u);
+                if (at >= 0 && at + 8 <= a.ncols) {
+                    copy16(dst + 16u * c, src + 8 * c);
+                    continue;
+                }
+                uint4 v = at < 0 ? make_uint4(kNegZero, kNegZero, kNegZero, kNegZero) : make_uint4(0u, 0u, 0u, 0u);
+                if (at >= 0 && at < a.ncols) {   // the row's end: what lies past it may never have been written
+                    const int left = a.ncols - at;
+                    auto cut = [&](unsigned w, int first) { return left > first + 1 ? w : left > first ? w & 0xffffu : 0u; };
+                    v = *reinterpret_cast<const uint4*>(src + 8 * c);
+                    v = make_uint4(cut(v.x, 0), cut(v.y, 2), cut(v.z, 4), cut(v.w, 6));
+                }
+                *reinterpret_cast<uint4*>(sm16 + 2 * (j * a.pitch_x) + 16 * c) = v;
             }
         }
     };
