@@ -40,6 +40,17 @@ def autotune_desc(desc: "_capi.FdmtDesc") -> tuple["_capi.FdmtDesc", float]:
     return out, ms.value
 
 
+def plan_passes(plan) -> list[list[int]]:
+    """[l0, l1, r0c] of every merge pass after the head: a plain level
+    (l1 = l0 + 1) or a fused segment of levels l0+1..l1; r0c > 0 marks an
+    input segment (it reads the channels and forms level 0 itself)."""
+    n = ctypes.c_int(0)
+    _capi.call("bfs_fdmt_plan_passes", plan, ctypes.byref(n), None, 0)
+    p = np.zeros(max(1, n.value) * 13, np.int32)
+    _capi.call("bfs_fdmt_plan_passes", plan, ctypes.byref(n), p.ctypes.data_as(ctypes.c_void_p), p.size)
+    return [[int(p[13 * i]), int(p[13 * i + 1]), int(p[13 * i + 12])] for i in range(n.value)]
+
+
 class CFdmtGpu:
     def __init__(self, Fmin: float, Fmax: float, nchan: int, cols: int, imaxDt: int,
                  fuse_depth: int = -1, external_ws: bool = False, head_tile: int = 0,
@@ -130,14 +141,7 @@ class CFdmtGpu:
 
     # --- plan introspection ------------------------------------------------
     def passes(self) -> list[list[int]]:
-        """[l0, l1, r0c] of every merge pass after the head: a plain level
-        (l1 = l0 + 1) or a fused segment of levels l0+1..l1; r0c > 0 marks an
-        input segment (it reads the channels and forms level 0 itself)."""
-        n = ctypes.c_int(0)
-        _capi.call("bfs_fdmt_plan_passes", self._plan, ctypes.byref(n), None, 0)
-        p = np.zeros(max(1, n.value) * 13, np.int32)
-        _capi.call("bfs_fdmt_plan_passes", self._plan, ctypes.byref(n), p.ctypes.data_as(ctypes.c_void_p), p.size)
-        return [[int(p[13 * i]), int(p[13 * i + 1]), int(p[13 * i + 12])] for i in range(n.value)]
+        return plan_passes(self._plan)
 
     @property
     def sched_bytes(self) -> float:

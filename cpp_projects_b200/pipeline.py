@@ -19,14 +19,24 @@ import torch
 
 from . import search
 from .cluster import complete_clusterization
-from .fdmt import CFdmtGpu
+from .fdmt import CFdmtGpu, plan_passes
 
 
 def fdmt_launches(plan: CFdmtGpu) -> int:
-    """Kernels one FDMT launches, at most: level 0 (or the fused head over the
-    first ``depth`` levels; none where the first segment forms level 0), then
-    one per merge pass (a plain level or a segment of several levels)."""
-    return 1 + plan.info.hbm_passes
+    """Kernels one FDMT launches: level 0 or the fused head over the first
+    ``depth`` levels (none where the first segment forms level 0), then one
+    per merge pass (a plain level or a segment of several levels)."""
+    return _fdmt_launches(plan.passes())
+
+
+def _fdmt_launches(passes: list) -> int:
+    return len(passes) + (0 if passes and passes[0][2] > 0 else 1)
+
+
+# Kernels of one search after the FDMT, at most (CUB's not counted): row
+# statistics, boxcar filter and search; compaction; field ranges, three passes
+# x (marks, table), keys, offsets, delegates (lanes, tree, keys).
+SEARCH_LAUNCHES, COMPACT_LAUNCHES, CLUSTER_LAUNCHES = 3, 1, 12
 
 
 # An FDMT schedule: (fuse_depth, head_tile, seg_levels, seg_rows, seg_threads,
@@ -121,9 +131,8 @@ class SearchPipeline:
         search.launch_row_stats(plane, stats)
         cands, n = search.boxcar_gather(plane, self.thr, self.widths_mode, self.param,
                                         stats=stats, out=self.cands)
-        # FDMT, row statistics, boxcar filter and search, compaction, clustering
-        # (3 passes x marks/table, keys, offsets, delegates, delegate keys)
-        self.launches += fdmt_launches(self.plans[i]) + 2 + (2 if n >= 2 else 0) + (12 if n else 0)
+        self.launches += (fdmt_launches(self.plans[i]) + SEARCH_LAUNCHES + (COMPACT_LAUNCHES if n >= 2 else 0) +
+                          (CLUSTER_LAUNCHES if n else 0))
         if n == 0:
             return BeamResult(0, np.zeros(0, search.CAND_DTYPE), np.zeros(0, np.int64))
         cl = complete_clusterization(cands, self.metrics)
@@ -185,25 +194,23 @@ class BatchedSearch:
         return sum(s.nchan * s.nsamp for s in self.shapes)
 
     def launches_per_run(self, n_candidates: int) -> int:
-        """Kernels of this library one run launches (CUB's not counted): per
-        beam the FDMT, row statistics and boxcar search; then the records'
-        compaction, clustering (3 passes, offsets, delegate lanes/tree,
-        delegate keys) and the per-beam split (inverse permutation, delegate
-        info, permutation, beam bounds)."""
+        """Kernels of this library one run launches, at most (CUB's not counted):
+        per beam the FDMT and SEARCH_LAUNCHES; then the records' compaction,
+        clustering and the per-beam split (inverse permutation, delegate info,
+        permutation, beam bounds)."""
         import ctypes
         k = 0
         for d in self._descs:
-            info = self._capi.FdmtInfo()
             p = ctypes.c_void_p()
             dd = self._capi.FdmtDesc.from_buffer_copy(d)
             if dd.fuse_depth == self._capi.BFS_FUSE_AUTOTUNE:  # the batch's plans: cached choice
                 from .fdmt import autotune_desc
                 dd, _ = autotune_desc(dd)
             self._capi.call("bfs_fdmt_plan_create_host", ctypes.byref(dd), ctypes.byref(p))
-            self._capi.call("bfs_fdmt_plan_info", p, ctypes.byref(info))
+            passes = plan_passes(p)
             self._capi.lib().bfs_fdmt_plan_destroy(p)
-            k += 1 + info.hbm_passes + 2
-        return k + ((2 + 12 + 4) if n_candidates else 0)
+            k += _fdmt_launches(passes) + SEARCH_LAUNCHES
+        return k + ((COMPACT_LAUNCHES + CLUSTER_LAUNCHES + 4) if n_candidates else 0)
 
     def run(self, inputs: list[torch.Tensor], stream=None) -> list[BeamResult]:
         from ._tensors import dev_ptr, stream_handle
