@@ -374,12 +374,20 @@ __global__ void k_gap_offsets(const K* __restrict__ keys, unsigned n, int wbits,
 }
 
 // Stream-ordered scratch: pieces of one block allocated up front, more blocks
-// where it runs out.
+// where it runs out.  What was allocated since a mark can be given back: the
+// kernels that used it come before what takes its place on the stream.
 struct Scratch {
     cudaStream_t s;
     std::vector<void*> ptrs;
     char* at = nullptr;
     size_t left = 0;
+    struct Mark { size_t blocks, left; char* at; };
+    Mark mark() const { return {ptrs.size(), left, at}; }
+    void release(const Mark& m) {
+        for (; ptrs.size() > m.blocks; ptrs.pop_back()) cudaFreeAsync(ptrs.back(), s);
+        at = m.at;
+        left = m.left;
+    }
     bfs_status reserve(size_t bytes) {
         void* p = nullptr;
         bfs_status st = stream_alloc(&p, bytes, s);
@@ -518,8 +526,10 @@ static bfs_status gap_order(const bfs_cand* d_cands, const int* d_group0, unsign
 // Groups as the sorting passes form them, from bitmaps of the (group, field)
 // cells (*done = false: not applicable).  A pass whose metric is negative
 // splits equal values too, and one that needs more than max(2^20, candidates)
-// words (28 bytes of scratch each; the sorting passes take 36 bytes per
-// candidate) is left to the sorting passes.  The groups before a pass are
+// words, or twice that with the passes before, is left to the sorting passes:
+// a word takes 8 bytes of scratch until the end and 20 during its pass, so
+// the whole stays within the 48 bytes per candidate that those take (the
+// final order 32 in place of a pass's 20).  The groups before a pass are
 // bounded by the ranges; where that bound asks for more than 2^16 words the
 // count is read back (one round trip) instead.
 // 0.3 M candidates: two sorting passes 150 us against 45 us.
@@ -536,6 +546,7 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
     const int th = 256;
     const unsigned long long most = std::max<unsigned long long>(1ull << 20, n);
     unsigned long long groups = groups0;   // before the pass, at most
+    unsigned long long held = 0;           // words of the passes before
     bool exact = true;
     using Count = thrust::counting_iterator<unsigned>;
     using Words = thrust::transform_iterator<GapWord, Count, GapState>;
@@ -550,7 +561,8 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
             exact = true;
         }
         const unsigned long long need = groups << (shift - 5);
-        if (shift >= 32 || need > most || need > (1ull << 26)) return BFS_OK;
+        held += need;
+        if (shift >= 32 || need > most || held > 2 * most || need > (1ull << 26)) return BFS_OK;
         const unsigned words = static_cast<unsigned>(need);
         const GapRule rule{shift, static_cast<unsigned>(metrics[f])};
         unsigned* bits;
@@ -561,13 +573,14 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
         BFS_CUDA(cub::DeviceScan::ExclusiveScan(nullptr, tmp_bytes, Words(Count(0u), GapWord{nullptr, 0u}),
                                                 static_cast<GapState*>(nullptr), rule, GapState{0u, 0u, 0u, 0u},
                                                 static_cast<int>(words), s));
-        // one piece: states, table, bits, the scan's own
-        const size_t at_tab = sizeof(GapState) * static_cast<size_t>(words), at_bits = at_tab + sizeof(uint2) * words;
+        BFS_TRY(sc.alloc(reinterpret_cast<void**>(&tab), sizeof(uint2) * static_cast<size_t>(words)));
+        // of this pass alone, one piece: states, bits, the scan's own
+        const Scratch::Mark pass = sc.mark();
+        const size_t at_bits = sizeof(GapState) * static_cast<size_t>(words);
         const size_t at_tmp = (at_bits + sizeof(unsigned) * words + 255) & ~static_cast<size_t>(255);
         char* piece;
         BFS_TRY(sc.alloc(reinterpret_cast<void**>(&piece), at_tmp + tmp_bytes));
         state = reinterpret_cast<GapState*>(piece);
-        tab = reinterpret_cast<uint2*>(piece + at_tab);
         bits = reinterpret_cast<unsigned*>(piece + at_bits);
         tmp = piece + at_tmp;
         BFS_CUDA(cudaMemsetAsync(bits, 0, sizeof(unsigned) * words, s));
@@ -579,6 +592,7 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
                                                 GapState{0u, 0u, 0u, 0u}, static_cast<int>(words), s));
         k_gap_table<<<(words + th - 1) / th, th, 0, s>>>(bits, state, words, rule, tab, total);
         BFS_LAUNCH_CHECK("k_gap_table");
+        sc.release(pass);
         maps.m[f] = GapMap{tab, fmin[f], shift};
         groups = std::min<unsigned long long>(n, groups * (range[f] / (static_cast<long long>(metrics[f]) + 1) + 1));
         exact = false;
@@ -588,11 +602,13 @@ static bfs_status cluster_by_gaps(const bfs_cand* d_cands, unsigned n, const int
     BFS_ARG(ng >= 1 && ng <= n, "bad group count %u", ng);
     const int wbits = bits_for(static_cast<unsigned long long>(range[2]));
     const int end_bit = wbits + bits_for(ng - 1);
+    const Scratch::Mark order = sc.mark();
     if (end_bit <= 32)
         BFS_TRY(gap_order<unsigned>(d_cands, d_group0, n, maps, fmin[2], wbits, end_bit, ng, d_perm, d_offsets, sc, s));
     else
         BFS_TRY(gap_order<unsigned long long>(d_cands, d_group0, n, maps, fmin[2], wbits, end_bit, ng, d_perm, d_offsets,
                                               sc, s));
+    sc.release(order);
     BFS_TRY(finish_delegates(d_cands, d_perm, n, d_offsets, ng, fmin[0],
                              bits_for(static_cast<unsigned long long>(range[0])), d_delegates, sc, s));
     *h_ngroups = ng;
@@ -641,9 +657,11 @@ extern "C" bfs_status bfs_cluster_grouped(const bfs_cand* d_cands, uint32_t n, c
         }
     }
     bool done = false;
+    const Scratch::Mark clean = sc.mark();
     BFS_TRY(cluster_by_gaps(d_cands, n, d_group0, d_group0 ? ngroups0 : 1u, metrics, fmin, frange, d_perm, d_offsets,
                             d_delegates, h_ngroups, sc, s, &done));
     if (done) return BFS_OK;
+    sc.release(clean);
     unsigned long long *k_in, *k_out;
     unsigned *v_in, *v_out, *gid, *flags, *scan;
     BFS_TRY(sc.alloc(reinterpret_cast<void**>(&k_in), sizeof(unsigned long long) * n));
