@@ -81,26 +81,28 @@ __global__ void k_pass_flags(const K* __restrict__ keys, unsigned n, int fbits, 
 }
 
 // Range of each field (biased so signed order is unsigned order), as the
-// complement of the smallest and the largest, both maxima over zeros.  One
+// complement of the smallest and the largest, both maxima over zeros; then the
+// largest initial group (as unsigned).  One
 // atomic per CTA and bound: 38.9 us with one per warp at 0.3 M candidates.
-constexpr int kRangeThreads = 512;
+constexpr int kRangeThreads = 512, kRanges = 7;
 __global__ void __launch_bounds__(kRangeThreads)
-k_field_range(const bfs_cand* __restrict__ c, unsigned n, unsigned* __restrict__ r) {
-    __shared__ unsigned sh[6];
-    if (threadIdx.x < 6) sh[threadIdx.x] = 0u;
+k_field_range(const bfs_cand* __restrict__ c, const int* __restrict__ g0, unsigned n, unsigned* __restrict__ r) {
+    __shared__ unsigned sh[kRanges];
+    if (threadIdx.x < kRanges) sh[threadIdx.x] = 0u;
     __syncthreads();
-    unsigned m[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    unsigned m[kRanges] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const bfs_cand v = c[i];
         const unsigned f[3] = {biased(v.mt), biased(v.mdt), biased(v.mwidth)};
         for (int k = 0; k < 3; ++k) { m[2 * k] = max(m[2 * k], ~f[k]); m[2 * k + 1] = max(m[2 * k + 1], f[k]); }
+        if (g0) m[6] = max(m[6], static_cast<unsigned>(__ldg(g0 + i)));
     }
-    for (int k = 0; k < 6; ++k) {
+    for (int k = 0; k < kRanges; ++k) {
         const unsigned v = __reduce_max_sync(0xffffffffu, m[k]);
         if ((threadIdx.x & 31) == 0) atomicMax(sh + k, v);
     }
     __syncthreads();
-    if (threadIdx.x < 6) atomicMax(r + threadIdx.x, sh[threadIdx.x]);
+    if (threadIdx.x < kRanges) atomicMax(r + threadIdx.x, sh[threadIdx.x]);
 }
 
 __global__ void k_pass_scatter(const unsigned* __restrict__ vals, const unsigned* __restrict__ scan,
@@ -643,14 +645,16 @@ extern "C" bfs_status bfs_cluster_grouped(const bfs_cand* d_cands, uint32_t n, c
     int fmin[3];
     long long frange[3];
     unsigned* range;
+    unsigned top_group = 0;   // largest initial group
     {
-        unsigned h_range[6];
-        BFS_TRY(sc.alloc(reinterpret_cast<void**>(&range), sizeof(unsigned) * 6));
-        BFS_CUDA(cudaMemsetAsync(range, 0, sizeof(unsigned) * 6, s));
+        unsigned h_range[kRanges];
+        BFS_TRY(sc.alloc(reinterpret_cast<void**>(&range), sizeof(unsigned) * kRanges));
+        BFS_CUDA(cudaMemsetAsync(range, 0, sizeof(unsigned) * kRanges, s));
         const int rb = static_cast<int>((n + kRangeThreads - 1) / kRangeThreads);
-        k_field_range<<<std::min(rb, 592), kRangeThreads, 0, s>>>(d_cands, n, range);
+        k_field_range<<<std::min(rb, 592), kRangeThreads, 0, s>>>(d_cands, d_group0, n, range);
         BFS_LAUNCH_CHECK("k_field_range");
-        BFS_TRY(read_back(h_range, range, 6, s));
+        BFS_TRY(read_back(h_range, range, kRanges, s));
+        top_group = h_range[6];
         for (int f = 0; f < 3; ++f) {
             fmin[f] = static_cast<int>(~h_range[2 * f] ^ 0x80000000u);
             frange[f] = static_cast<long long>(static_cast<int>(h_range[2 * f + 1] ^ 0x80000000u)) - fmin[f];
@@ -658,8 +662,10 @@ extern "C" bfs_status bfs_cluster_grouped(const bfs_cand* d_cands, uint32_t n, c
     }
     bool done = false;
     const Scratch::Mark clean = sc.mark();
-    BFS_TRY(cluster_by_gaps(d_cands, n, d_group0, d_group0 ? ngroups0 : 1u, metrics, fmin, frange, d_perm, d_offsets,
-                            d_delegates, h_ngroups, sc, s, &done));
+    // (the gap tables have cells for groups below ngroups0 only; the sorting passes take any)
+    if (!d_group0 || top_group < ngroups0)
+        BFS_TRY(cluster_by_gaps(d_cands, n, d_group0, d_group0 ? ngroups0 : 1u, metrics, fmin, frange, d_perm, d_offsets,
+                                d_delegates, h_ngroups, sc, s, &done));
     if (done) return BFS_OK;
     sc.release(clean);
     unsigned long long *k_in, *k_out;

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 import torch
 
-from cpp_projects_b200 import cluster, search
+from cpp_projects_b200 import _capi, cluster, search
+from cpp_projects_b200._tensors import dev_ptr, stream_handle
 from oracle import pyoracle
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +55,30 @@ def test_scratch_is_bounded(cuda, tmax, dmax, metrics):
     cl = cluster.complete_clusterization(c, metrics)
     used, groups = _pool_high(False) - before, cl.offsets.shape[0] - 1
     assert used <= 48 * n + (64 * 8 + 16) * groups + (8 << 20), (used / n, groups)
+
+
+@pytest.mark.parametrize("top", [4, 7])   # below ngroups0, and ids that fit its bits but not the count
+def test_initial_groups_beyond_the_count(cuda, top):
+    """Ids of 0..ngroups0-1 are asked for; larger ones take the sorting passes, which
+    have no table of them: the groups are those of each id's candidates alone."""
+    rng = np.random.default_rng(top)
+    n, ids = 3000, np.sort(rng.integers(0, top + 1, 3000)).astype(np.int32)
+    ids[-1] = top
+    c = np.zeros(n, pyoracle.CAND_DTYPE)
+    c["mt"], c["mdt"], c["mwidth"] = rng.integers(0, 900, n), rng.integers(0, 60, n), rng.integers(0, 6, n)
+    c["msnr"] = 7.0 + rng.integers(0, 9, n)
+    g0, d = torch.from_numpy(ids).to(cuda), search.cands_from_numpy(c, cuda)
+    perm, dl = torch.empty((2, n), dtype=torch.int32, device=cuda)
+    offs, ng = torch.empty(n + 1, dtype=torch.int32, device=cuda), ctypes.c_uint32(0)
+    metrics = (2, 1, 2)
+    _capi.call("bfs_cluster_grouped", dev_ptr(d), ctypes.c_uint32(n), dev_ptr(g0), ctypes.c_uint32(5),
+               (ctypes.c_int * 3)(*metrics), dev_ptr(perm), dev_ptr(offs), dev_ptr(dl), ctypes.byref(ng), stream_handle())
+    wperm, woffs = [], [0]
+    for i in range(top + 1):
+        at = np.flatnonzero(ids == i)
+        if len(at):
+            p, o, _ = pyoracle.cluster(c[at], metrics)
+            wperm.append(at[p])
+            woffs += [int(v) + at[0] for v in o[1:]]
+    np.testing.assert_array_equal(perm.cpu().numpy(), np.concatenate(wperm))
+    np.testing.assert_array_equal(offs[: ng.value + 1].cpu().numpy(), woffs)
