@@ -44,7 +44,7 @@ long long boxcar_ordered_records(int rows, int cols);
 bfs_status launch_boxcar_ordered(const float* d_plane, int rows, int cols, const float* d_stats, float thr,
                                  const float* d_thr, int mode, int param, int snr_fast, bfs_cand* d_out,
                                  unsigned capacity, unsigned* d_count, unsigned* rec_first, unsigned* rec_count,
-                                 unsigned* work, unsigned* work_n, cudaStream_t s);
+                                 unsigned* work, unsigned* work_n, cudaStream_t s, bool full = false);
 bfs_status compact_ordered(const bfs_cand* src, const unsigned* rec_first, const unsigned* rec_count,
                            long long nrec, const long long* beam_rec, int nb, bfs_cand* dst, int* tags,
                            cudaStream_t s);

@@ -16,8 +16,8 @@
 //
 // Compaction, in the canonical order (mdt, mt, width), the reference's heap
 // order.  Width sets of k_boxcar_pair: a filter lists the tiles that can hold a
-// candidate, each tile's candidates are one block in that order and a scan
-// places the blocks.  Other width sets (k_boxcar): lanes that pass a test are
+// candidate (low thresholds: k_boxcar_full takes them all), each tile's
+// candidates are one block in that order and a scan places the blocks.  Other width sets (k_boxcar): lanes that pass a test are
 // appended with one atomicAdd per warp, and the list is sorted by the key with a
 // stable device radix sort.
 #include <cub/device/device_radix_sort.cuh>
@@ -149,6 +149,8 @@ struct WidthConsts {
     // per filter class (window_class): 0.9999 sqrt(w) of its smallest width
     // in the set, +inf when it holds none
     float cls[8];
+    float lo, hi;            // thresholds in (lo, hi]: no filter (k_boxcar_full)
+    __host__ __device__ bool full(float thr) const { return thr > lo && thr <= hi; }
 };
 
 // ---- filter ---------------------------------------------------------------
@@ -170,6 +172,12 @@ struct WidthConsts {
 inline int window_class(int w) {
     return w == 1 ? 0 : w == 2 ? 1 : w <= 5 ? 2 : w <= 9 ? 3 : w <= 17 ? 4 : w <= 33 ? 5 : w <= 65 ? 6 : 7;
 }
+// Per class the largest of its sums over a tile's pair of rows, in deviations,
+// that three in ten tiles of unit noise exceed.  A threshold whose bound lies
+// below it for a class of the set lists more tiles than the filter saves: a
+// listed tile costs three to four times one of k_boxcar_full, which then
+// searches the plane unfiltered.
+constexpr float kNoiseTop[8] = {3.25f, 6.5f, 8.75f, 11.2f, 15.7f, 23.8f, 38.5f, 65.5f};
 
 // ---- ordered boxcar over row pairs -------------------------------------------
 // The exact search of the tiles the filter lists, writing the candidates of
@@ -391,6 +399,234 @@ k_boxcar_pair(const float* __restrict__ plane, int rows, int cols, const float* 
     }
 }
 
+// ---- unfiltered planes: a tile per warp, eight starts per lane -----------------
+// For thresholds that noise comes near in many tiles.  Bound by the
+// instructions per tile, of which eight starts per lane take a third of
+// k_boxcar_pair's; each warp stages its tile in its own padded shared region
+// and waits for no other.  4096 x 45001 of noise, the whole call: widths 1..32
+// at 4.5 deviations 454 us (918 through the filter), at 3.5 546 (1715), widths
+// 1..128 at 5.0 1017 (2471); at 7.0 the filter's 169 and 294 against 432 and
+// 1001 unfiltered.
+// Down to a threshold of about one few of a lane's windows pass; below it
+// their quotients are a chain, unless the set has one or two widths.
+constexpr int kFullStarts = 8;
+constexpr float kFullLow = 1.0f;
+constexpr int kFullFrom = 2000;   // tiles of row pairs: fewer do not fill the chip with a warp each
+
+// Shared layout of a warp's staged tile: logical float4 f (positions 2f,
+// 2f + 1 of both rows) sits at f + f / 4, one float4 of padding after every
+// four, so the eight lanes of a quarter warp — whose windows start 4 float4s
+// apart — read eight different bank groups.
+__device__ __forceinline__ int pad4(int f) { return f + (f >> 2); }
+
+// pair_widths over kFullStarts starts (f0 = the lane's first logical float4;
+// snr[64 r + 8 j + c] = the S/N of row r's window (start j, width code c)).
+template <int MODE, int WMAX>
+__device__ __forceinline__ void full_widths(const float4* __restrict__ win4, int f0, int tb, int cols, bool edge,
+                                            float thr, float thr_lo, int snr_fast, const WidthConsts& wc,
+                                            unsigned long long (&pass)[2], float (&snr)[128]) {
+    constexpr int S = kFullStarts;
+    constexpr int kPos = S + WMAX - 1;   // positions this lane reads
+    constexpr int kVec = (kPos + 1) / 2; // float4s (two positions each)
+    constexpr int kFullAhead = 4;            // window pairs are read this many steps before use
+    unsigned long long win[2 * kVec];
+    unsigned long long sum[S];
+    constexpr int kPre = (S + kFullAhead + 1) / 2 < kVec ? (S + kFullAhead + 1) / 2 : kVec;
+#pragma unroll
+    for (int v = 0; v < kPre; ++v) {
+        const float4 q = win4[pad4(f0 + v)];
+        win[2 * v] = pack2(q.x, q.y);
+        win[2 * v + 1] = pack2(q.z, q.w);
+    }
+#pragma unroll
+    for (int j = 0; j < S; ++j) sum[j] = 0ull;   // +0.0 in both halves
+#pragma unroll
+    for (int w = 1; w <= WMAX; ++w) {
+        // step w reads positions w - 1 .. w + S - 2; the pair starting at
+        // position w + S - 2 + kFullAhead is fetched now, kFullAhead steps early
+        const int pn = w + S - 2 + kFullAhead;
+        if ((pn & 1) == 0 && pn / 2 >= kPre && pn / 2 < kVec) {
+            const float4 q = win4[pad4(f0 + pn / 2)];
+            win[pn] = pack2(q.x, q.y);
+            win[pn + 1] = pack2(q.z, q.w);
+        }
+#pragma unroll
+        for (int j = 0; j < S; ++j) sum[j] = add2_rn(sum[j], win[j + w - 1]);
+        if (MODE == 0 && (w & (w - 1)) != 0) continue;
+        const float sq = wc.sq[w];
+        // RN(sum / sq) > thr needs sum > RN(RN(thr sq) (1 - 1e-5)) for thr > 0
+        const float lim = thr_lo > -INFINITY ? __fmul_rn(__fmul_rn(thr, sq), 0.99999f) : -INFINITY;
+        float h[2 * S], hm[S];
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+            unpack2(sum[j], h[2 * j], h[2 * j + 1]);
+            hm[j] = fmaxf(h[2 * j], h[2 * j + 1]);   // both rows at start j
+        }
+        float mx = max3f(hm[0], hm[1], hm[2]);
+#pragma unroll
+        for (int k = 3; k + 1 < S; k += 2) mx = max3f(mx, hm[k], hm[k + 1]);
+        if (S % 2 == 0) mx = fmaxf(mx, hm[S - 1]);
+        if (!__any_sync(0xffffffffu, mx > lim)) continue;
+        const int code = (MODE == 1) ? w - 1 : 31 - __clz(w);
+        // windows inside the row: starts j < inside
+        const int inside = edge ? cols - (tb + w - 1) : S;
+        // windows over the bound: a bit each (one code path for all of them)
+        unsigned over = 0;
+#pragma unroll
+        for (int k = 0; k < 2 * S; ++k)
+            if (h[k] > lim && (k >> 1) < inside) over |= 1u << k;
+#pragma unroll 1
+        while (over) {
+            const int k = __ffs(over) - 1;
+            over &= over - 1;
+            float sj = h[0];
+#pragma unroll
+            for (int i = 1; i < 2 * S; ++i)
+                if (i == k) sj = h[i];
+            const float q = snr_fast ? __fdividef(sj, sq) : __fdiv_rn(sj, sq);
+            if (q > thr) {
+                const int r = k & 1, bit = 8 * (k >> 1) + code;
+                pass[r] |= 1ull << bit;
+                snr[64 * r + bit] = q;
+            }
+        }
+    }
+}
+
+template <int MODE, int WMAX>
+__global__ void __launch_bounds__(kPairThreads, WMAX <= 8 ? 8 : WMAX <= 32 ? 6 : WMAX <= 64 ? 4 : 2)
+k_boxcar_full(const float* __restrict__ plane, int rows, int cols, const float* __restrict__ stats,
+              const float* __restrict__ d_thr, float thr_host, float thr_lo_host, int snr_fast, int vec,
+              bfs_cand* __restrict__ out, unsigned capacity, unsigned* __restrict__ d_count,
+              unsigned* __restrict__ rec_first, unsigned* __restrict__ rec_count, const WidthConsts wc) {
+    // staged positions of a warp: every start's windows, a multiple of 4
+    constexpr int kSpan = (kPairTile + WMAX - 1 + 3) / 4 * 4;
+    constexpr int kF4 = kSpan / 2;                      // logical float4s (kSpan positions x 2 rows)
+    __shared__ float4 tile4[kPairWarps][kF4 + kF4 / 4]; // padded (pad4)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wt = blockIdx.x * kPairWarps + warp;     // warp tile
+    const int tw = wt * kPairTile;
+    if (tw >= cols) return;                            // warp-uniform; no other warp is waited for
+    const int row0 = 2 * static_cast<int>(blockIdx.y);
+    const bool has1 = row0 + 1 < rows;
+    const float* x0 = plane + static_cast<size_t>(row0) * cols;
+    const float* x1 = has1 ? x0 + cols : x0;
+    float m0 = 0.0f, s0 = 1.0f, m1 = 0.0f, s1 = 1.0f;
+    if (stats) {
+        m0 = stats[row0]; s0 = stats[rows + row0];
+        if (has1) { m1 = stats[row0 + 1]; s1 = stats[rows + row0 + 1]; }
+    }
+    auto nz = [&](float v, float m, float s) { return stats ? norm_sample(v, m, s) : v; };
+    float4* t4 = tile4[warp];
+    float* tile = reinterpret_cast<float*>(t4);        // position p, row r at 4 pad4(p / 2) + 2 (p % 2) + r
+    const bool interior = tw + kSpan <= cols;
+    if (interior && vec) {
+        // 16-byte loads of both rows, every load in flight before the first use
+        constexpr int kQ = kSpan / 4;                   // float4s per row
+        constexpr int kPer = (kQ + 31) / 32;
+        float4 a[kPer], b[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int q = lane + 32 * k;
+            if (k < kPer - 1 || q < kQ) {
+                a[k] = __ldg(reinterpret_cast<const float4*>(x0 + tw) + q);
+                b[k] = has1 ? __ldg(reinterpret_cast<const float4*>(x1 + tw) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int q = lane + 32 * k;
+            if (k < kPer - 1 || q < kQ) {
+                const float b0 = has1 ? nz(b[k].x, m1, s1) : 0.0f, b1 = has1 ? nz(b[k].y, m1, s1) : 0.0f;
+                const float b2 = has1 ? nz(b[k].z, m1, s1) : 0.0f, b3 = has1 ? nz(b[k].w, m1, s1) : 0.0f;
+                t4[pad4(2 * q)] = make_float4(nz(a[k].x, m0, s0), b0, nz(a[k].y, m0, s0), b1);
+                t4[pad4(2 * q + 1)] = make_float4(nz(a[k].z, m0, s0), b2, nz(a[k].w, m0, s0), b3);
+            }
+        }
+    } else if (interior) {
+        // 4-byte loads (rows not 16-byte aligned), all in flight first
+        constexpr int kPer = (kSpan + 31) / 32;
+        float a[kPer], b[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int p = lane + 32 * k;
+            if (k < kPer - 1 || p < kSpan) {
+                a[k] = __ldg(x0 + tw + p);
+                b[k] = has1 ? __ldg(x1 + tw + p) : 0.0f;
+            }
+        }
+        float2* t2 = reinterpret_cast<float2*>(t4);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int p = lane + 32 * k;
+            if (k < kPer - 1 || p < kSpan)
+                t2[2 * pad4(p >> 1) + (p & 1)] = make_float2(nz(a[k], m0, s0), has1 ? nz(b[k], m1, s1) : 0.0f);
+        }
+    } else {
+        for (int p = lane; p < kSpan; p += 32) {
+            const int t = tw + p;
+            const bool in = t < cols;
+            const int e = 4 * pad4(p >> 1) + 2 * (p & 1);
+            tile[e] = in ? nz(__ldg(x0 + t), m0, s0) : 0.0f;
+            tile[e + 1] = (in && has1) ? nz(__ldg(x1 + t), m1, s1) : 0.0f;
+        }
+    }
+    __syncwarp();
+    float thr = thr_host, thr_lo = thr_lo_host;
+    if (d_thr) {
+        thr = __ldg(d_thr);
+        thr_lo = thr > 0.0f ? thr * 0.99999f : -INFINITY;
+    }
+    const int p0 = lane * kFullStarts;
+    const int tb = tw + p0;
+    const int f0 = p0 / 2;
+    unsigned long long pass[2] = {0ull, 0ull};
+    float snr[128];   // S/N of the passing windows (indexed like their bits)
+    full_widths<MODE, WMAX>(t4, f0, tb, cols, !interior, thr, thr_lo, snr_fast, wc, pass, snr);
+    if (!has1) pass[1] = 0ull;
+
+    // the warp's block: row 0's candidates, then row 1's, lanes in order
+    const unsigned c0 = __popcll(pass[0]), c1 = __popcll(pass[1]);
+    unsigned i0 = c0, i1 = c1;   // inclusive scans over the lanes
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned u0 = __shfl_up_sync(0xffffffffu, i0, d), u1 = __shfl_up_sync(0xffffffffu, i1, d);
+        if (lane >= d) { i0 += u0; i1 += u1; }
+    }
+    const unsigned tot0 = __shfl_sync(0xffffffffu, i0, 31), tot1 = __shfl_sync(0xffffffffu, i1, 31);
+    unsigned first = 0;
+    if (lane == 0) {
+        first = (tot0 + tot1) ? atomicAdd(d_count, tot0 + tot1) : 0u;
+        const int nwt = (cols + kPairTile - 1) / kPairTile;
+        const size_t rec = static_cast<size_t>(row0) * nwt + wt;
+        rec_first[rec] = first;
+        rec_count[rec] = tot0;
+        if (has1) {
+            rec_first[rec + nwt] = first + tot0;
+            rec_count[rec + nwt] = tot1;
+        }
+    }
+    if (tot0 + tot1 == 0) return;   // warp-uniform
+    first = __shfl_sync(0xffffffffu, first, 0);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        unsigned idx = first + (r ? tot0 + i1 - c1 : i0 - c0);
+        unsigned long long m = pass[r];
+        while (m) {   // bit order = (start, width) order
+            const int bit = __ffsll(static_cast<long long>(m)) - 1;
+            m &= m - 1;
+            if (idx < capacity) {
+                const int code = bit & 7;
+                bfs_cand c;
+                c.mt = tb + (bit >> 3); c.mdt = row0 + r; c.mwidth = MODE == 1 ? code + 1 : code;
+                c.msnr = snr[64 * r + bit];
+                out[idx] = c;
+            }
+            ++idx;
+        }
+    }
+}
+
 // b[k] -> sums j blocks further on (block index lane + 32 k + j)
 template <int K>
 __device__ __forceinline__ void block_shift(float (&o)[K], const float (&b)[K], int j, int lane) {
@@ -519,6 +755,10 @@ k_boxcar_filter(const float* __restrict__ plane, int rows, int cols, const float
     const unsigned pt = blockIdx.y * nwt + wt;
     const int row0 = 2 * static_cast<int>(blockIdx.y);
     const float thr = d_thr ? __ldg(d_thr) : thr_host;
+    if (d_thr && wc.full(thr)) {   // (known on the device only: the caller searches unfiltered)
+        if (pt == 0 && lane == 0) work_n[1] = 1u;
+        return;
+    }
     const bool has1 = row0 + 1 < rows;
     bool may = !(thr > 0.0f);
     if (!may) {
@@ -871,11 +1111,13 @@ long long boxcar_ordered_records(int rows, int cols) {
 // d_out in blocks, one per (row, warp tile), each in canonical order; records
 // rec_first / rec_count (boxcar_ordered_records entries, (row, tile) order)
 // locate the blocks for compact_ordered.  work: one entry per row pair and
-// warp tile; *work_n: 0.
+// warp tile; *work_n: 0.  A threshold in device memory (d_thr) may ask for the
+// unfiltered search: work_n[1] (0 before) is then 1, nothing was searched, and
+// the call is to be made again with `full`.
 bfs_status launch_boxcar_ordered(const float* d_plane, int rows, int cols, const float* d_stats, float thr,
                                  const float* d_thr, int mode, int param, int snr_fast, bfs_cand* d_out,
                                  unsigned capacity, unsigned* d_count, unsigned* rec_first, unsigned* rec_count,
-                                 unsigned* work, unsigned* work_n, cudaStream_t s) {
+                                 unsigned* work, unsigned* work_n, cudaStream_t s, bool full) {
     BFS_ARG(d_plane && d_count && rec_first && rec_count && work && work_n, "null argument");
     BFS_ARG(rows >= 1 && cols >= 1, "bad shape %dx%d", rows, cols);
     BFS_ARG((rows + 1) / 2 <= 65535, "rows > 131070 not supported");
@@ -894,7 +1136,18 @@ bfs_status launch_boxcar_ordered(const float* d_plane, int rows, int cols, const
     const dim3 fgrid((cols + kPerCta - 1) / kPerCta, (rows + 1) / 2);
     // the searching kernel's CTAs take the listed tiles in turn
     const int grid = static_cast<int>(std::min<long long>(pairs, 148LL * 8));
+    const int nwidths = mode == BFS_WIDTHS_POW2 ? param + 1 : param;
+    wc.lo = nwidths >= 3 ? kFullLow : 0.0f;
+    wc.hi = 0.0f;
+    for (int c = 0; c < 8 && pairs >= kFullFrom; ++c) wc.hi = std::max(wc.hi, kNoiseTop[c] / wc.cls[c]);
+    const int vec = cols % 4 == 0 && reinterpret_cast<uintptr_t>(d_plane) % 16 == 0 ? 1 : 0;
 #define BFS_BOX_PAIR(M, W)                                                                                        \
+    if (full || (!d_thr && wc.full(thr))) {                                                                       \
+        k_boxcar_full<M, W><<<fgrid, kPairThreads, 0, s>>>(d_plane, rows, cols, d_stats, d_thr, thr, thr_lo,      \
+                                                           snr_fast, vec, d_out, capacity, d_count, rec_first,    \
+                                                           rec_count, wc);                                        \
+        break;                                                                                                    \
+    }                                                                                                             \
     k_boxcar_filter<W><<<fgrid, kFilterThreads, 0, s>>>(d_plane, rows, cols, d_stats, d_thr, thr, rec_count,     \
                                                         work, work_n, wc);                                        \
     k_boxcar_pair<M, W><<<grid, kPairThreads, 0, s>>>(d_plane, rows, cols, d_stats, d_thr, thr, thr_lo, snr_fast,  \
@@ -1007,16 +1260,24 @@ extern "C" bfs_status bfs_boxcar_gather(const float* d_plane, int rows, int cols
     unsigned* rec = d_count + 64;
     bfs_status st = BFS_OK;
     {
-        cudaError_t e = cudaMemsetAsync(d_count, 0, 2 * sizeof(unsigned), s);
+        cudaError_t e = cudaMemsetAsync(d_count, 0, 3 * sizeof(unsigned), s);
         if (e != cudaSuccess) st = fail(BFS_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
     }
-    if (st == BFS_OK)
-        st = ordered ? launch_boxcar_ordered(d_plane, rows, cols, d_stats, thr, d_thr, widths_mode, param, snr_fast,
-                                             d_out, capacity, d_count, rec, rec + nrec, rec + 2 * nrec, d_count + 1, s)
-                     : launch_boxcar(d_plane, rows, cols, d_stats, thr, d_thr, widths_mode, param,
-                                     snr_fast, d_out, capacity, d_count, s, 0, nullptr);
-    unsigned count = 0;
-    if (st == BFS_OK) st = read_back(&count, d_count, 1, s);
+    auto search = [&](bool full) {
+        return ordered ? launch_boxcar_ordered(d_plane, rows, cols, d_stats, thr, d_thr, widths_mode, param, snr_fast,
+                                               d_out, capacity, d_count, rec, rec + nrec, rec + 2 * nrec, d_count + 1, s,
+                                               full)
+                       : launch_boxcar(d_plane, rows, cols, d_stats, thr, d_thr, widths_mode, param,
+                                       snr_fast, d_out, capacity, d_count, s, 0, nullptr);
+    };
+    if (st == BFS_OK) st = search(false);
+    unsigned words[3] = {0, 0, 0};
+    if (st == BFS_OK) st = read_back(words, d_count, 3, s);
+    if (st == BFS_OK && words[2]) {
+        st = search(true);
+        if (st == BFS_OK) st = read_back(words, d_count, 1, s);
+    }
+    const unsigned count = words[0];
     if (st == BFS_OK) {
         *h_count = count;
         const unsigned n = count < capacity ? count : capacity;

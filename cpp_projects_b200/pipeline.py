@@ -34,7 +34,8 @@ def _fdmt_launches(passes: list) -> int:
 
 
 # Kernels of one search after the FDMT, at most (CUB's not counted): row
-# statistics, boxcar filter and search; compaction; field ranges, three passes
+# statistics, boxcar filter and search (one unfiltered search at low
+# thresholds); compaction; field ranges, three passes
 # x (marks, table), keys, offsets, delegates (lanes, tree, keys).
 SEARCH_LAUNCHES, COMPACT_LAUNCHES, CLUSTER_LAUNCHES = 3, 1, 12
 
