@@ -615,178 +615,211 @@ bool build_adj_run(const FdmtPlanHost& p, const AdjointTables& tab, int l0, int 
         const int* off = tab.off.data() + tab.off_pos[lo + 1];
         const int* ent = tab.ent.data() + 2 * tab.ent_pos[lo + 1];
         const int n = p.lv[lo].total_rows();
-        t.off.reserve(n + 1);
+        t.off.resize(n + 1);
+        if (hi == lo + 1) {
+            t.v.resize(off[n]);
+            for (int i = 0; i <= n; ++i) t.off[i] = off[i];
+            for (int k = 0; k < off[n]; ++k) t.v[k] = {ent[2 * k], ent[2 * k + 1], true};
+            return t;
+        }
+        const int* off2 = tab.off.data() + tab.off_pos[lo + 2];
+        const int* ent2 = tab.ent.data() + 2 * tab.ent_pos[lo + 2];
+        size_t most = 0;
+        for (int k = 0; k < off[n]; ++k) most += off2[ent[2 * k] + 1] - off2[ent[2 * k]];
+        t.v.resize(most);
+        Term* v = t.v.data();
         for (int i = 0; i < n; ++i) {
-            t.off.push_back(static_cast<int>(t.v.size()));
+            t.off[i] = static_cast<int>(v - t.v.data());
             for (int k = off[i]; k < off[i + 1]; ++k) {
-                const int g = ent[2 * k], s = ent[2 * k + 1];
-                if (hi == lo + 1) { t.v.push_back({g, s, true}); continue; }
-                const int* off2 = tab.off.data() + tab.off_pos[lo + 2];
-                const int* ent2 = tab.ent.data() + 2 * tab.ent_pos[lo + 2];
-                for (int q = off2[g]; q < off2[g + 1]; ++q)
-                    t.v.push_back({ent2[2 * q], s + ent2[2 * q + 1], q + 1 == off2[g + 1]});
+                const int g = ent[2 * k], s = ent[2 * k + 1], end = off2[g + 1];
+                for (int q = off2[g]; q < end; ++q) *v++ = {ent2[2 * q], s + ent2[2 * q + 1], q + 1 == end};
             }
         }
-        t.off.push_back(static_cast<int>(t.v.size()));
+        t.off[n] = static_cast<int>(most);
         return t;
     };
     const Terms up = terms(lm, l1), down = terms(l0, lm);
     constexpr int kNone = 1 << 30;
-    // per mid row: least shift of its terms (kNone: no row reads it, its
-    // gradient is zero) and first row that reads it
+    // per mid row: least and largest shift of its terms (kNone: no row reads
+    // it, its gradient is zero) and first row that reads it
     const int nmid = p.lv[lm].total_rows();
-    std::vector<int> least(nmid, kNone), reader(nmid, kNone);
+    std::vector<int> least(nmid, kNone), most(nmid, 0), reader(nmid, kNone);
     for (int g = 0; g < nmid; ++g)
         for (int k = up.off[g]; k < up.off[g + 1]; ++k) {
             least[g] = std::min(least[g], up.v[k].shift);
+            most[g] = std::max(most[g], up.v[k].shift);
             reader[g] = std::min(reader[g], up.v[k].row);
         }
+    // outputs (level-l0 rows, or channels): their window starts E before t0,
+    // E the least shift of their terms; ordered by first reader within the
+    // sub-bands of level l1
+    const int units = final ? p.nchan : p.lv[l0].total_rows();
+    auto terms_of = [&](int i) { return std::make_pair(down.off[i * r0c], down.off[(i + 1) * r0c]); };
+    std::vector<int> lead(units);
+    std::vector<std::pair<int, int>> bands;   // {end in order, weight: the larger of outputs and level-l1 rows}
+    // buckets: a band's level-l1 rows, then its outputs that no row reads
+    std::vector<int> order(units), bucket(units), at(p.lv[l1].total_rows() + p.lv[l1].nsub + 1, 0);
+    for (int band = 0, i = 0; band < p.lv[l1].nsub; ++band) {
+        const int b0 = i, end = p.lv[l0].cum[std::min(p.lv[l0].nsub, (band + 1) << m)];
+        for (; i < units && i * r0c < end; ++i) {
+            int key = p.lv[l1].cum[band + 1], e = kNone;
+            const auto [k0, k1] = terms_of(i);
+            for (int k = k0; k < k1; ++k) {
+                const Term& x = down.v[k];
+                key = std::min(key, reader[x.row]);
+                if (least[x.row] != kNone) e = std::min(e, x.shift + least[x.row]);
+            }
+            lead[i] = e == kNone ? 0 : e & ~7;
+            bucket[i] = key + band;
+            ++at[bucket[i] + 1];
+        }
+        bands.push_back({i, std::max(i - b0, p.lv[l1].rows[band])});
+    }
+    for (size_t k = 1; k < at.size(); ++k) at[k] += at[k - 1];
+    for (int i = 0; i < units; ++i) order[at[bucket[i]]++] = i;
+    std::vector<int> mid_slot(nmid, -1), in_slot(p.lv[l1].total_rows(), -1);
     auto with_rows = [&](const int G) {
-        // outputs (level-l0 rows, or channels) by their first reader, those of a
-        // sub-band of level l1 in parts of at most G, small sub-bands together
-        const int units = final ? p.nchan : p.lv[l0].total_rows();
-        std::vector<std::pair<int, int>> order;   // {first reader, output}
-        std::vector<std::vector<int>> outs;
-        auto cut = [&](size_t i0, size_t i1, int parts) {
-            for (int k = 0; k < parts; ++k) {
-                std::vector<int> o;
-                for (size_t i = i0 + (i1 - i0) * k / parts; i < i0 + (i1 - i0) * (k + 1) / parts; ++i)
-                    o.push_back(order[i].second);
-                std::sort(o.begin(), o.end());
-                if (!o.empty()) outs.push_back(std::move(o));
+        // tiles: those of a sub-band of level l1 in parts of at most G, small sub-bands together
+        std::vector<int> cuts{0};   // ends of the tiles' outputs in `order`
+        auto cut = [&](int i1, int parts) {
+            const int i0 = cuts.back();
+            for (int k = 1; k <= parts; ++k) {
+                const int end = i0 + static_cast<int>(static_cast<long long>(i1 - i0) * k / parts);
+                if (end > cuts.back()) cuts.push_back(end);
             }
         };
-        size_t open = 0;     // start of the outputs not yet cut
-        int weight = 0;      // of their sub-bands: the larger of their output and level-l1 rows
-        for (int band = 0, i = 0; band < p.lv[l1].nsub; ++band) {
-            const size_t b0 = order.size();
-            const int end = p.lv[l0].cum[std::min(p.lv[l0].nsub, (band + 1) << m)];
-            for (; i < units && i * r0c < end; ++i) {
-                int key = kNone;
-                for (int r = i * r0c; r < (i + 1) * r0c; ++r)
-                    for (int k = down.off[r]; k < down.off[r + 1]; ++k) key = std::min(key, reader[down.v[k].row]);
-                order.push_back({key, i});
-            }
-            std::sort(order.begin() + b0, order.end());
-            const int w = std::max(static_cast<int>(order.size() - b0), p.lv[l1].rows[band]);
+        int weight = 0;   // of the sub-bands not yet cut
+        for (size_t b = 0; b < bands.size(); ++b) {
+            const int b0 = b ? bands[b - 1].first : 0, w = bands[b].second;
             if (weight + w > G) {
-                if (b0 > open) cut(open, b0, 1);
-                open = b0;
+                cut(b0, 1);
                 weight = 0;
             }
-            if (w > G) {
-                cut(open, order.size(), (w + G - 1) / G);
-                open = order.size();
-            } else {
-                weight += w;
-            }
+            if (w > G) cut(bands[b].first, (w + G - 1) / G);
+            else weight += w;
         }
-        if (order.size() > open) cut(open, order.size(), 1);
+        cut(units, 1);
         AdjRun s;
         s.l0 = l0; s.l1 = l1; s.final = final;
-        struct Tile { std::vector<int> outs, e, mid, em, in; };
+        // per tile its outputs, mid rows (with the lead and the reach of their
+        // windows, whose sum is the width) and input rows, one after another in
+        // `outs`, `mid` and `in`
+        struct Mid { int row, em, reach; };
+        struct Tile { size_t outs, mid, in; int n2, n1, n_in, len; };
         std::vector<Tile> tiles;
-        std::vector<int> mid_slot(nmid, -1), in_slot(p.lv[l1].total_rows(), -1), width;
+        std::vector<int> outs = order, in;
+        std::vector<Mid> mid;
+        tiles.reserve(cuts.size());
+        mid.reserve(2 * units + 64);
+        in.reserve(2 * units + 64);
         int need_x = 0, max_in = 0, max_mid = 0;
-        for (auto& o : outs) {
-            Tile t;
-            t.outs = std::move(o);
-            // an output's window starts E before t0: the least shift of its terms
-            for (int i : t.outs) {
-                int e = kNone;
-                for (int r = i * r0c; r < (i + 1) * r0c; ++r)
-                    for (int k = down.off[r]; k < down.off[r + 1]; ++k)
-                        if (least[down.v[k].row] != kNone) e = std::min(e, down.v[k].shift + least[down.v[k].row]);
-                e = e == kNone ? 0 : e & ~7;
-                t.e.push_back(e);
+        for (size_t c = 1; c < cuts.size(); ++c) {
+            Tile t{};
+            t.outs = cuts[c - 1];
+            t.mid = mid.size();
+            t.in = in.size();
+            t.n2 = cuts[c] - cuts[c - 1];
+            int* o = outs.data() + t.outs;
+            std::sort(o, o + t.n2);
+            for (int j = 0; j < t.n2; ++j) {
+                const int e = lead[o[j]];
                 s.max_e = std::max(s.max_e, e);
-                for (int r = i * r0c; r < (i + 1) * r0c; ++r)
-                    for (int k = down.off[r]; k < down.off[r + 1]; ++k) {
-                        const int g = down.v[k].row;
-                        if (least[g] == kNone) continue;
-                        if (mid_slot[g] < 0) {
-                            mid_slot[g] = static_cast<int>(t.mid.size());
-                            t.mid.push_back(g);
-                            t.em.push_back(-kNone);
+                int n = 0;   // terms
+                for (int r = 0; r < r0c; ++r)
+                    for (int k = down.off[o[j] * r0c + r]; k < down.off[o[j] * r0c + r + 1]; ++k) {
+                        const Term& x = down.v[k];
+                        if (least[x.row] == kNone) continue;
+                        n += final ? r + 1 : 1;
+                        int& slot = mid_slot[x.row];
+                        if (slot < 0) {
+                            slot = t.n1++;
+                            mid.push_back({x.row, -kNone, -kNone});
                         }
-                        int& em = t.em[mid_slot[g]];
-                        em = std::max(em, e - down.v[k].shift);
+                        Mid& d = mid[t.mid + slot];
+                        d.em = std::max(d.em, e - x.shift);
+                        d.reach = std::max(d.reach, kSegTile + x.shift + r - e);
                     }
+                t.len += (n + 3) & ~3;
             }
-            width.assign(t.mid.size(), 0);
-            for (size_t j = 0; j < t.outs.size(); ++j)
-                for (int r = t.outs[j] * r0c; r < (t.outs[j] + 1) * r0c; ++r)
-                    for (int k = down.off[r]; k < down.off[r + 1]; ++k) {
-                        const int q = mid_slot[down.v[k].row];
-                        if (q >= 0) width[q] = std::max(width[q], kSegTile + down.v[k].shift + r % r0c - t.e[j] + t.em[q]);
-                    }
             bool fits = true;
-            for (size_t q = 0; q < t.mid.size(); ++q) {
-                fits = fits && width[q] <= kRunMid;
-                for (int k = up.off[t.mid[q]]; k < up.off[t.mid[q] + 1]; ++k) {
-                    need_x = std::max(need_x, up.v[k].shift - t.em[q] + width[q]);
+            const Mid* md = mid.data() + t.mid;
+            for (int q = 0; q < t.n1; ++q) {
+                fits = fits && md[q].em + md[q].reach <= kRunMid;
+                need_x = std::max(need_x, most[md[q].row] + md[q].reach);
+                t.len += (up.off[md[q].row + 1] - up.off[md[q].row] + 3) & ~3;
+                for (int k = up.off[md[q].row]; k < up.off[md[q].row + 1]; ++k) {
                     int& slot = in_slot[up.v[k].row];
                     if (slot < 0) {
                         slot = 0;
-                        t.in.push_back(up.v[k].row);
+                        in.push_back(up.v[k].row);
                     }
                 }
             }
-            std::sort(t.in.begin(), t.in.end());
-            for (int g : t.mid) mid_slot[g] = -1;
-            for (int d : t.in) in_slot[d] = -1;
-            max_in = std::max(max_in, static_cast<int>(t.in.size()));
-            max_mid = std::max(max_mid, static_cast<int>(t.mid.size()));
+            t.n_in = static_cast<int>(in.size() - t.in);
+            for (int q = 0; q < t.n1; ++q) mid_slot[md[q].row] = -1;
+            for (int k = 0; k < t.n_in; ++k) in_slot[in[t.in + k]] = -1;
+            max_in = std::max(max_in, t.n_in);
+            max_mid = std::max(max_mid, t.n1);
             if (!fits || 4ull * (static_cast<size_t>(max_in) * need_x + static_cast<size_t>(max_mid) * kRunMid) > smem_limit)
                 return false;
-            tiles.push_back(std::move(t));
+            t.len += ((t.n1 + 3 * t.n2 + 3) & ~3) + 4;   // (the kernel reads ahead)
+            s.max_blob = std::max(s.max_blob, t.len);
+            s.pitch_x = (need_x + 3 + 3) & ~3;   // + the largest lead
+            s.y0 = max_in * s.pitch_x + kRunMid;          // a mid row's read may run past the last input row
+            s.blob0 = s.y0 + max_mid * kRunMid + kSegTile;
+            s.smem_bytes = 4 * (static_cast<size_t>(s.blob0) + 2 * static_cast<size_t>(s.max_blob));
+            if (s.pitch_x > kRunMaxPitch || max_in > 256 || s.smem_bytes > smem_limit) return false;
+            std::sort(in.begin() + t.in, in.end());
+            tiles.push_back(t);
         }
-        s.pitch_x = (need_x + 3 + 3) & ~3;   // + the largest lead
-        if (s.pitch_x > kRunMaxPitch || max_in > 256) return false;
-        s.y0 = max_in * s.pitch_x + kRunMid;          // a mid row's read may run past the last input row
-        s.blob0 = s.y0 + max_mid * kRunMid + kSegTile;
-        std::vector<int> head, term;
+        s.tiles.reserve(tiles.size());
+        s.rows.reserve(2 * in.size());
+        std::vector<int> head, terms_buf(s.max_blob);
+        int* const term = terms_buf.data();
         for (const Tile& t : tiles) {
             AdjTile r{};
             r.row = static_cast<int>(s.rows.size() / 2);
             r.blob = static_cast<int>(s.blob.size());
-            r.n_in = static_cast<int>(t.in.size());
-            r.n1 = static_cast<int>(t.mid.size());
-            r.n2 = static_cast<int>(t.outs.size());
-            for (int e : t.e) r.max_e = std::max(r.max_e, e);
-            for (size_t j = 0; j < t.in.size(); ++j) {
-                const int lead = static_cast<int>((static_cast<long long>(t.in[j]) * in_pitch) & 3);
-                in_slot[t.in[j]] = static_cast<int>(j) * s.pitch_x + lead;
-                s.rows.insert(s.rows.end(), {t.in[j], lead});
+            r.n_in = t.n_in;
+            r.n1 = t.n1;
+            r.n2 = t.n2;
+            const int *o = outs.data() + t.outs, *ti = in.data() + t.in;
+            const Mid* md = mid.data() + t.mid;
+            for (int j = 0; j < t.n2; ++j) r.max_e = std::max(r.max_e, lead[o[j]]);
+            for (int j = 0; j < t.n_in; ++j) {
+                const int before = static_cast<int>((static_cast<long long>(ti[j]) * in_pitch) & 3);
+                in_slot[ti[j]] = j * s.pitch_x + before;
+                s.rows.push_back(ti[j]);
+                s.rows.push_back(before);
             }
             head.clear();
-            term.clear();
+            size_t n = 0;   // terms written
             const int base = (r.n1 + 3 * r.n2 + 3) & ~3;
             // closes a row's terms from `from` on: kind, end mark, padding
             auto close = [&](size_t from, bool channel) {
                 const int at = base + static_cast<int>(from);
-                if (term.size() == from) return at | kAdjZero;
-                const size_t n = term.size() - from;
+                if (n == from) return at | kAdjZero;
                 int kind = kAdjTerms;
-                if (!channel && n == 2 && (term[from] & 1)) kind = kAdjOnes;
-                if (!channel && n == 4 && !(term[from] & 1) && (term[from + 1] & 1) && !(term[from + 2] & 1)) kind = kAdjPairs;
-                term.back() |= kAdjEnd;
-                while (term.size() % 4) term.push_back(0);
+                if (!channel && n == from + 2 && (term[from] & 1)) kind = kAdjOnes;
+                if (!channel && n == from + 4 && !(term[from] & 1) && (term[from + 1] & 1) && !(term[from + 2] & 1))
+                    kind = kAdjPairs;
+                term[n - 1] |= kAdjEnd;
+                while (n % 4) term[n++] = 0;
                 return at | kind;
             };
-            for (size_t q = 0; q < t.mid.size(); ++q) {
-                mid_slot[t.mid[q]] = static_cast<int>(q);
-                const size_t from = term.size();
-                for (int k = up.off[t.mid[q]]; k < up.off[t.mid[q] + 1]; ++k) {
+            for (int q = 0; q < t.n1; ++q) {
+                mid_slot[md[q].row] = q;
+                const size_t from = n;
+                for (int k = up.off[md[q].row]; k < up.off[md[q].row + 1]; ++k) {
                     const Term& x = up.v[k];
-                    if (x.shift - t.em[q] < 0) return false;
-                    term.push_back(4 * (in_slot[x.row] + x.shift - t.em[q]) | (x.last ? 1 : 0));
+                    if (x.shift - md[q].em < 0) return false;
+                    term[n++] = 4 * (in_slot[x.row] + x.shift - md[q].em) | (x.last ? 1 : 0);
                 }
                 head.push_back(close(from, false));
             }
-            for (size_t j = 0; j < t.outs.size(); ++j) {
-                const int i = t.outs[j];
-                const size_t from = term.size();
+            for (int j = 0; j < t.n2; ++j) {
+                const int i = o[j];
+                const size_t from = n;
                 for (int rr = 0; rr < r0c; ++rr)
                     for (int rd = 0; rd <= (final ? rr : 0); ++rd) {
                         int last = -1;   // last term of this value
@@ -797,28 +830,27 @@ bool build_adj_run(const FdmtPlanHost& p, const AdjointTables& tab, int l0, int 
                                 if (x.last && last >= 0) term[last] |= 1;
                                 continue;
                             }
-                            last = static_cast<int>(term.size());
-                            term.push_back(4 * (s.y0 + q * kRunMid + t.em[q] + x.shift - t.e[j] + rd) | (x.last ? 1 : 0));
+                            last = static_cast<int>(n);
+                            term[n++] = 4 * (s.y0 + q * kRunMid + md[q].em + x.shift - lead[i] + rd) | (x.last ? 1 : 0);
                         }
                         if (last < 0) continue;   // the row's gradient is zero
                         if (final) term[last] |= 3 | rr << 20 | rd << 23 | (rd == rr ? 1 << 26 : 0);
                         else term[last] |= 1;
                     }
-                head.insert(head.end(), {i, t.e[j], close(from, final)});
+                const int at = close(from, final);
+                head.push_back(i);
+                head.push_back(lead[i]);
+                head.push_back(at);
             }
             head.resize(base, 0);
-            head.insert(head.end(), term.begin(), term.end());
-            head.insert(head.end(), {0, 0, 0, 0});   // (the kernel reads ahead)
-            while (head.size() % 4) head.push_back(0);
-            r.len = static_cast<int>(head.size());
-            s.max_blob = std::max(s.max_blob, r.len);
+            r.len = t.len;
             s.blob.insert(s.blob.end(), head.begin(), head.end());
+            s.blob.insert(s.blob.end(), term, term + n);
+            s.blob.resize(r.blob + r.len, 0);
             s.tiles.push_back(r);
-            for (int g : t.mid) mid_slot[g] = -1;
-            for (int d : t.in) in_slot[d] = -1;
+            for (int q = 0; q < t.n1; ++q) mid_slot[md[q].row] = -1;
+            for (int k = 0; k < t.n_in; ++k) in_slot[ti[k]] = -1;
         }
-        s.smem_bytes = 4 * (static_cast<size_t>(s.blob0) + 2 * static_cast<size_t>(s.max_blob));
-        if (s.smem_bytes > smem_limit) return false;
         *out = std::move(s);
         return true;
     };
