@@ -74,8 +74,8 @@ def test_run_segment_schedules_can_be_created(fmin, fmax, nchan, max_dt, levels)
 def test_tuned_plans_time_the_default_schedule(cuda, fmin, fmax, nchan, max_dt):
     d = _capi.FdmtDesc(fmin=fmin, fmax=fmax, nchan=nchan, ncols=1000, max_dt=max_dt)
     t, ms = autotune_desc(d)
-    # a short plane's passes cost a launch each: the fewest passes, those of the default, win clearly
-    assert 0.0 < ms < 1e3 and t.seg_levels == 4
+    # a short plane's passes cost a launch each: no more of them than the default's
+    assert 0.0 < ms < 1e3 and info_of(t)[1] <= -(-(nchan.bit_length() - 1) // 4)
     f = CFdmtGpu(fmin, fmax, nchan, 1000, max_dt, fuse_depth=-2)
     own = (f.info.fuse_depth, f.info.hbm_passes, f.info.seg_levels)
     assert own == info_of(t) == info_of(t, host=True)
