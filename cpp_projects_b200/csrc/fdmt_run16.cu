@@ -143,6 +143,10 @@ __global__ void __launch_bounds__(kThreads16, 2) k_fdmt_run16(const Run16Args a)
         for (int i = threadIdx.x; i < nent; i += kThreads16) copy16(se + 16u * i, a.ent + t.ent + i);
         const int t0 = tt * kRun16Tile;
         const int pieces = a.pitch_x >> 3;
+        // the last row's reads run past its end, into a row that this tile does
+        // not load: what lies there would decide whether sums left the range
+        if (threadIdx.x < kRun16Over / 8 && t.n_in * a.pitch_x < a.zero_x)
+            *reinterpret_cast<uint4*>(sm16 + 2 * (t.n_in * a.pitch_x) + 16 * threadIdx.x) = make_uint4(0u, 0u, 0u, 0u);
         for (int i = 0, j = warp; j < t.n_in; ++i, j += kWarps16) {
             const int row = __shfl_sync(0xffffffffu, mine.x, i), lead = __shfl_sync(0xffffffffu, mine.y, i);
             const int ts = t0 - lead;   // a multiple of 8: a piece lies before sample 0 or from it on

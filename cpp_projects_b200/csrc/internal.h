@@ -304,6 +304,7 @@ constexpr int kRunOutChunks = kSegTile / 32;
 constexpr int kRunMaxPitch = 384;
 constexpr int kRun16Tile = 2 * kSegTile;          // 16-bit plans: the same bytes per row
 constexpr int kRun16Mid = 2 * kRunMid;
+constexpr int kRun16Over = 72;                    // values past its last input row that a tile may read (cleared)
 
 struct RunTile {                 // device-side
     int row;                     // first of the tile's input rows
