@@ -1520,24 +1520,14 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
     const bool runs = base.precision == BFS_PREC_F32 && plan_host_part(&d0, probe, false) == BFS_OK &&
                       !probe->runs.empty() && probe->runs[0].s1 > 0;
     if (runs) {
-        // (named with 32 rows as before where that description is accepted;
-        // run segments choose their own)
-        for (int seg : {4, 3, 2})
-            for (int rows : {32, 0}) {
-                bfs_fdmt_desc d = d0;
-                d.fuse_depth = 0;
-                d.seg_levels = seg;
-                d.seg_rows = rows;
-                if (plan_host_part(&d, probe, true) != BFS_OK) continue;
-                cands.push_back({0, 0, seg, rows, 0});
-                // small planes, whose passes cost little more than their launches: after a head, too
-                // (128 x 4000, max delay 32: 13.0 us after three levels, 14.0 without a head)
-                if (seg == 4 && static_cast<long long>(base.nchan) * base.ncols <= (1 << 20) && base.plan_kind == BFS_PLAN_KEITH)
-                    for (int k : {2, 3, 4}) cands.push_back({k, 256, seg, rows, 0});
-                break;
-            }
-    }
-    if (cands.empty()) {
+        for (int seg : {4, 3, 2}) {
+            cands.push_back({0, 0, seg, 0, 0});
+            // small planes, whose passes cost little more than their launches: after a head, too
+            // (128 x 4000, max delay 32: 13.0 us after three levels, 14.0 without a head)
+            if (seg == 4 && static_cast<long long>(base.nchan) * base.ncols <= (1 << 20) && base.plan_kind == BFS_PLAN_KEITH)
+                for (int k : {2, 3, 4}) cands.push_back({k, 256, seg, 0, 0});
+        }
+    } else {
     // one merge pass per level: head depth x head tile
     cands.push_back({0, 0, 1, 0, 0});
     for (int k : {2, 3, 4, 5})
@@ -1625,6 +1615,13 @@ static bfs_status tune_fdmt(const bfs_fdmt_desc& base, TuneVal* best) {
         timed = true;
         v.ms = *ms;
         if (v.ms < win.ms) win = v;
+    }
+    // run segments choose their own rows per tile; the description names 32,
+    // as it always has, where one that does is accepted
+    if (timed && runs) {
+        bfs_fdmt_desc d = desc_of(win);
+        d.seg_rows = 32;
+        if (plan_host_part(&d, probe, true) == BFS_OK) win.rows = 32;
     }
     // 16-bit plans: the depth decides where values are rounded, so it is the
     // plain passes' (one per level) best; run segments give their bits and

@@ -152,6 +152,10 @@ __global__ void __launch_bounds__(kThreads16, 2) k_fdmt_run16(const Run16Args a)
             const int ts = t0 - lead;   // a multiple of 8: a piece lies before sample 0 or from it on
             const S* src = static_cast<const S*>(a.in) + static_cast<size_t>(row) * a.in_pitch + ts;
             const unsigned dst = sbase + 2u * (j * a.pitch_x);
+            if (ts >= 0 && ts + a.pitch_x <= a.ncols) {
+                for (int c = lane; c < pieces; c += 32) copy16(dst + 16u * c, src + 8 * c);
+                continue;
+            }
             for (int c = lane; c < pieces; c += 32) {
                 const int at = ts + 8 * c;
                 if (at >= 0 && at + 8 <= a.ncols) {
