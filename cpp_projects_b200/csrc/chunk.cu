@@ -120,21 +120,20 @@ __device__ __forceinline__ float2 chirp_factor(double dm, int ichan, int isft, i
 // Chirp: one thread per (bin of the mbin sub-band, sub-band, coarse channel);
 // the factor is applied to every polarisation and FFT segment at the
 // fft-shifted position of the nbin spectrum.
-// tab: a table of the factors, to be read (known) or to receive them.
-__global__ void k_chirp(const float2* __restrict__ in, float2* __restrict__ out, float2* __restrict__ tab, int known,
-                        double dm, int nchan, int len_sft, int mbin, int nbin, int nseg, double fmin,
-                        double bw_sub, double bw_chan) {
+// TAB: a table of the factors is read, or receives them.
+enum ChirpTab { kNoTab, kFillTab, kReadTab };
+template <ChirpTab TAB>
+__global__ void k_chirp(const float2* __restrict__ in, float2* __restrict__ out, float2* __restrict__ tab, double dm,
+                        int nchan, int len_sft, int mbin, int nbin, int nseg, double fmin, double bw_sub,
+                        double bw_chan) {
     const int ibin = blockIdx.x * blockDim.x + threadIdx.x;
     if (ibin >= mbin) return;
     const int isft = blockIdx.y, ichan = blockIdx.z;
     const size_t at = (static_cast<size_t>(ichan) * len_sft + isft) * mbin + ibin;
     float2 cf;
-    if (known) {
-        cf = tab[at];
-    } else {
-        cf = chirp_factor(dm, ichan, isft, ibin, len_sft, mbin, nbin, fmin, bw_sub, bw_chan);
-        if (tab) tab[at] = cf;
-    }
+    if constexpr (TAB == kReadTab) cf = tab[at];
+    else cf = chirp_factor(dm, ichan, isft, ibin, len_sft, mbin, nbin, fmin, bw_sub, bw_chan);
+    if constexpr (TAB == kFillTab) tab[at] = cf;
     const size_t pos = static_cast<size_t>(ichan) * nbin + (isft * mbin + ibin + nbin / 2) % nbin;
     const size_t stride = static_cast<size_t>(nbin) * nchan;
     for (int i = 0; i < nseg; ++i) {
@@ -427,9 +426,9 @@ static bfs_status chunk_voltages(bfs_chunk* c, const void* d_spec, double dm, fl
         known = i < c->kept.size();
         if (i < c->kept_max) tab = c->kept_tab + i * n;
     }
-    k_chirp<<<grid, 256, 0, s>>>(static_cast<const float2*>(d_spec), d_volt, tab, known, dm, d.nchan, d.len_sft,
-                                 c->mbin, d.nbin, d.nfft * d.npol / 2, static_cast<double>(d.fmin),
-                                 bw_sub, bw_chan);
+    auto* kern = known ? k_chirp<kReadTab> : tab ? k_chirp<kFillTab> : k_chirp<kNoTab>;
+    kern<<<grid, 256, 0, s>>>(static_cast<const float2*>(d_spec), d_volt, tab, dm, d.nchan, d.len_sft, c->mbin, d.nbin,
+                              d.nfft * d.npol / 2, static_cast<double>(d.fmin), bw_sub, bw_chan);
     BFS_LAUNCH_CHECK("k_chirp");
     if (tab && !known && runs_now(s)) c->kept.push_back(dm);   // (its table is filled by this launch)
     bfs_status st = cufft_check(cufftSetStream(c->inv, s), "cufftSetStream");
