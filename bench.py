@@ -562,7 +562,7 @@ def run_ours(args):
                                "candidate buffers)",
                        "parallelism": f"{world} independent rank(s), beams sharded, no collective"},
             "roofline": {"bound": "hbm",
-                         "kernel": "FDMT (fused head or level 0, then fused merge segments)",
+                         "kernel": "FDMT (run segments k_fdmt_run, the first from the channels)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak if plain else None, "peak_source": peak_kind,
                          "traffic": traffic,
@@ -823,7 +823,7 @@ def run_config4(args):
         "config": {"workload": "config4", "nchan": b.nchan, "nsamp": b.nsamp, "max_dt": b.max_dt,
                    "step": "w*x -> FDMT -> S/N at 8 pulse cells -> backward (adjoint boxcar, adjoint FDMT)",
                    "l2": "no flush: 256 MiB planes exceed L2"},
-        "roofline": {"bound": "hbm", "kernel": "adjoint FDMT (level gathers + level-0 adjoint)",
+        "roofline": {"bound": "hbm", "kernel": "adjoint FDMT (run segments k_adj_run)",
                      "achieved": alg / (adj_ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": alg / (adj_ms / 1e3) / 1e9 / peak, "peak_source": peak_kind, "traffic": None},
         "adjoint": {"forward_fdmt_ms": fwd_ms, "adjoint_fdmt_ms": adj_ms, "ratio": adj_ms / fwd_ms,

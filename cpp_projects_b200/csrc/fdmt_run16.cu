@@ -106,13 +106,12 @@ __device__ __noinline__ float plain16(const char* sm, int4 q, int col, int l) {
 
 // The shape of the loops is k_fdmt_run's.  A lane holds two neighbouring
 // columns, so that an input at an even offset costs one shared wavefront per 64
-// columns, at an odd one two and a cut.  Bound by instruction issue (58 % of the
-// slots at 16 warps per SM) and the dependent latencies between them: 4096 x
-// 131072, levels 2..12 in three passes (4 + 4 + 3): 2.53 ms; one plain pass per
-// level 5.52 ms.  Without the halvings 2.34 ms, with every offset even 2.20.
-// Tiles of 256 samples, three CTAs per SM: 3.31 ms (a row's fixed
-// instructions are as many as its merges); four CTAs spill, 4.01.  The range
-// tested row by row 2.95 ms.
+// columns, at an odd one two and a cut.  Bound by instruction issue (59-63 % of
+// the slots at 16 warps per SM) and the dependent latencies between them: 4096 x
+// 131072, levels 1..12 in three passes of four: 2.39 ms; one plain pass per level
+// 5.9 ms.  Slower: tiles of 256 samples at three CTAs per SM (a row's fixed
+// instructions are as many as its merges), four CTAs (spills), the range tested
+// row by row.
 template <typename S, int S1, int S2, bool F32OUT>
 __global__ void __launch_bounds__(kThreads16, 2) k_fdmt_run16(const Run16Args a) {
     using V = typename Pair<S>::V;
