@@ -1325,6 +1325,10 @@ static bfs_status build_passes(const bfs_fdmt_desc* desc, bfs_fdmt_plan* p, int 
         // run segments where every row of a level has the scale of its level
         // (a power-of-two channel count), else one plain pass per level
         const auto even = [&] {
+            bool pairs = true;   // every row of every level sums two of the level below: 2^l channels
+            for (int l = 1; l <= h.niter && pairs; ++l)
+                pairs = std::find_if(h.lv[l].b_row.begin(), h.lv[l].b_row.end(), [](int b) { return b < 0; }) == h.lv[l].b_row.end();
+            if (pairs) return true;
             const std::vector<std::vector<int>> ex = row_exponents(h);
             for (int l = k; l <= h.niter; ++l)
                 for (int e : ex[l])
@@ -1726,12 +1730,12 @@ extern "C" bfs_status bfs_fdmt_plan_create(const bfs_fdmt_desc* desc_in, bfs_fdm
     // row tables of the plain levels; with 16-bit planes w packs the per-row
     // scale exponents
     std::vector<std::vector<int>> ex;
-    if (p->precision != BFS_PREC_F32) ex = row_exponents(h);
     std::vector<int4> tab;
     p->tab_off.assign(h.niter + 1, 0);
     for (size_t i = 0; i < p->passes.size(); ++i) {
         if (p->runs[i].s1 > 0 || !p->passes[i].tiles.empty()) continue;
         const int l = p->passes[i].l1;
+        if (p->precision != BFS_PREC_F32 && ex.empty()) ex = row_exponents(h);
         p->tab_off[l] = tab.size();
         const FdmtLevel& L = h.lv[l];
         for (int g = 0; g < L.total_rows(); ++g) {
